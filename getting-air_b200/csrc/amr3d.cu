@@ -33,7 +33,7 @@
 
 #include "../../include/lbm.h"
 #include "amr3d.cuh"
-#include "cell_update.cuh"
+#include "dense_block.cuh"
 #include "host_params.cuh"
 #include "scan.cuh"
 #include "sample.cuh"
@@ -735,16 +735,27 @@ __global__ void __launch_bounds__(kTileThreads)
 }
 
 // ---- L0 step, skipping covered blocks ------------------------------------
+// The dense step's launch mapping and update; the block of a cell by
+// multiplication (row_magic of rb).
 template <int Q>
 __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) / 4 : kStepMinBlocks)
     amr3_coarse(const float *__restrict__ fin, float *__restrict__ fout, float *__restrict__ mac,
-                const __grid_constant__ StepParams sp, const int *__restrict__ block_slot, int rb, int nbx, int nby) {
+                const __grid_constant__ StepParams sp, const int *__restrict__ block_slot, unsigned rb_magic, int nbx,
+                int nby) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
-  const int x = blockIdx.x * kStepThreads + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
-  if (x >= sp.nx) return;
-  if (block_slot[((z / rb) * nby + y / rb) * nbx + x / rb] >= 0) return;
+  const BlockMap m = block_map(sp, kStepThreads);
+  const int c = m.c0 + threadIdx.x;
+  if (c >= m.lim) return;
+  int x, y;
+  block_cell(sp, m, c, x, y);
+  auto blk = [&](int v) { return (int)__umulhi((unsigned)v, rb_magic); };  // v / rb
+  if (block_slot[(blk(m.bz) * nby + blk(y)) * nbx + blk(x)] >= 0) return;
+  if (block_kind(sp, m, kStepThreads) == kFluid) {
+    cell3_fluid<Q, float>(fin, fout, mac, sp, x, y, m.bz);
+    return;
+  }
   CellForce cf;
-  cell3<Q, float>(fin, fout, mac, sp, x, y, z, false, cf);
+  cell3<Q, float>(fin, fout, mac, sp, x, y, m.bz, false, cf);
 }
 
 // ---- pool force (common_d3_force_pool.wgsl) -------------------------------
@@ -1252,25 +1263,6 @@ int coalesce_subs(const Amr3Params &p, int sms) {
   return subs;
 }
 
-// A launch that may begin while the previous kernel on the stream drains
-// (programmatic dependent launch; in a graph, a programmatic edge): the
-// macro-step's kernels wait at their first instruction (griddepcontrol.wait)
-// until the previous one has completed and its writes are visible, so the
-// order is the stream's; the new grid's launch overlaps the old one's tail.
-template <typename... K, typename... A>
-void launch_pdl(dim3 g, dim3 b, cudaStream_t st, void (*k)(K...), A &&...args) {
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = g;
-  lc.blockDim = b;
-  lc.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = 1;
-  cudaLaunchKernelEx(&lc, k, std::forward<A>(args)...);
-}
-
 template <int Q>
 void launch_coalesce(cudaStream_t st, const float *fp, float *fc, float4 *macc, const float4 *macp,
                      const Amr3Params &p, int subs) {
@@ -1317,7 +1309,7 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
     // and every tile restricted into L0's new buffer.
     StepParams sp = a->sp;
     sp.write_mac = write_mac ? 1 : 0;
-    const dim3 gs((p.nx + kStepThreads - 1) / kStepThreads, p.ny, p.nz);
+    const dim3 gs = step_grid(sp);
     const dim3 g = tile_grid(a);
     const dim3 gl((p.T3 + kListThreads - 1) / kListThreads, p.slots);
     const int rb3 = p.rb * p.rb * p.rb;
@@ -1328,8 +1320,8 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
     const float f2c_rescale = 2.f * (tc - 1.f) / (tf - 1.f);
     AMR3_DISPATCH(q, {
       if (p.c.has_body) launch_pool_force<Q>(a, p, st);
-      amr3_coarse<Q><<<gs, kStepThreads, 0, st>>>(a->fc[cp], a->fc[1 - cp], a->macc, sp, a->d_block_slot, p.rb,
-                                                   p.nbx, p.nby);
+      amr3_coarse<Q><<<gs, kStepThreads, 0, st>>>(a->fc[cp], a->fc[1 - cp], a->macc, sp, a->d_block_slot,
+                                                   row_magic(p.rb), p.nbx, p.nby);
       amr3_interp<Q><<<g, tile_block(a), 0, st>>>(a->fc[cp], a->fp[0], p, 1, nullptr);
       Amr3Params pa = p;
       pa.write_mac = 0;
@@ -1366,9 +1358,9 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
   }
   StepParams sp = a->sp;
   sp.write_mac = write_mac ? 1 : 0;
-  const dim3 gs((p.nx + kStepThreads - 1) / kStepThreads, p.ny, p.nz);
+  const dim3 gs = step_grid(sp);
   AMR3_DISPATCH(q, launch_pdl(gs, dim3(kStepThreads), st, amr3_coarse<Q>, (const float *)a->fc[cp], a->fc[1 - cp],
-                              a->macc, sp, (const int *)a->d_block_slot, p.rb, p.nbx, p.nby));
+                              a->macc, sp, (const int *)a->d_block_slot, row_magic(p.rb), p.nbx, p.nby));
 }
 
 void destroy_graphs(lbm_amr3d *a) {

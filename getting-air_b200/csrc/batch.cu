@@ -94,52 +94,6 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
   }
 }
 
-// One D2Q9 cell of a domain with no body and outside any force region:
-// cell2_core with the tests that cannot fire taken out (no solid link,
-// chi = 0 and u_s = 0, so the Guo force is the body force) and only the
-// moving-wall patch of a wall row kept, the same arithmetic in the same
-// order, so the same bits.
-template <typename S>
-__device__ __forceinline__ void cell2_fluid(const S *__restrict__ fin, float (&f)[9], S *__restrict__ fout,
-                                            float *__restrict__ mac, const StepParams &p, int x, int y) {
-  using L = Lattice<9>;
-  const int W = p.nx, H = p.ny;
-  const int cell = y * W + x;
-  if (p.wall_y && (y == 0 || y == H - 1)) {
-    const S *fi = fin + p.base;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const int ex = L::ex(i), ey = L::ey(i), o = L::opp(i);
-      const int ysrc = y - ey;
-      if (ysrc < 0 || ysrc >= H) {
-        const float wu = ysrc < 0 ? p.wall_u0 : p.wall_u1;
-        const float corr = 2.f * L::w(i) * (float)ex * wu * kInvCS2;
-        f[i] = Codec<S>::ld(fi + (int64_t)o * p.n + cell, o, p.pk) + corr;
-      }
-    }
-  }
-  float rho, mxs, mys, mzs;
-  moments<L, 9>(f, rho, mxs, mys, mzs);
-  const float rhoDen = fmaxf(rho, 1e-6f);
-  const float inv = 1.0f / rhoDen;
-  const float uxs = mxs * inv, uys = mys * inv;
-  const float chi = 0.f, usx = 0.f, usy = 0.f;
-  const float Fx = rho * chi * (usx - uxs) + p.fx;
-  const float Fy = rho * chi * (usy - uys) + p.fy;
-  const float hinv = 0.5f * inv;
-  const float ux = fmaf(Fx, hinv, uxs);
-  const float uy = fmaf(Fy, hinv, uys);
-  float spw = 0.f;
-  if (p.sponge_w > 0.f) {
-    const float dx = fminf((float)x, (float)(W - 1 - x));
-    const float dy = fminf((float)y, (float)(H - 1 - y));
-    spw = sponge_weight_inv(fminf(dx, dy), p.sponge_inv);
-  }
-  MemSink<S> sink{fout + p.base, p.n, cell, p.pk};
-  collide_store<L, 9>(f, rho, ux, uy, 0.f, Fx, Fy, 0.f, p.omega, spw, p.ftarget, sink);
-  if (p.write_mac) reinterpret_cast<float4 *>(mac + 4 * p.base)[cell] = make_float4(rho, ux, uy, 0.f);
-}
-
 // The fluid tiles of a D2Q9 batch (cell2_fluid). Without the bounce-back
 // and force code the update fits 64 registers, and 1024 resident
 // threads per SM keep more loads in flight: the loop is memory-latency

@@ -55,6 +55,27 @@ LBM_HD float body_circumradius(const lbm_body &b) {
   }
 }
 
+// Half-extents of a 3D body along the axes, in its pose: at most the
+// circumradius, with slack for the f32 rotation; the circumradius where the
+// quaternion is not a unit one. (An axis-aligned cube's box holds a fifth of
+// the cells of its circumsphere's.)
+LBM_HD void body_extents(const lbm_body &b, float ext[3]) {
+  const float rc = body_circumradius(b);
+  for (int a = 0; a < 3; ++a) ext[a] = rc;
+  const float w = b.qw, x = b.qx, y = b.qy, z = b.qz;
+  if (b.shape == LBM_SHAPE_SPHERE || !(fabsf(w * w + x * x + y * y + z * z - 1.0f) < 1e-3f)) return;
+  const float R[3][3] = {{1.f - 2.f * (y * y + z * z), 2.f * (x * y - w * z), 2.f * (x * z + w * y)},
+                         {2.f * (x * y + w * z), 1.f - 2.f * (x * x + z * z), 2.f * (y * z - w * x)},
+                         {2.f * (x * z - w * y), 2.f * (y * z + w * x), 1.f - 2.f * (x * x + y * y)}};
+  const bool box = b.shape == LBM_SHAPE_ROUNDBOX;
+  const float h[3] = {b.a, box ? b.b : b.a, b.c};
+  for (int a = 0; a < 3; ++a) {
+    float s = 0.f;
+    for (int j = 0; j < 3; ++j) s += box ? fabsf(R[a][j] * h[j]) : (R[a][j] * h[j]) * (R[a][j] * h[j]);
+    ext[a] = fminf(rc, (box ? s : sqrtf(s)) * 1.002f + 0.1f);
+  }
+}
+
 // Inclusive cell box [x0,x1]x[y0,y1]x[z0,z1] outside which no cell can add
 // to the body force: a bounce-back link is at most sqrt(3) long, the
 // swept-cell term reaches one step of surface motion, and the penalty's chi
@@ -63,20 +84,24 @@ LBM_HD float body_circumradius(const lbm_body &b) {
 // the domain is within reach. On a windowed axis (win[a] set) the box is
 // not clipped: it may start below 0 or end past the last cell, to be read
 // modulo the axis, and it covers the whole axis once it is that long.
+// `tight` false: around the circumsphere whatever the pose.
 LBM_HD bool body_cell_box(const lbm_body &b, int q, int nx, int ny, int nz, int bounceback, int swept_force,
-                          float chi_eps, int box[6], int *swept, float *band, const int *win = nullptr) {
+                          float chi_eps, int box[6], int *swept, float *band, const int *win = nullptr,
+                          bool tight = true) {
   const float rc = body_circumradius(b);
+  float ext[3] = {rc, rc, rc};
+  if (q != 9 && tight) body_extents(b, ext);
   const float speed = sqrtf(b.vx * b.vx + b.vy * b.vy + b.vz * b.vz) +
                       sqrtf(b.wx * b.wx + b.wy * b.wy + b.wz * b.wz) * rc;
   *swept = (q != 9 && bounceback && swept_force && speed > 0.f) ? 1 : 0;
   *band = 2.0f + speed;
   const float margin = bounceback ? (3.0f + speed) : (8.0f * chi_eps + 2.0f);
-  const float reach = rc + margin;
   const bool wrap2d = (q == 9);  // the 2D SDF takes the nearest periodic image
   const float centre[3] = {b.cx, b.cy, b.cz};
   const int len[3] = {nx, ny, nz};
   for (int a = 0; a < 3; ++a) {
     if (a == 2 && q == 9) { box[4] = box[5] = 0; break; }
+    const float reach = ext[a] + margin;
     int lo = (int)floorf(centre[a] - reach), hi = (int)ceilf(centre[a] + reach);
     if (win && win[a]) {
       if (hi - lo + 1 >= len[a]) { lo = 0; hi = len[a] - 1; }
@@ -256,6 +281,23 @@ struct BodyPose {
   int swept;
   float swept_band;
 };
+
+// The reach box of a pose from its cell box (body_cell_box; any = false: the
+// body reaches no cell, an empty box), as StepParams::nbox holds it.
+LBM_HD void reach_box3(const int box[6], bool any, int nx, int ny, int nz, int nbox[6]) {
+  const int len[3] = {nx, ny, nz};
+  for (int a = 0; a < 3; ++a) {
+    if (!any) {
+      nbox[2 * a] = 0;
+      nbox[2 * a + 1] = -1;
+      continue;
+    }
+    int lo = box[2 * a] % len[a];
+    if (lo < 0) lo += len[a];
+    nbox[2 * a] = lo;
+    nbox[2 * a + 1] = lo + (box[2 * a + 1] - box[2 * a]);
+  }
+}
 
 struct BodyDyn {
   lbm_body_state st;

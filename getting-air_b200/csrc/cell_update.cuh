@@ -13,6 +13,8 @@
 //   cell2   lbm_step.wgsl:137-270 (step) + lbm_force.wgsl main
 #pragma once
 
+#include <type_traits>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -37,22 +39,34 @@ constexpr float kInvCS2 = 3.0f;
 template <typename S> struct Codec;
 template <> struct Codec<float> {
   static __device__ __forceinline__ float ld(const float *p, int, const Pack &) { return __ldg(p); }
+  static __device__ __forceinline__ float dec(float v, int, const Pack &) { return v; }
   static __device__ __forceinline__ void st(float *p, float v, int, const Pack &) {
     if (LBM_STREAMING_STORES) __stcs(p, v); else *p = v;
   }
 };
+// FP32 populations that other blocks of the same launch write (a persistent
+// kernel): read from L2.
+struct CgFloat {
+  float v;
+};
+template <> struct Codec<CgFloat> {
+  static __device__ __forceinline__ float ld(const CgFloat *p, int, const Pack &) { return __ldcg(&p->v); }
+  static __device__ __forceinline__ void st(CgFloat *p, float v, int, const Pack &) { p->v = v; }
+};
 template <> struct Codec<__half> {
-  static __device__ __forceinline__ float ld(const __half *p, int i, const Pack &k) {
-    return fmaf(__half2float(__ldg(p)), k.inv, k.off[i]);
+  static __device__ __forceinline__ float dec(__half v, int i, const Pack &k) {
+    return fmaf(__half2float(v), k.inv, k.off[i]);
   }
+  static __device__ __forceinline__ float ld(const __half *p, int i, const Pack &k) { return dec(__ldg(p), i, k); }
   static __device__ __forceinline__ void st(__half *p, float v, int i, const Pack &k) {
     *p = __float2half_rn(fmaf(v, k.scale, k.noff[i]));
   }
 };
 template <> struct Codec<__nv_bfloat16> {
-  static __device__ __forceinline__ float ld(const __nv_bfloat16 *p, int i, const Pack &k) {
-    return fmaf(__bfloat162float(__ldg(p)), k.inv, k.off[i]);
+  static __device__ __forceinline__ float dec(__nv_bfloat16 v, int i, const Pack &k) {
+    return fmaf(__bfloat162float(v), k.inv, k.off[i]);
   }
+  static __device__ __forceinline__ float ld(const __nv_bfloat16 *p, int i, const Pack &k) { return dec(__ldg(p), i, k); }
   static __device__ __forceinline__ void st(__nv_bfloat16 *p, float v, int i, const Pack &k) {
     *p = __float2bfloat16_rn(fmaf(v, k.scale, k.noff[i]));
   }
@@ -60,33 +74,66 @@ template <> struct Codec<__nv_bfloat16> {
 
 // ---- deterministic block reduction + last-block finish -------------------
 
+// The warp's sums of 8 values per lane: v8[lane % 8] of lane k holds value k's
+// sum, k = 0..7. Each of the first three rounds halves the values a lane
+// carries (it keeps one half and adds its partner's copy of it), so 9
+// exchanges do what 8 trees of 5 do, in a fixed order.
+__device__ __forceinline__ double warp_sum8(const double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  double a[4], b[2], c;
+  const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double keep = h4 ? v[k + 4] : v[k], give = h4 ? v[k] : v[k + 4];
+    a[k] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double keep = h2 ? a[k + 2] : a[k], give = h2 ? a[k] : a[k + 2];
+    b[k] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+  }
+  {
+    const double keep = h1 ? b[1] : b[0], give = h1 ? b[0] : b[1];
+    c = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+  }
+  c += __shfl_xor_sync(0xffffffffu, c, 8);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  return c;
+}
+
 template <int NV, int THREADS>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm) {
   constexpr int NW = THREADS / 32;
-#pragma unroll
-  for (int k = 0; k < NV; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0)
+  if constexpr (NV == 8) {
+    const double c = warp_sum8(v);
+    __syncthreads();
+    if (lane < 8) sm[lane * NW + warp] = c;
+  } else {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) sm[k * NW + warp] = v[k];
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sm[k * NW + warp] = v[k];
+  }
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       double t = lane < NW ? sm[k * NW + lane] : 0.0;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+      for (int o = 16; o > 0; o >>= 1)
+        if (o < NW) t += __shfl_down_sync(0xffffffffu, t, o);
       v[k] = t;
     }
   }
 }
 
 // The fixed-order sum of nparts partials by one warp (lane = threadIdx.x):
-// lane l adds partials l, l + 32, ... in order, then a shuffle tree; lane 0
-// writes out. Every caller that sums the same partials this way gets the
+// lane l adds partials l, l + 32, ... in order, then the warp's fixed tree. Every caller that sums the same partials this way gets the
 // same bits.
 template <int NV>
 __device__ __forceinline__ void sum_partials_warp(const double *partials, int nparts, double *out) {
@@ -97,13 +144,19 @@ __device__ __forceinline__ void sum_partials_warp(const double *partials, int np
   for (int j = lane; j < nparts; j += 32)
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] += __ldcg(&partials[(int64_t)j * NV + k]);
+  if constexpr (NV == 8) {
+    const double c = warp_sum8(acc);
+    if (lane < 8) out[lane] = c;
+    __syncwarp();  // lane 0 may read the whole sum next
+  } else {
 #pragma unroll
-  for (int k = 0; k < NV; ++k)
+    for (int k = 0; k < NV; ++k)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
-  if (lane == 0)
+      for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
+    if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < NV; ++k) out[k] = acc[k];
+      for (int k = 0; k < NV; ++k) out[k] = acc[k];
+  }
 }
 
 // Writes this block's partial (thread 0 holds it), and if this block is the
@@ -192,23 +245,38 @@ __device__ __forceinline__ void publish_force(const ForceAcc &a, double *partial
 }
 
 // The sum of a launch's force partials, spread over the first blocks of a
-// later launch so that no block waits on more than one round of loads:
-// block b adds the partials of group b (kSumGroup consecutive ones, one per
-// thread, then the block tree) into groups[b]; the last group to finish
-// (a ticket behind one fence per group, not per partial) sums the groups in
-// order into out. The order depends only on nparts, so every launch that
-// sums the same partials with THREADS = kSumGroup gets the same bits.
+// later launch so that no block waits on more than a round or two of loads:
+// up to kSumOne of them are one block's (one to four per thread, then the
+// block tree). More are cut into groups of kSumGroup: block b adds those of
+// group b, one per thread, into groups[b]; the last group to finish (a
+// ticket behind one fence per group, not per partial) sums the groups in
+// order into out. The order depends only on nparts (threads past kSumGroup
+// add zeros), so every launch that sums the same partials gets the same bits.
 template <int THREADS>
-__device__ __forceinline__ bool sum_partials_grouped(const double *partials, int nparts, double *groups,
+__device__ __forceinline__ void sum_partials_grouped(const double *partials, int nparts, double *groups,
                                                      unsigned int *counter, double *out, int b) {
-  static_assert(THREADS == kSumGroup, "one partial per thread");
+  static_assert(THREADS >= kSumGroup, "one partial per thread");
   __shared__ double sm[kForceSlots * (THREADS / 32)];
   double acc[kForceSlots];
   const int j = b * kSumGroup + (int)threadIdx.x;
+  const bool mine = threadIdx.x < kSumGroup && j < nparts;
 #pragma unroll
-  for (int k = 0; k < kForceSlots; ++k) acc[k] = j < nparts ? partials[(int64_t)j * kForceSlots + k] : 0.0;
+  for (int k = 0; k < kForceSlots; ++k) acc[k] = mine ? partials[(int64_t)j * kForceSlots + k] : 0.0;
+  if (nparts <= kSumOne) {
+    // no second level: no fence and no ticket
+    if (threadIdx.x < kSumGroup)
+#pragma unroll 1
+      for (int m = j + kSumGroup; m < nparts; m += kSumGroup)
+#pragma unroll
+        for (int k = 0; k < kForceSlots; ++k) acc[k] += partials[(int64_t)m * kForceSlots + k];
+    block_sum<kForceSlots, THREADS>(acc, sm);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < kForceSlots; ++k) out[k] = acc[k];
+    return;
+  }
   block_sum<kForceSlots, THREADS>(acc, sm);
-  return finish_sum<kForceSlots, THREADS>(acc, groups, counter, sum_groups(nparts), b, out, sm);
+  finish_sum<kForceSlots, THREADS>(acc, groups, counter, sum_groups(nparts), b, out, sm);
 }
 
 // Returns true in the block that summed the partials (the last to finish).
@@ -223,6 +291,22 @@ __device__ __forceinline__ bool reduce_force(const ForceAcc &a, double *partials
   v[7] = 0.0;
   block_sum<kForceSlots, THREADS>(v, sm);
   return finish_sum<kForceSlots, THREADS>(v, partials, counter, nparts, part, out, sm);
+}
+
+// Cell `cell` of a plane. 16-bit storage addresses it by a 32-bit byte offset
+// from the plane's base, which is the same for the whole block (a plane of
+// fewer than 2^31 cells has fewer than 2^32 bytes): its step is bound by
+// instruction issue, and a 64-bit address per population was a fifth of it
+// (256x128x128 sphere, 104.6 -> 99.2 us per step; D3Q27 150.9 -> 137.3). FP32
+// planes can be larger, and their step is bound by memory (103.6 against
+// 104.4 us with the offsets).
+template <typename S> __device__ __forceinline__ S *plane_cell(S *plane, int cell) {
+  if constexpr (sizeof(S) == 2) {
+    using B = std::conditional_t<std::is_const_v<S>, const char, char>;
+    return reinterpret_cast<S *>(reinterpret_cast<B *>(plane) + (size_t)((unsigned)cell * 2u));
+  } else {
+    return plane + cell;
+  }
 }
 
 // The BGK collision with Guo forcing and the sponge blend, written over
@@ -245,7 +329,7 @@ template <typename S> struct MemSink {
   int64_t n;
   int cell;
   const Pack &pk;
-  __device__ __forceinline__ void put(int i, float v) { Codec<S>::st(fo + (int64_t)i * n + cell, v, i, pk); }
+  __device__ __forceinline__ void put(int i, float v) { Codec<S>::st(plane_cell(fo + (int64_t)i * n, cell), v, i, pk); }
 };
 struct NullSink {
   __device__ __forceinline__ void put(int, float) {}
@@ -260,51 +344,77 @@ struct NullSink {
 // the negative. TRT = false is the BGK loop alone (dw ignored); the kernels
 // pick the instantiation from dw != 0 per launch, so the BGK code keeps its
 // register allocation.
+//
+// Every operation is explicit (no contraction left to the compiler), so that
+// a cell's bits do not depend on the kernel it is updated in. Only the
+// nonzero components of e enter e.u and e.F (edot): written as ex*ux + ey*uy
+// + ez*uz the products with 0 stay in the code (0 * NaN is not 0), two of
+// them per direction pair and dot product.
+__device__ __forceinline__ float edot(int ex, int ey, int ez, float x, float y, float z) {
+  float v = x;
+  bool have = ex != 0, neg = ex < 0;
+  if (ey) {
+    if (!have) { v = y; neg = ey < 0; }
+    else if ((ey < 0) == neg) v = __fadd_rn(v, y);
+    else if (neg) { v = __fsub_rn(y, v); neg = false; }
+    else v = __fsub_rn(v, y);
+    have = true;
+  }
+  if (ez) {
+    if (!have) { v = z; neg = ez < 0; }
+    else if ((ez < 0) == neg) v = __fadd_rn(v, z);
+    else if (neg) { v = __fsub_rn(z, v); neg = false; }
+    else v = __fsub_rn(v, z);
+  }
+  return neg ? -v : v;
+}
+
 template <class L, int Q, class Sink, bool TRT = false>
 __device__ __forceinline__ void collide_store(const float (&f)[Q], float rho, float ux, float uy, float uz, float Fx,
                                               float Fy, float Fz, float omg, float spw, const float *ftarget,
                                               Sink &sink, float dw = 0.f) {
-  const float usq = ux * ux + uy * uy + uz * uz;
-  const float uF = ux * Fx + uy * Fy + uz * Fz;
-  const float ks = 1.0f - spw;
-  const float a = (omg * ks) * rho;
-  const float b = (1.0f - 0.5f * omg) * ks;
-  const float keep = (1.0f - omg) * ks;
-  const float c0 = fmaf(a, fmaf(-1.5f, usq, 1.0f), -3.0f * b * uF);
-  sink.put(0, fmaf(keep, f[0], fmaf(spw, ftarget[0], L::w(0) * c0)));
-  if (!TRT) {
+  float usq = __fmaf_rn(ux, ux, __fmul_rn(uy, uy));
+  float uF = __fmaf_rn(ux, Fx, __fmul_rn(uy, Fy));
+  if (L::D == 3) {
+    usq = __fmaf_rn(uz, uz, usq);
+    uF = __fmaf_rn(uz, Fz, uF);
+  }
+  const float ks = __fsub_rn(1.0f, spw);
+  const float a = __fmul_rn(__fmul_rn(omg, ks), rho);
+  const float b = __fmul_rn(__fmaf_rn(-0.5f, omg, 1.0f), ks);
+  const float keep = __fmul_rn(__fsub_rn(1.0f, omg), ks);
+  const float c0 = __fmaf_rn(a, __fmaf_rn(-1.5f, usq, 1.0f), __fmul_rn(__fmul_rn(-3.0f, b), uF));
+  auto blend = [&](int i, float v) { return __fmaf_rn(spw, ftarget[i], v); };
+  sink.put(0, __fmaf_rn(keep, f[0], blend(0, __fmul_rn(L::w(0), c0))));
+  const float kd = TRT ? __fmul_rn(ks, -dw) : 0.f, nrho3 = TRT ? __fmul_rn(-3.0f, rho) : 0.f;
+  float a45, b9, a3, b3, wc0;  // per weight class, the classes in direction order
 #pragma unroll
-    for (int i = 1; i < Q; ++i) {
-      const int j = L::opp(i);
-      if (j < i) continue;
-      const float ex = (float)L::ex(i), ey = (float)L::ey(i), ez = (float)L::ez(i);
-      const float w = L::w(i);
-      const float eu = ex * ux + ey * uy + ez * uz;
-      const float eF = ex * Fx + ey * Fy + ez * Fz;
-      const float t = fmaf((9.0f * w) * b, eF, ((4.5f * w) * a) * eu);
-      const float A = fmaf(eu, t, w * c0);
-      const float B = fmaf((3.0f * w) * a, eu, ((3.0f * w) * b) * eF);
-      sink.put(i, fmaf(keep, f[i], fmaf(spw, ftarget[i], A + B)));
-      sink.put(j, fmaf(keep, f[j], fmaf(spw, ftarget[j], A - B)));
+  for (int i = 1; i < Q; ++i) {
+    const int j = L::opp(i);
+    const float w = L::w(i);
+    if (i == 1 || L::w(i) != L::w(i - 1)) {
+      a45 = __fmul_rn(4.5f * w, a);
+      b9 = __fmul_rn(9.0f * w, b);
+      a3 = __fmul_rn(3.0f * w, a);
+      b3 = __fmul_rn(3.0f * w, b);
+      wc0 = __fmul_rn(w, c0);
     }
-  } else {
-    const float kd = -ks * dw;
-    const float rho3 = 3.0f * rho;
-#pragma unroll
-    for (int i = 1; i < Q; ++i) {
-      const int j = L::opp(i);
-      if (j < i) continue;
-      const float ex = (float)L::ex(i), ey = (float)L::ey(i), ez = (float)L::ez(i);
-      const float w = L::w(i);
-      const float eu = ex * ux + ey * uy + ez * uz;
-      const float eF = ex * Fx + ey * Fy + ez * Fz;
-      const float t = fmaf((9.0f * w) * b, eF, ((4.5f * w) * a) * eu);
-      const float A = fmaf(eu, t, w * c0);
-      const float B = fmaf((3.0f * w) * a, eu, ((3.0f * w) * b) * eF);
-      const float D = kd * fmaf(0.5f, f[i] - f[j], w * fmaf(1.5f, eF, -rho3 * eu));
-      sink.put(i, fmaf(keep, f[i], fmaf(spw, ftarget[i], A + B)) + D);
-      sink.put(j, fmaf(keep, f[j], fmaf(spw, ftarget[j], A - B)) - D);
+    if (j < i) continue;
+    const float eu = edot(L::ex(i), L::ey(i), L::ez(i), ux, uy, uz);
+    const float eF = edot(L::ex(i), L::ey(i), L::ez(i), Fx, Fy, Fz);
+    const float t = __fmaf_rn(b9, eF, __fmul_rn(a45, eu));
+    const float A = __fmaf_rn(eu, t, wc0);
+    const float B = __fmaf_rn(a3, eu, __fmul_rn(b3, eF));
+    float oi = __fmaf_rn(keep, f[i], blend(i, __fadd_rn(A, B)));
+    float oj = __fmaf_rn(keep, f[j], blend(j, __fsub_rn(A, B)));
+    if (TRT) {
+      const float odd = __fmul_rn(w, __fmaf_rn(1.5f, eF, __fmul_rn(nrho3, eu)));
+      const float D = __fmaf_rn(0.5f, __fsub_rn(f[i], f[j]), odd);
+      oi = __fmaf_rn(kd, D, oi);
+      oj = __fmaf_rn(-kd, D, oj);
     }
+    sink.put(i, oi);
+    sink.put(j, oj);
   }
 }
 
@@ -313,21 +423,22 @@ template <class L, int Q>
 __device__ __forceinline__ void moments(const float (&f)[Q], float &rho, float &mx, float &my, float &mz) {
   rho = f[0];
   mx = my = mz = 0.f;
+  bool hx = false, hy = false, hz = false;  // whether a sum has begun (compile-time)
 #pragma unroll
   for (int i = 1; i < Q; ++i) {
     const int j = L::opp(i);
     if (j < i) continue;
     const float s = f[i] + f[j], d = f[i] - f[j];
     rho += s;
-    if (L::ex(i) == 1) mx += d; else if (L::ex(i) == -1) mx -= d;
-    if (L::ey(i) == 1) my += d; else if (L::ey(i) == -1) my -= d;
-    if (L::ez(i) == 1) mz += d; else if (L::ez(i) == -1) mz -= d;
+    if (L::ex(i)) { mx = L::ex(i) > 0 ? (hx ? mx + d : d) : mx - d; hx = true; }
+    if (L::ey(i)) { my = L::ey(i) > 0 ? (hy ? my + d : d) : my - d; hy = true; }
+    if (L::ez(i)) { mz = L::ez(i) > 0 ? (hz ? mz + d : d) : mz - d; hz = true; }
   }
 }
 
 __device__ __forceinline__ float sponge_weight_inv(float d, float inv_sw) {
-  float w = fminf(fmaxf(1.0f - d * inv_sw, 0.0f), 1.0f);
-  return w * w * (3.0f - 2.0f * w);
+  const float w = fminf(fmaxf(__fmaf_rn(-d, inv_sw, 1.0f), 0.0f), 1.0f);
+  return __fmul_rn(__fmul_rn(w, w), __fmaf_rn(-2.0f, w, 3.0f));
 }
 
 // ---- row-major walks without divisions --------------------------------------
@@ -358,6 +469,83 @@ struct CellWalk {
   }
 };
 
+// The D3Q27 directions (D3Q19 their first 19), as a table in constant
+// memory for loops over a runtime direction index.
+struct DirTable {
+  signed char ex[27], ey[27], ez[27];
+};
+constexpr DirTable make_dirs() {
+  DirTable t{};
+  for (int i = 0; i < 27; ++i) {
+    t.ex[i] = (signed char)detail::ex27(i);
+    t.ey[i] = (signed char)detail::ey27(i);
+    t.ez[i] = (signed char)detail::ez27(i);
+  }
+  return t;
+}
+static __constant__ DirTable c_dirs = make_dirs();
+
+// The directions of a cell at pos whose pull source lies inside the body, as
+// phi3 < 0 decides.
+//  * Sphere: phi3 < 0 is sqrt(d^2) < a, and as the square root rounds
+//    monotonically that is d^2 < a2, the smallest number whose root reaches
+//    a (p.ball2). With the squares of the three offsets per axis shared, a
+//    link costs two additions and a comparison instead of a square root of
+//    its own: 18 roots were most of a near cell's time.
+//  * Box and spheroid: from the source's position in the body's frame, the
+//    cell's less a combination of the frame's columns, so a link costs no
+//    rotation: the spheroid's side of its equation rr = 1 needs no Newton
+//    step, the box's distance no call. That position is rounded differently
+//    from phi3's, so where the outcome is within a margin far above the
+//    rounding (1e-3), phi3 itself decides.
+template <int Q>
+static __device__ __noinline__ unsigned solid_links_call(float x, float y, float z, const lbm_body *b, const Win *w) {
+  const Q4 q = {b->qw, b->qx, b->qy, b->qz};
+  const V3 l0 = q_rot_inv(q, body_delta({x, y, z}, *b, *w));
+  const V3 cx = q_rot_inv(q, {1.f, 0.f, 0.f}), cy = q_rot_inv(q, {0.f, 1.f, 0.f}), cz = q_rot_inv(q, {0.f, 0.f, 1.f});
+  const bool spheroid = b->shape == LBM_SHAPE_SPHEROID, box = b->shape == LBM_SHAPE_ROUNDBOX;
+  const float ia2 = 1.f / (b->a * b->a), ic2 = 1.f / (b->c * b->c);
+  unsigned solid = 0u;
+#pragma unroll 1
+  for (int i = 1; i < Q; ++i) {
+    const float ex = (float)c_dirs.ex[i], ey = (float)c_dirs.ey[i], ez = (float)c_dirs.ez[i];
+    const V3 l = {l0.x - (ex * cx.x + ey * cy.x + ez * cz.x), l0.y - (ex * cx.y + ey * cy.y + ez * cz.y),
+                  l0.z - (ex * cx.z + ey * cy.z + ez * cz.z)};
+    float d = 0.f;  // its sign, where |d| is above the margin
+    if (spheroid) {
+      d = (l.x * l.x + l.y * l.y) * ia2 + l.z * l.z * ic2 - 1.f;
+    } else if (box) {
+      const float hx = fabsf(l.x) - (b->a - b->r), hy = fabsf(l.y) - (b->b - b->r), hz = fabsf(l.z) - (b->c - b->r);
+      const float mx = fmaxf(hx, 0.f), my = fmaxf(hy, 0.f), mz = fmaxf(hz, 0.f);
+      d = sqrtf(mx * mx + my * my + mz * mz) + fminf(fmaxf(hx, fmaxf(hy, hz)), 0.f) - b->r;
+    }
+    // (a moving window takes the source's own nearest image: phi3 decides)
+    const bool cut = fabsf(d) > 1e-3f && !w->on ? d < 0.f : phi3_call(x - ex, y - ey, z - ez, b, w) < 0.f;
+    solid |= cut ? 1u << i : 0u;
+  }
+  return solid;
+}
+
+template <int Q>
+__device__ __forceinline__ unsigned solid_links(const StepParams &p, const V3 &pos) {
+  using L = Lattice<Q>;
+  if (p.body.shape != LBM_SHAPE_SPHERE || p.win.on) return solid_links_call<Q>(pos.x, pos.y, pos.z, &p.body, &p.win);
+  unsigned solid = 0u;
+  float xx[3], yy[3], zz[3];  // of the sources at e = -1, 0, +1
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const float o = (float)(e - 1);
+    const float dx = (pos.x - o) - p.body.cx, dy = (pos.y - o) - p.body.cy, dz = (pos.z - o) - p.body.cz;
+    xx[e] = __fmul_rn(dx, dx);
+    yy[e] = __fmul_rn(dy, dy);
+    zz[e] = __fmul_rn(dz, dz);
+  }
+#pragma unroll
+  for (int i = 1; i < Q; ++i)
+    if (__fadd_rn(__fadd_rn(xx[L::ex(i) + 1], yy[L::ey(i) + 1]), zz[L::ez(i) + 1]) < p.ball2) solid |= 1u << i;
+  return solid;
+}
+
 // ---- 3D cell update ---------------------------------------------------------
 // Pull-stream (periodic sources, then bounce-back patches: body first with
 // Ladd's correction at local rho_w, then walls), moments, Guo forcing with
@@ -365,24 +553,24 @@ struct CellWalk {
 // (the caller's block can see the body) the cell's force/torque contribution
 // is returned in cf.
 
-// Everything after the pull gather, for one cell: bounce-back patches,
-// moments, forcing, collision into `sink`, mac, force. `fi` is the domain's
-// base in the input arena (own-cell loads of the bounce-back patches).
-template <int Q, typename S, class Sink, bool TRT = false>
-__device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[Q], float *__restrict__ mac,
-                                           const StepParams &p, int x, int y, int z, bool force, CellForce &cf,
-                                           Sink &sink) {
+// What the body and the walls mean for a cell: its distance, the body's
+// velocity there, whether it is held at the body's state (SOLID_EQ), and the
+// links to patch. Decided before the gather is issued: a body's links may
+// take a call, which would have to save the populations in flight.
+struct Geom3 {
+  float phi;
+  V3 us;
+  unsigned solid, wall;
+  bool in_solid;
+};
+
+// (x, y, z): the cell in the domain's own coordinates.
+template <int Q>
+__device__ __forceinline__ Geom3 classify3(const StepParams &p, int x, int y, int z) {
   using L = Lattice<Q>;
-  // z indexes the stored planes; the physics (body, walls, sponge, reach
-  // box) sees the domain's own z, which for a slab is offset by p.zoff in a
-  // domain p.nzg planes deep (both the identity for a whole domain)
   const int nx = p.nx, ny = p.ny, nz = p.nzg;
-  const int64_t n = p.n;
-  const int cell = (z * ny + y) * nx + x;
-  z += p.zoff;
   const V3 pos = {(float)x, (float)y, (float)z};
-  float phi = 1e30f;
-  V3 us = {0.f, 0.f, 0.f};
+  Geom3 g{1e30f, {0.f, 0.f, 0.f}, 0u, 0u, false};
   bool see = p.has_body;
   if (see && p.nbox_on) {
     int dx = x - p.nbox[0], dy = y - p.nbox[2], dz = z - p.nbox[4];
@@ -392,36 +580,57 @@ __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[
     see = dx <= p.nbox[1] - p.nbox[0] && dy <= p.nbox[3] - p.nbox[2] && dz <= p.nbox[5] - p.nbox[4];
   }
   if (see) {
-    phi = phi3(pos, p.body, p.win);
-    us = body_velocity3(pos, p.body, p.win);
+    g.phi = phi3(pos, p.body, p.win);
+    g.us = body_velocity3(pos, p.body, p.win);
   }
   const bool bbody = p.has_body && p.bb;
+  // A cell held at the body's state uses nothing it pulls, so its links need
+  // no patch. For the others a link reaches a solid source only from within
+  // |e| <= sqrt(3) of the surface, as a signed distance is 1-Lipschitz.
+  g.in_solid = p.solid_eq && bbody && g.phi < 0.f;
+  if (g.in_solid) return g;
+  if (bbody && g.phi < 2.5f) g.solid = solid_links<Q>(p, pos);
   const bool at_wall = (p.wall_x && (x == 0 || x == nx - 1)) || (p.wall_y && (y == 0 || y == ny - 1)) ||
                        (p.wall_z && (z == 0 || z == nz - 1));
-  // A link reaches a solid source only from within |e| <= sqrt(3) of the
-  // surface, and a signed distance is 1-Lipschitz.
-  const bool near = bbody && phi < 2.5f;
-  float fbx = 0.f, fby = 0.f, fbz = 0.f;
-
-  // 1b. Bounce-back links. Every link is classified first (SDF and wall
-  // tests, no memory access), then the cell's own populations that the
-  // patches read are loaded together: a near cell waits for one memory
-  // latency instead of one per solid link. (The rest direction never
-  // patches: its source is the cell itself.)
-  if (near || at_wall) {
-    unsigned solid = 0u, wall = 0u;
+  if (at_wall) {
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
-      const int ex = L::ex(i), ey = L::ey(i), ez = L::ez(i);
-      if (near && phi3({pos.x - (float)ex, pos.y - (float)ey, pos.z - (float)ez}, p.body, p.win) < 0.f) {
-        solid |= 1u << i;
-      } else if (at_wall) {
-        const int sx = x - ex, sy = y - ey, sz = z - ez;
-        const bool out = (p.wall_x && (sx < 0 || sx >= nx)) || (p.wall_y && (sy < 0 || sy >= ny)) ||
-                         (p.wall_z && (sz < 0 || sz >= nz));
-        if (out) wall |= 1u << i;
-      }
+      const int sx = x - L::ex(i), sy = y - L::ey(i), sz = z - L::ez(i);
+      const bool out = (p.wall_x && (sx < 0 || sx >= nx)) || (p.wall_y && (sy < 0 || sy >= ny)) ||
+                       (p.wall_z && (sz < 0 || sz >= nz));
+      if (out) g.wall |= 1u << i;
     }
+  }
+  return g;
+}
+
+// Everything after the pull gather, for one cell: bounce-back patches,
+// moments, forcing, collision into `sink`, mac, force. `fi` is the domain's
+// base in the input arena (own-cell loads of the bounce-back patches).
+template <int Q, typename S, class Sink, bool TRT = false>
+__device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[Q], float *__restrict__ mac,
+                                           const StepParams &p, const Geom3 &g, int x, int y, int z, bool force,
+                                           CellForce &cf, Sink &sink) {
+  using L = Lattice<Q>;
+  // z indexes the stored planes; the physics (body, walls, sponge, reach
+  // box) sees the domain's own z, which for a slab is offset by p.zoff in a
+  // domain p.nzg planes deep (both the identity for a whole domain)
+  const int nx = p.nx, ny = p.ny, nz = p.nzg;
+  const int64_t n = p.n;
+  const int cell = (z * ny + y) * nx + x;
+  z += p.zoff;
+  const V3 pos = {(float)x, (float)y, (float)z};
+  const float phi = g.phi;
+  const V3 us = g.us;
+  const unsigned solid = g.solid, wall = g.wall;
+  const bool bbody = p.has_body && p.bb, in_solid = g.in_solid;
+  float fbx = 0.f, fby = 0.f, fbz = 0.f;
+
+  // 1b. Bounce-back links, all classified already (classify3): the cell's own
+  // populations that the patches read are loaded together, so a near cell
+  // waits for one memory latency instead of one per solid link. (The rest
+  // direction never patches: its source is the cell itself.)
+  {
     if (solid | wall) {
       const bool all = bbody && p.rho_w_local && phi < 2.f;  // rho_w sums every population
       float own[Q];
@@ -467,9 +676,9 @@ __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[
   // 3. Solid coupling and Guo forcing: u = u* + F / (2 rho).
   const float chi = (p.has_body && !p.bb) ? chi_from_phi(phi, p.chi_eps) : 0.f;
   const float rc = rho * chi;
-  const float Fx = rc * (us.x - uxs) + p.fx;
-  const float Fy = rc * (us.y - uys) + p.fy;
-  const float Fz = rc * (us.z - uzs) + p.fz;
+  const float Fx = __fmaf_rn(rc, us.x - uxs, p.fx);
+  const float Fy = __fmaf_rn(rc, us.y - uys, p.fy);
+  const float Fz = __fmaf_rn(rc, us.z - uzs, p.fz);
   const float hinv = 0.5f * inv;
   const float ux = fmaf(Fx, hinv, uxs);
   const float uy = fmaf(Fy, hinv, uys);
@@ -492,7 +701,6 @@ __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[
   }
 
   // 4. Collide + sponge blend, 5. solid interior held at feq(1, u_body).
-  const bool in_solid = p.solid_eq && bbody && phi < 0.f;
   if (!in_solid) {
     collide_store<L, Q, Sink, TRT>(f, rho, ux, uy, uz, Fx, Fy, Fz, p.omega, spw, p.ftarget, sink, p.trt_dw);
   } else {
@@ -565,7 +773,7 @@ __device__ __forceinline__ void gather3(const S *__restrict__ fi, const StepPara
     const int ex = L::ex(i), ey = L::ey(i), ez = L::ez(i);
     const int off = (ex == 1 ? xo_p : (ex == -1 ? xo_m : 0)) + (ey == 1 ? yo_p : (ey == -1 ? yo_m : 0)) +
                     (ez == 1 ? zo_p : (ez == -1 ? zo_m : 0));
-    f[i] = Codec<S>::ld(fi + (int64_t)i * n + (cell + off), i, p.pk);
+    f[i] = Codec<S>::ld(plane_cell(fi + (int64_t)i * n, cell + off), i, p.pk);
   }
 }
 
@@ -576,10 +784,11 @@ __device__ __forceinline__ void cell3(const S *__restrict__ fin, S *__restrict__
                                       float *__restrict__ mac, const StepParams &p, int x, int y,
                                       int z, bool force, CellForce &cf) {
   const S *fi = fin + p.base;
+  const Geom3 g = classify3<Q>(p, x, y, z + p.zoff);
   float f[Q];
   gather3<Q, S>(fi, p, x, y, z, f);
   MemSink<S> sink{fout + p.base, p.n, (z * p.ny + y) * p.nx + x, p.pk};
-  cell3_core<Q, S, MemSink<S>, TRT>(fi, f, mac, p, x, y, z, force, cf, sink);
+  cell3_core<Q, S, MemSink<S>, TRT>(fi, f, mac, p, g, x, y, z, force, cf, sink);
 }
 
 // cell3 with the collision picked from the launch's parameters (a
@@ -634,10 +843,11 @@ template <int Q, typename S>
 __device__ __forceinline__ void cell3_force(const S *__restrict__ fin, const StepParams &p, int x, int y, int z,
                                             CellForce &cf) {
   const S *fi = fin + p.base;
+  const Geom3 g = classify3<Q>(p, x, y, z + p.zoff);
   float f[Q];
   gather3<Q, S>(fi, p, x, y, z, f);
   NullSink sink;
-  cell3_core<Q, S>(fi, f, nullptr, p, x, y, z, true, cf, sink);
+  cell3_core<Q, S>(fi, f, nullptr, p, g, x, y, z, true, cf, sink);
 }
 
 // ---- 2D cell update (D2Q9) ---------------------------------------------------
@@ -688,11 +898,16 @@ __device__ __forceinline__ void cell2_core(const S *__restrict__ fin, float (&f)
   const float fW = (float)W, fH = (float)H;
   const float px = (float)x, py = (float)y;
   float rx = 0.f, ry = 0.f, usx = 0.f, usy = 0.f, phi = 1e30f;
-  if (p.has_body) {
+  // outside the reach box (p.nbox) no link ends in the body and chi is 0:
+  // the distance (two divisions, a square root, for an ellipse the Newton
+  // steps) is not evaluated there
+  bool see = p.has_body;
+  if (see && p.nbox_on) see = x >= p.nbox[0] && x <= p.nbox[1] && y >= p.nbox[2] && y <= p.nbox[3];
+  if (see) {
     rx = wrap_delta(px - p.body.cx, fW);
     ry = wrap_delta(py - p.body.cy, fH);
-    usx = p.body.vx - p.body.wz * ry;
-    usy = p.body.vy + p.body.wz * rx;
+    usx = __fmaf_rn(-p.body.wz, ry, p.body.vx);
+    usy = __fmaf_rn(p.body.wz, rx, p.body.vy);
     phi = phi2(px, py, p.body, fW, fH);
   }
   const bool bbody = p.has_body && p.bb;
@@ -702,30 +917,56 @@ __device__ __forceinline__ void cell2_core(const S *__restrict__ fin, float (&f)
   if (near || at_wall) {
     const int xm = x == 0 ? W - 1 : x - 1, xp = x == W - 1 ? 0 : x + 1;
     const int ym = y == 0 ? H - 1 : y - 1, yp = y == H - 1 ? 0 : y + 1;
+    // Every link is classified first, then the cell's own populations that the
+    // patches read are loaded together: a warp of near cells, whose links
+    // differ from lane to lane, waits for one memory latency instead of one
+    // per direction. An unrotated circle's links are found as the sphere's
+    // (solid_links): squares shared, compared with p.ball2.
+    unsigned solid = 0u, wall = 0u;
+    if (near && phi2_is_circle(p.body)) {
+      float xx[3], yy[3];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      const int ex = L::ex(i), ey = L::ey(i), o = L::opp(i);
-      bool solid = false;
-      if (near) {
-        const int sx = ex == 1 ? xm : (ex == -1 ? xp : x);
-        const int sy = ey == 1 ? ym : (ey == -1 ? yp : y);
-        solid = phi2((float)sx, (float)sy, p.body, fW, fH) < 0.f;
+      for (int e = 0; e < 3; ++e) {
+        const float dx = wrap_delta((float)(e == 2 ? xm : (e == 0 ? xp : x)) - p.body.cx, fW);
+        const float dy = wrap_delta((float)(e == 2 ? ym : (e == 0 ? yp : y)) - p.body.cy, fH);
+        xx[e] = __fmul_rn(dx, dx);
+        yy[e] = __fmul_rn(dy, dy);
       }
-      if (solid) {
-        const float fopp = Codec<S>::ld(fi + (int64_t)o * n + cell, o, p.pk);
-        const float corr = 2.f * L::w(i) * ((float)ex * usx + (float)ey * usy) * kInvCS2;
-        f[i] = fopp + corr;
-        if (phi >= 0.f) {
-          const float m = 2.f * fopp + corr;
-          fbx += -(float)ex * m;
-          fby += -(float)ey * m;
-        }
-      } else if (at_wall) {
-        const int ysrc = y - ey;
-        if (ysrc < 0 || ysrc >= H) {
-          const float wu = ysrc < 0 ? p.wall_u0 : p.wall_u1;
-          const float corr = 2.f * L::w(i) * (float)ex * wu * kInvCS2;
-          f[i] = Codec<S>::ld(fi + (int64_t)o * n + cell, o, p.pk) + corr;
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        if (__fadd_rn(xx[L::ex(i) + 1], yy[L::ey(i) + 1]) < p.ball2) solid |= 1u << i;
+    } else if (near) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const int sx = L::ex(i) == 1 ? xm : (L::ex(i) == -1 ? xp : x);
+        const int sy = L::ey(i) == 1 ? ym : (L::ey(i) == -1 ? yp : y);
+        if (phi2((float)sx, (float)sy, p.body, fW, fH) < 0.f) solid |= 1u << i;
+      }
+    }
+    if (at_wall) {
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        if (y - L::ey(i) < 0 || y - L::ey(i) >= H) wall |= 1u << i;
+    }
+    if (solid | wall) {
+      float own[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i)
+        own[i] = ((solid | wall) >> L::opp(i)) & 1u ? Codec<S>::ld(fi + (int64_t)i * n + cell, i, p.pk) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const float ex = (float)L::ex(i), ey = (float)L::ey(i), fopp = own[L::opp(i)];
+        if ((solid >> i) & 1u) {
+          const float corr = __fmul_rn(2.f * L::w(i) * (ex * usx + ey * usy), kInvCS2);
+          f[i] = __fadd_rn(fopp, corr);
+          if (phi >= 0.f) {
+            const float m = __fmaf_rn(2.f, fopp, corr);
+            fbx += -ex * m;
+            fby += -ey * m;
+          }
+        } else if ((wall >> i) & 1u) {
+          const float corr = __fmul_rn(2.f * L::w(i) * ex * (y - L::ey(i) < 0 ? p.wall_u0 : p.wall_u1), kInvCS2);
+          f[i] = __fadd_rn(fopp, corr);
         }
       }
     }
@@ -735,7 +976,7 @@ __device__ __forceinline__ void cell2_core(const S *__restrict__ fin, float (&f)
   const float rhoDen = fmaxf(rho, 1e-6f);
   const float inv = 1.0f / rhoDen;
   const float uxs = mxs * inv, uys = mys * inv;
-  const float chi = (p.has_body && !p.bb) ? chi_from_phi(phi, p.chi_eps) : 0.f;
+  const float chi = (see && !p.bb) ? chi_from_phi(phi, p.chi_eps) : 0.f;
   const float Fx = rho * chi * (usx - uxs) + p.fx;
   const float Fy = rho * chi * (usy - uys) + p.fy;
   const float hinv = 0.5f * inv;
@@ -761,10 +1002,10 @@ __device__ __forceinline__ void cell2_core(const S *__restrict__ fin, float (&f)
       Codec<S>::st(fo_ + (int64_t)i * n + cell, w * 1.0f * (1.f + 3.f * eu + 4.5f * eu * eu - 1.5f * ussq), i, p.pk);
     }
   }
-  if (p.write_mac) reinterpret_cast<float4 *>(mac + 4 * p.base)[cell] = make_float4(rho, ux, uy, 0.f);
+  if (p.write_mac && mac) reinterpret_cast<float4 *>(mac + 4 * p.base)[cell] = make_float4(rho, ux, uy, 0.f);
 
   if (force) {
-    if (!bbody && p.has_body) {
+    if (!bbody && see) {
       const float c2 = chi_from_phi(phi, p.chi_eps);
       if (c2 >= 1e-6f) {
         fbx = -(rho * c2 * (usx - uxs));
@@ -775,6 +1016,52 @@ __device__ __forceinline__ void cell2_core(const S *__restrict__ fin, float (&f)
     cf.fy = fby;
     cf.tz = rx * fby - ry * fbx;
   }
+}
+
+// One D2Q9 cell that no body reaches, outside any force region:
+// cell2_core with the tests that cannot fire taken out (no solid link,
+// chi = 0 and u_s = 0, so the Guo force is the body force) and only the
+// moving-wall patch of a wall row kept, the same arithmetic in the same
+// order, so the same bits.
+template <typename S>
+__device__ __forceinline__ void cell2_fluid(const S *__restrict__ fin, float (&f)[9], S *__restrict__ fout,
+                                            float *__restrict__ mac, const StepParams &p, int x, int y) {
+  using L = Lattice<9>;
+  const int W = p.nx, H = p.ny;
+  const int cell = y * W + x;
+  if (p.wall_y && (y == 0 || y == H - 1)) {
+    const S *fi = fin + p.base;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+      const int ex = L::ex(i), ey = L::ey(i), o = L::opp(i);
+      const int ysrc = y - ey;
+      if (ysrc < 0 || ysrc >= H) {
+        const float wu = ysrc < 0 ? p.wall_u0 : p.wall_u1;
+        const float corr = __fmul_rn(2.f * L::w(i) * (float)ex * wu, kInvCS2);
+        f[i] = __fadd_rn(Codec<S>::ld(fi + (int64_t)o * p.n + cell, o, p.pk), corr);
+      }
+    }
+  }
+  float rho, mxs, mys, mzs;
+  moments<L, 9>(f, rho, mxs, mys, mzs);
+  const float rhoDen = fmaxf(rho, 1e-6f);
+  const float inv = 1.0f / rhoDen;
+  const float uxs = mxs * inv, uys = mys * inv;
+  const float chi = 0.f, usx = 0.f, usy = 0.f;
+  const float Fx = rho * chi * (usx - uxs) + p.fx;
+  const float Fy = rho * chi * (usy - uys) + p.fy;
+  const float hinv = 0.5f * inv;
+  const float ux = fmaf(Fx, hinv, uxs);
+  const float uy = fmaf(Fy, hinv, uys);
+  float spw = 0.f;
+  if (p.sponge_w > 0.f) {
+    const float dx = fminf((float)x, (float)(W - 1 - x));
+    const float dy = fminf((float)y, (float)(H - 1 - y));
+    spw = sponge_weight_inv(fminf(dx, dy), p.sponge_inv);
+  }
+  MemSink<S> sink{fout + p.base, p.n, cell, p.pk};
+  collide_store<L, 9>(f, rho, ux, uy, 0.f, Fx, Fy, 0.f, p.omega, spw, p.ftarget, sink);
+  if (p.write_mac) reinterpret_cast<float4 *>(mac + 4 * p.base)[cell] = make_float4(rho, ux, uy, 0.f);
 }
 
 }  // namespace lbm

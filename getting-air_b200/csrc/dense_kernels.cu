@@ -34,98 +34,18 @@
 // every step costs its launch gaps (measured at 256x128x128: +9 %, +10 %
 // and +7 % of the step against no force at all, and +1 % for this form).
 
-#include <type_traits>
-#include <utility>
+#include <algorithm>
 
-#include "cell_update.cuh"
+#include "dense_block.cuh"
 
 namespace lbm {
 
 namespace {
 
 // ---- dense fused steps -------------------------------------------------------
-// One thread per cell, kStepThreads (64) cells of a row per CTA, grid
-// (NX/64, NY, NZ): the row and plane come straight from blockIdx, no
-// division.
-
-// The previous step's force, in this launch's first blocks (before their
-// own cells, so that the group's fence has no stores of theirs to wait on).
-__device__ __forceinline__ void sum_previous(const StepParams &p) {
-  const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  if (p.prev_parts && b < sum_groups(p.prev_parts))
-    sum_partials_grouped<kStepThreads>(p.prev_partials, p.prev_parts, p.groups, p.counter, p.force_out, b);
-}
-
-// Whether a cell of [lo, hi] lies in the interval [a, a + len] read modulo
-// n (a in [0, n); len < 0 is empty): the reach-box test of cell3_core for a
-// whole span of cells.
-__device__ __forceinline__ bool span_hits(int lo, int hi, int a, int len, int n) {
-  if (len >= n - 1) return true;
-  const int b = a + len;
-  return (lo <= b && hi >= a) || (lo + n <= b && hi + n >= a);
-}
-
-// What a launch block of the 3D step must evaluate, decided once per block
-// (warp-uniform): kGeneral runs cell3 for every cell; kFluid runs
-// cell3_fluid, for blocks that take no part in the force reduction, have no
-// cell within reach of a bounce-back body (or no body), touch no wall and
-// are not windowed. Penalty bodies reach every cell through chi and always
-// take kGeneral. (A third kind without the sponge blend, for blocks beyond
-// the sponge band, had fewer instructions per update but a slower step: a
-// third hot copy of the update raised instruction-fetch and memory stalls.)
-enum BlockKind { kGeneral = 0, kFluid = 1 };
-
-__device__ __forceinline__ int block_kind(const StepParams &p, int lo, int hi, int y, int z, bool region) {
-  if (region || p.win.on) return kGeneral;
-  if (p.has_body) {
-    if (!p.bb || !p.nbox_on) return kGeneral;
-    if (span_hits(lo, hi, p.nbox[0], p.nbox[1] - p.nbox[0], p.nx) &&
-        span_hits(y, y, p.nbox[2], p.nbox[3] - p.nbox[2], p.ny) &&
-        span_hits(z, z, p.nbox[4], p.nbox[5] - p.nbox[4], p.nzg))
-      return kGeneral;
-  }
-  if ((p.wall_x && (lo == 0 || hi == p.nx - 1)) || (p.wall_y && (y == 0 || y == p.ny - 1)) ||
-      (p.wall_z && (z == 0 || z == p.nzg - 1)))
-    return kGeneral;
-  return kFluid;
-}
-
-template <int Q, typename S, bool TRT>
-__device__ __forceinline__ void d3_step_block(const S *__restrict__ fin, S *__restrict__ fout,
-                                              float *__restrict__ mac, const StepParams &p) {
-  sum_previous(p);
-  const int x = blockIdx.x * kStepThreads + threadIdx.x;
-  // bz: the stored plane (a slab skips its ghost plane below); zg: the
-  // domain's plane, which the force region and the block kind are in
-  const int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z + p.zlo;
-  const int zg = bz + p.zoff;
-  // the force region, read modulo the grid (it can cross a windowed seam;
-  // a slab's region is its own share, with no seam)
-  int dx = bx - p.rbx0, dy = by - p.rby0, dz = zg - p.rbz0;
-  dx += dx < 0 ? (int)gridDim.x : 0;
-  dy += dy < 0 ? (int)gridDim.y : 0;
-  dz += (dz < 0 && p.zlo == 0) ? p.nzg : 0;
-  const int rx = p.rbx1 - p.rbx0, ry = p.rby1 - p.rby0, rz = p.rbz1 - p.rbz0;
-  const bool region = p.force_on && dx < rx && dy < ry && dz < rz;
-  // The fluid path pays for 16-bit storage (issue-bound: 0.1106 against
-  // 0.1167 ms per step on the 256x128x128 sphere) but not for FP32, whose
-  // step is bound by memory latency and ran 0.1123 against 0.1110 ms with
-  // it (D3Q27: 0.1589 against 0.1537 ms): FP32 takes the general path
-  // everywhere.
-  const int lo = bx * kStepThreads, hi = min(lo + kStepThreads, p.nx) - 1;
-  const int kind = std::is_same<S, float>::value ? kGeneral : block_kind(p, lo, hi, by, zg, region);
-  if (kind == kFluid) {
-    if (x < p.nx) cell3_fluid<Q, S, TRT>(fin, fout, mac, p, x, by, bz);
-    return;
-  }
-  CellForce cf;
-  if (x < p.nx) cell3<Q, S, TRT>(fin, fout, mac, p, x, by, bz, region, cf);
-  if (region) {
-    ForceAcc acc;
-    acc.add(cf);
-    publish_force<kStepThreads>(acc, p.partials, (dz * ry + dy) * rx + dx);
-  }
-}
+// One thread per cell, kStepThreads (64) cells per CTA: of a row, grid
+// (NX/64, NY, NZ), the row and plane straight from blockIdx, or of the
+// plane's cells as one run (choose_step_map).
 
 // A copy of the launch's parameters in shared memory with the body pose,
 // swept-cell band and force region of this step taken from the device
@@ -151,12 +71,40 @@ __device__ __forceinline__ void stage_pose(const StepParams &p, StepParams &sp) 
   __syncthreads();
 }
 
+// A block that no body, wall, force region or window touches runs the fluid
+// update; the others the general one, with the body's links and the walls
+// classified before the gather (Geom3). FP32 is bound by HBM (D3Q19: 152 bytes
+// a cell), 16-bit storage by instruction issue, small domains by the latency
+// of the force region's blocks. 256x128x128 sphere, us per step, before and
+// after the explicit collision, these kinds, the dedicated sum blocks, the
+// tight reach box and (16-bit) the 32-bit offsets:
+//             FP32             FP16             BF16
+//   D3Q19  107.1 -> 102.6   106.6 -> 98.7    106.6 -> 99.4
+//   D3Q27  153.9 -> 146.2   154.3 -> 136.0   154.6 -> 135.6
+// and a D3Q19 FP32 sphere in 64^3 13.1 -> 9.9. (Two cells a thread in packed
+// arithmetic, and planes staged by bulk copies, both ran slower: more
+// registers, so fewer warps to hide the gather.)
 template <int Q, typename S, bool TRT>
 __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) / 4 : kStepMinBlocks)
     d3_step(const S *__restrict__ fin, S *__restrict__ fout, float *__restrict__ mac,
             const __grid_constant__ StepParams p) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
-  d3_step_block<Q, S, TRT>(fin, fout, mac, p);
+  if (sum_previous(p)) return;
+  const BlockMap m = block_map(p, kStepThreads);
+  const int c = m.c0 + threadIdx.x;
+  int x, y;
+  block_cell(p, m, c, x, y);
+  if (block_kind(p, m, kStepThreads) == kFluid) {
+    if (c < m.lim) cell3_fluid<Q, S, TRT>(fin, fout, mac, p, x, y, m.bz);
+    return;
+  }
+  CellForce cf;
+  if (c < m.lim) cell3<Q, S, TRT>(fin, fout, mac, p, x, y, m.bz, m.region, cf);
+  if (m.region) {
+    ForceAcc acc;
+    acc.add(cf);
+    publish_force<kStepThreads>(acc, p.partials, m.part);
+  }
 }
 
 // The step of a free body: the pose comes from the device (written by the
@@ -167,7 +115,12 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
                  const __grid_constant__ StepParams p) {
   __shared__ StepParams sp;
   stage_pose(p, sp);
-  d3_step_block<Q, S, TRT>(fin, fout, mac, sp);
+  const BlockMap m = block_map(sp, kStepThreads);
+  const int c = m.c0 + threadIdx.x;
+  int x, y;
+  block_cell(sp, m, c, x, y);
+  CellForce cf;
+  if (c < m.lim) cell3<Q, S, TRT>(fin, fout, mac, sp, x, y, m.bz, false, cf);
 }
 
 // Integrates the free body under the force just summed and publishes the
@@ -223,9 +176,9 @@ template <typename S>
 __global__ void __launch_bounds__(kStepThreads)
     d2_step(const S *__restrict__ fin, S *__restrict__ fout, float *__restrict__ mac,
             const __grid_constant__ StepParams p) {
-  sum_previous(p);
+  if (sum_previous<kStepThreads, true>(p)) return;
   const int x = blockIdx.x * kStepThreads + threadIdx.x;
-  const int bx = blockIdx.x, by = blockIdx.y;
+  const int bx = blockIdx.x, by = (int)blockIdx.y - p.sum_layers;
   const bool region = p.force_on && bx >= p.rbx0 && bx < p.rbx1 && by >= p.rby0 && by < p.rby1;
   CellForce cf;
   if (x < p.nx) cell2<S>(fin, fout, mac, p, x, by, region, cf);
@@ -396,40 +349,41 @@ int grid_for(int64_t n, int threads) {
 }  // namespace
 
 namespace {
-// A launch that may begin while the previous kernel on the stream drains
-// (programmatic dependent launch): the step and force-sum kernels wait at
-// their first instruction (griddepcontrol.wait) until that kernel has
-// completed and its writes are visible, so the order is the stream's; what
-// overlaps is the new grid's launch and scheduling with the old one's tail.
-// Measured on B200 for one-step calls: 0.124 -> 0.120 ms per step, and with
-// a force readback after each 0.129 -> 0.124 ms.
-template <typename... K, typename... A>
-void launch_pdl(dim3 g, dim3 b, cudaStream_t st, void (*k)(K...), A &&...args) {
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = g;
-  lc.blockDim = b;
-  lc.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = 1;
-  cudaLaunchKernelEx(&lc, k, std::forward<A>(args)...);
-}
 cudaError_t launch_step_kernel(int q, int storage, const void *f_in, void *f_out, float *mac, const StepParams &p,
                                cudaStream_t st) {
-  dim3 grid((p.nx + kStepThreads - 1) / kStepThreads, p.ny, q == 9 ? 1 : p.nz - 2 * p.zlo);
+  if (q != 9 && p.pose_in) {
+    LBM_DISPATCH(q, storage, {
+      auto run = [&](auto k) {
+        k<<<step_grid(p), kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, p);
+      };
+      if constexpr (Q != 9) {
+        if (p.trt_dw != 0.f) run(d3_step_free<Q, S, true>);
+        else run(d3_step_free<Q, S, false>);
+      }
+    });
+  }
+  StepParams r = p;
+  dim3 grid = step_grid(p);
+  if (q == 9) grid = dim3((p.nx + kStepThreads - 1) / kStepThreads, p.ny, 1);
+  if (p.force_on && q != 9) r.rot = std::max(0, p.rbz0 - p.zoff - p.zlo);
+  if (p.prev_parts) {
+    // The sum's blocks: rows in front of a D2Q9 grid, layers in front of a 3D
+    // one. (A whole plane in front of a D2Q9 grid is mostly blocks that start
+    // and leave, 0.4 ns each: 2048x1024 took 49 us per step, 34 without it.)
+    unsigned &along = q == 9 ? grid.y : grid.z;
+    r.sum_layers = sum_layers_for(p, q == 9 ? grid.x : grid.x * grid.y);
+    if (along + r.sum_layers > 65535u) {  // no room for them: a launch of their own
+      r.sum_layers = r.prev_parts = 0;
+      launch_pdl(dim3(sum_groups(p.prev_parts)), dim3(kStepThreads), st, force_finish, p.prev_partials, p.prev_parts,
+                 p.groups, p.counter, p.force_out);
+    }
+    along += r.sum_layers;
+  }
   LBM_DISPATCH(q, storage, {
-    if constexpr (Q == 9)
-      d2_step<S><<<grid, kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, p);
-    else if (p.pose_in && p.trt_dw != 0.f)
-      d3_step_free<Q, S, true><<<grid, kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, p);
-    else if (p.pose_in)
-      d3_step_free<Q, S, false><<<grid, kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, p);
-    else if (p.trt_dw != 0.f)
-      launch_pdl(grid, dim3(kStepThreads), st, d3_step<Q, S, true>, (const S *)f_in, (S *)f_out, mac, p);
-    else
-      launch_pdl(grid, dim3(kStepThreads), st, d3_step<Q, S, false>, (const S *)f_in, (S *)f_out, mac, p);
+    auto run = [&](auto k) { launch_pdl(grid, dim3(kStepThreads), st, k, (const S *)f_in, (S *)f_out, mac, r); };
+    if constexpr (Q == 9) d2_step<S><<<grid, kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, r);
+    else if (p.trt_dw != 0.f) run(d3_step<Q, S, true>);
+    else run(d3_step<Q, S, false>);
   });
 }
 }  // namespace

@@ -162,7 +162,10 @@ __device__ __forceinline__ float chi_from_phi(float phi, float eps) {
 // ---- 2D card geometry ----------------------------------------------------
 
 // WGSL round() ties to even; rintf does the same in the default mode.
-__device__ __forceinline__ float wrap_delta(float d, float n) { return d - n * rintf(d / n); }
+// (Within half a period rint(d / n) is 0 and d itself the result: no division.)
+__device__ __forceinline__ float wrap_delta(float d, float n) {
+  return fabsf(d) < 0.49f * n ? d : d - n * rintf(d / n);
+}
 
 __device__ __forceinline__ float phi2_inline(float px, float py, const lbm_body &b, float W, float H) {
   float ca = cosf(b.theta), sa = sinf(b.theta);
@@ -201,8 +204,12 @@ static __device__ __noinline__ float phi2_call(float px, float py, const lbm_bod
 // An unrotated circle (every pinned cylinder) takes the closed form inline:
 // cos(0) = 1 and sin(0) = 0 make the rotation exact, so this is the same
 // value the general path returns.
+__device__ __forceinline__ bool phi2_is_circle(const lbm_body &b) {
+  return b.theta == 0.0f && fabsf(b.a - b.b) <= 1e-6f * fmaxf(b.a, b.b);
+}
+
 __device__ __forceinline__ float phi2(float px, float py, const lbm_body &b, float W, float H) {
-  if (b.theta == 0.0f && fabsf(b.a - b.b) <= 1e-6f * fmaxf(b.a, b.b)) {
+  if (phi2_is_circle(b)) {
     const float lx = wrap_delta(px - b.cx, W), ly = wrap_delta(py - b.cy, H);
     return __fsqrt_rn(__fadd_rn(__fmul_rn(lx, lx), __fmul_rn(ly, ly))) - b.a;
   }

@@ -32,6 +32,9 @@ bool force_cell_box(const lbm_config &c, StepParams &p, int box[6]);
 // (p.rb*). Returns p.force_on.
 bool set_body_regions(const lbm_config &c, StepParams &p, bool force);
 
+// The force region (p.rb*) of the cell box under the launch mapping of p.
+void set_force_blocks(const int box[6], StepParams &p);
+
 float lattice_weight(int q, int i);
 
 // 16-bit storage encoding of a domain (far-field equilibrium offsets).

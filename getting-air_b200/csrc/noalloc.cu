@@ -106,7 +106,22 @@ int lbm_step_noalloc(const lbm_config *cfg, const void *f_in, void *f_out, float
   lbm::fill_step_params(*cfg, n, 0, p);
   // the reach box and force region exactly as a session sets them
   if (lbm::set_body_regions(*cfg, p, force_out != nullptr)) {
-    const int64_t parts = (int64_t)(p.rbx1 - p.rbx0) * (p.rby1 - p.rby0) * (p.rbz1 - p.rbz0);
+    // what is refused depends neither on the launch mapping nor on the pose:
+    // the blocks of 64 cells of a row around the circumsphere decide, and
+    // where the mapping itself would need more partials than the scratch
+    // holds, the step runs by rows
+    int box[6], r[6];
+    int swept;
+    float band;
+    lbm::body_cell_box(cfg->body, cfg->q, cfg->nx, cfg->ny, cfg->nz, cfg->use_bounceback, cfg->swept_force,
+                       cfg->chi_eps, box, &swept, &band, cfg->q != 9 ? cfg->window : nullptr, false);
+    lbm::box_region(box, p.nx, p.ny, p.nz, nullptr, r);
+    const int64_t parts = (int64_t)(r[1] - r[0]) * (r[3] - r[2]) * (r[5] - r[4]);
+    lbm::force_cell_box(*cfg, p, box);
+    if (parts <= kNoAllocMaxParts && lbm::force_parts(cfg->q, p) > kNoAllocMaxParts) {
+      p.flat = 0;
+      lbm::set_force_blocks(box, p);
+    }
     if (parts > kNoAllocMaxParts)
       return nfail(LBM_ENOSPC, "the body's force region spans " + std::to_string(parts) +
                                    " launch blocks; the fixed scratch holds " + std::to_string(kNoAllocMaxParts));

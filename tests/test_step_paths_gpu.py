@@ -1,0 +1,73 @@
+"""GPU tests of the step's alternative paths: whichever path a size, storage
+or topology selects, a cell gets the same bits.
+
+* 3D dense launch mappings (rows, or a plane's cells as one run) and block
+  kinds, against the same domain in a batch, which updates one cell per
+  thread by plain indices.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def dense_and_batch(lbm, q, dims, steps, seed=0, **kw):
+    n = int(np.prod(dims))
+    rng = np.random.RandomState(seed)
+    mac = np.empty((n, 4), np.float32)
+    mac[:, 0] = 1 + 0.01 * (rng.rand(n) - 0.5)
+    mac[:, 1:] = 0.05 * (rng.rand(n, 3) - 0.3)
+    if q == 9:
+        mac[:, 3] = 0
+    cfg = lbm.config_from(q, dims, **kw)
+    s, b = lbm.Solver(cfg), lbm.Batch([cfg])
+    s.init_macro(mac)
+    b.init_macro(0, mac)
+    s.step(steps)
+    b.step(steps)
+    assert np.array_equal(s.read_f(), b.read_f(0))
+    assert np.array_equal(s.read_mac(), b.read_mac(0))
+    f, g = s.forces(), b.forces()[0]
+    # FP64 sums of the same cell contributions, differently grouped
+    assert np.allclose(f, g, rtol=1e-10, atol=1e-12 * max(np.abs(g).max(), 1e-300))
+    s.close()
+    b.close()
+    return f
+
+
+BODY = dict(has_body=1, use_bounceback=1, sponge_w=4.0, sponge_u=(0.04, 0.0, 0.0), force=(1e-6, 0.0, 0.0))
+# edges of the 64- and 128-cell blocks, odd rows (no word holds two cells),
+# the smallest rows, planes of an odd number of cells
+DIMS = [(3, 3, 3), (4, 3, 5), (5, 5, 3), (63, 7, 5), (64, 6, 5), (65, 5, 7), (100, 9, 6), (127, 5, 5), (128, 4, 6),
+        (129, 5, 3), (130, 6, 4), (151, 7, 5), (256, 3, 4)]
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("dims", DIMS)
+def test_fluid_domain_equals_batch(lbm, dims, storage):
+    dense_and_batch(lbm, 19, dims, 4, tau=0.6, force=(1e-5, -2e-5, 3e-6), storage=storage)
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("q,trt,dims", [(19, 0, (66, 24, 22)), (19, 1, (51, 23, 20)), (27, 0, (100, 26, 24)),
+                                        (27, 1, (128, 20, 25)), (27, 1, (37, 30, 21))])
+def test_body_domain_equals_batch(lbm, q, trt, dims, storage):
+    body = dict(shape="sphere", centre=(dims[0] / 3.0, dims[1] / 2.0, dims[2] / 2.0), a=4.0)
+    f = dense_and_batch(lbm, q, dims, 5, tau=0.58, storage=storage, trt=trt, trt_lambda=0.1875, body=body, **BODY)
+    assert abs(f[0]) > 0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+def test_walls_and_body_at_the_edge_equal_batch(lbm, storage):
+    body = dict(shape="roundbox", centre=(3.0, 20.5, 2.0), a=4.0, b=3.0, c=3.0, r=1.0, quat=(0.96, 0.28, 0.0, 0.0))
+    f = dense_and_batch(lbm, 19, (70, 22, 18), 5, tau=0.6, storage=storage, wall=(1, 1, 1), body=body, has_body=1,
+                        use_bounceback=1)
+    assert abs(f[0]) > 0
+
+
+def test_spheroid_links_equal_batch_and_oracle_side(lbm):
+    body = dict(shape="spheroid", centre=(15.3, 11.8, 12.1), a=5.0, c=2.5, quat=(0.9, 0.3, 0.3, 0.1))
+    qn = np.linalg.norm(body["quat"])
+    body["quat"] = tuple(v / qn for v in body["quat"])
+    f = dense_and_batch(lbm, 19, (40, 24, 24), 6, tau=0.6, body=body, **BODY)
+    assert abs(f[0]) > 0
