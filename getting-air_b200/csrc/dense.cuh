@@ -93,7 +93,8 @@ struct StepParams {
   // Layers (along z; D2Q9: rows) of blocks in front of the grid that only sum
   // the previous launch's force partials (sum_layers_for).
   int sum_layers;
-  // The plane that a 3D launch's first blocks take: the force region's first, so that its blocks, whose chain of link tests, own
+  // The plane (3D) or row (D2Q9) that the launch's first blocks take: the
+  // force region's first, so that its blocks, whose chain of link tests, own
   // populations and block sums is the longest, do not start last.
   int rot;
 };

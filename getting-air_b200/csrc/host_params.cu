@@ -170,10 +170,37 @@ bool force_cell_box(const lbm_config &c, StepParams &p, int box[6]) {
                        &p.swept_band, c.q != 9 ? c.window : nullptr);
 }
 
+// The reach box of a D2Q9 body: with bounce-back the force box (links from
+// within 2.5 of the surface); with the penalty the cells where chi is not 0.
+// chi = (1 - tanh(phi / eps)) / 2 is 0 in FP32 from phi = 12 eps on (1 -
+// tanh(12) = 7.6e-11, far below half an ulp of 1), and phi2 is at least the
+// distance from the body's bounding circle -- or its algebraic far value,
+// which it only takes beyond 64, hence the limit on eps. A box that crosses
+// an edge covers that axis.
+bool reach_box2(const lbm_config &c, const int fbox[6], bool any, int box[6]) {
+  if (c.use_bounceback) {
+    for (int k = 0; k < 6; ++k) box[k] = any ? fbox[k] : -(k & 1);
+    return true;
+  }
+  if (!(c.chi_eps > 0.f && c.chi_eps <= 4.f)) return false;
+  const float reach = body_circumradius(c.body) + 12.0f * c.chi_eps + 1.0f;
+  const float ctr[2] = {c.body.cx, c.body.cy};
+  const int len[2] = {c.nx, c.ny};
+  for (int a = 0; a < 2; ++a) {
+    const float lo = std::floor(ctr[a] - reach), hi = std::ceil(ctr[a] + reach);
+    const bool in = lo >= 0.f && hi <= (float)(len[a] - 1);
+    box[2 * a] = in ? (int)lo : 0;
+    box[2 * a + 1] = in ? (int)hi : len[a] - 1;
+  }
+  box[4] = box[5] = 0;
+  return true;
+}
+
 bool set_body_regions(const lbm_config &c, StepParams &p, bool force) {
   int box[6];
   const bool any = force_cell_box(c, p, box);
   p.nbox_on = 0;
+  if (c.q == 9 && c.has_body) p.nbox_on = reach_box2(c, box, any, p.nbox) ? 1 : 0;
   if (c.q != 9 && c.has_body && c.use_bounceback) {
     p.nbox_on = 1;
     reach_box3(box, any, c.nx, c.ny, c.nz, p.nbox);

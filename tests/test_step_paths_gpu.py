@@ -3,7 +3,8 @@ or topology selects, a cell gets the same bits.
 
 * 3D dense launch mappings (rows, or a plane's cells as one run) and block
   kinds, against the same domain in a batch, which updates one cell per
-  thread by plain indices.
+  thread by plain indices;
+* the D2Q9 reach box, against the batch, which evaluates the body everywhere.
 """
 import numpy as np
 import pytest
@@ -70,4 +71,15 @@ def test_spheroid_links_equal_batch_and_oracle_side(lbm):
     qn = np.linalg.norm(body["quat"])
     body["quat"] = tuple(v / qn for v in body["quat"])
     f = dense_and_batch(lbm, 19, (40, 24, 24), 6, tau=0.6, body=body, **BODY)
+    assert abs(f[0]) > 0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "bf16"])
+@pytest.mark.parametrize("bb", [0, 1])
+@pytest.mark.parametrize("body", [dict(centre=(40.0, 30.0, 0.0), a=5.0, b=5.0),
+                                  dict(centre=(3.0, 30.5, 0.0), a=6.0, b=3.0, theta=0.4),
+                                  dict(centre=(100.2, 58.7, 0.0), a=4.0, b=4.0, v=(0.01, 0.0, 0.0), w=(0.0, 0.0, 0.01))])
+def test_2d_reach_box_equals_batch(lbm, body, bb, storage):
+    f = dense_and_batch(lbm, 9, (130, 61, 1), 6, tau=0.6, storage=storage, has_body=1, use_bounceback=bb,
+                        sponge_w=4.0, sponge_u=(0.04, 0.0, 0.0), body=dict(shape="ellipse", **body))
     assert abs(f[0]) > 0
