@@ -276,10 +276,14 @@ LBM_HD lbm_body body_pose(const lbm_body &shape, const lbm_body_state &s) {
 
 struct BodyPose {
   lbm_body body;
-  int region[6];     // launch blocks that can feel the body: per axis the
-                     // first (in the grid) and first + count, read modulo it
+  int box[6];        // the cells that can feel the body: per axis the first
+                     // (in the grid) and the count, read modulo the grid
   int swept;
   float swept_band;
+  // Bounce-back: the reach box of this pose in cells (StepParams::nbox);
+  // nbox_on = 0 for a penalty body.
+  int nbox_on;
+  int nbox[6];
 };
 
 // The reach box of a pose from its cell box (body_cell_box; any = false: the
@@ -306,8 +310,24 @@ struct BodyDyn {
   int q, nx, ny, nz, bounceback, swept_force;
   int win[3];        // moving-window axes (the box is not clipped on them)
   float chi_eps;
-  int cap[3];        // force-pass grid: the largest box, in launch blocks
+  int cap[3];        // the largest box the force pass is launched for, in cells
   int overflow;      // steps whose box exceeded cap (clipped)
 };
+
+// The force pass's cells of a pose from its cell box (body_cell_box), the
+// count per axis clipped to cap and to the grid; true when cap clipped it.
+LBM_HD bool force_box(const int box[6], int nx, int ny, int nz, const int cap[3], int r[6]) {
+  const int len[3] = {nx, ny, nz};
+  bool clipped = false;
+  for (int a = 0; a < 3; ++a) {
+    int lo = box[2 * a] % len[a], n = box[2 * a + 1] - box[2 * a] + 1;
+    if (lo < 0) lo += len[a];
+    if (n >= len[a]) { lo = 0; n = len[a]; }
+    if (n > cap[a]) { n = cap[a]; clipped = true; }
+    r[2 * a] = lo;
+    r[2 * a + 1] = n;
+  }
+  return clipped;
+}
 
 }  // namespace lbm

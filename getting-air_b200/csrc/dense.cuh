@@ -119,28 +119,24 @@ LBM_HD unsigned row_magic(int nx) { return (unsigned)(((1ull << 32) + (unsigned)
 constexpr int kStepThreads = LBM_STEP_THREADS;
 constexpr int kStepMinBlocks = LBM_STEP_MIN_BLOCKS;
 
-LBM_HD int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
 // The launch blocks of the dense step grid (kStepThreads cells along x, one
 // row per block in y and z) that cover an inclusive cell box: per axis the
 // first block, wrapped into the grid, and first + count, read modulo the
 // grid -- the box of a windowed axis can cross the periodic seam. A box as
-// long as the grid covers all of it; a count above cap[a] is clipped to it
-// and reported (cap NULL: no limit).
-LBM_HD bool box_region(const int box[6], int nx, int ny, int nz, const int *cap, int r[6]) {
+// long as the grid covers all of it.
+inline void box_region(const int box[6], int nx, int ny, int nz, int r[6]) {
   const int unit[3] = {kStepThreads, 1, 1};
   const int nb[3] = {(nx + kStepThreads - 1) / kStepThreads, ny, nz};
-  bool clipped = false;
   for (int a = 0; a < 3; ++a) {
     const int b0 = floor_div(box[2 * a], unit[a]), b1 = floor_div(box[2 * a + 1], unit[a]);
     int first = b0 % nb[a], count = b1 - b0 + 1;
     if (first < 0) first += nb[a];
     if (count >= nb[a]) { first = 0; count = nb[a]; }
-    if (cap && count > cap[a]) { count = cap[a]; clipped = true; }
     r[2 * a] = first;
     r[2 * a + 1] = first + count;
   }
-  return clipped;
 }
 // Force partials summed per block by sum_partials_grouped, and the number of
 // such blocks. A dense step of a small body has about a hundred partials: in
@@ -196,9 +192,9 @@ cudaError_t launch_step(int q, int storage, const void *f_in, void *f_out, float
                         const StepParams &p, cudaStream_t st);
 // Free-body force pass: the cells near the body (pose p.pose_in), FP64
 // force/torque into p.force_out, then the body integrated into p.pose_out.
-// `cap` is the launch grid (the largest box, in blocks).
-cudaError_t launch_force_pass(int q, int storage, const void *f_in, const StepParams &p, const int cap[3],
-                              cudaStream_t st);
+// `parts` is the launch grid (the largest box's cells, kForceThreads a block).
+constexpr int kForceThreads = 128;
+cudaError_t launch_force_pass(int q, int storage, const void *f_in, const StepParams &p, int parts, cudaStream_t st);
 cudaError_t launch_init_eq(int q, int storage, const float *mac_in, void *f_out, int64_t n, const Pack &pk,
                            cudaStream_t st);
 // The equilibrium of one state (rho, ux, uy, uz) in every cell, with that

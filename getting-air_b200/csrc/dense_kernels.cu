@@ -48,7 +48,7 @@ namespace {
 // plane's cells as one run (choose_step_map).
 
 // A copy of the launch's parameters in shared memory with the body pose,
-// swept-cell band and force region of this step taken from the device
+// swept-cell band and reach box of this step taken from the device
 // (free-body launches, where the pose is produced on the device).
 __device__ __forceinline__ void stage_pose(const StepParams &p, StepParams &sp) {
   const unsigned *src = reinterpret_cast<const unsigned *>(&p);
@@ -58,15 +58,10 @@ __device__ __forceinline__ void stage_pose(const StepParams &p, StepParams &sp) 
   if (threadIdx.x == 0) {
     const BodyPose &bp = *p.pose_in;
     sp.body = bp.body;
-    sp.nbox_on = 0;  // the pose moves on the device: evaluate the SDF everywhere
+    sp.nbox_on = bp.nbox_on;
+    for (int k = 0; k < 6; ++k) sp.nbox[k] = bp.nbox[k];
     sp.swept = bp.swept;
     sp.swept_band = bp.swept_band;
-    sp.rbx0 = bp.region[0];
-    sp.rbx1 = bp.region[1];
-    sp.rby0 = bp.region[2];
-    sp.rby1 = bp.region[3];
-    sp.rbz0 = bp.region[4];
-    sp.rbz1 = bp.region[5];
   }
   __syncthreads();
 }
@@ -108,17 +103,29 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
 }
 
 // The step of a free body: the pose comes from the device (written by the
-// force pass just before); no force reduction.
+// force pass just before); no force reduction. Blocks beyond the pose's
+// reach box run the fluid update with the launch's own parameters; the
+// others stage them with the pose in shared memory. (Evaluating the body's
+// distance at every cell, as before the pose carried its reach box, was
+// most of the step: a spheroid's takes an arctangent and three Newton
+// steps of sines and cosines. A spheroid in 96x64x64 with its force pass, bound
+// by the latter's chain of sums: 116.0 -> 46.7 us per step.)
 template <int Q, typename S, bool TRT>
-__global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) / 4 : kStepMinBlocks)
+__global__ void __launch_bounds__(kStepThreads, Q == 27 ? 10 : 12)
     d3_step_free(const S *__restrict__ fin, S *__restrict__ fout, float *__restrict__ mac,
                  const __grid_constant__ StepParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ StepParams sp;
-  stage_pose(p, sp);
-  const BlockMap m = block_map(sp, kStepThreads);
+  const BodyPose &bp = *p.pose_in;
+  const BlockMap m = block_map(p, kStepThreads);
   const int c = m.c0 + threadIdx.x;
   int x, y;
-  block_cell(sp, m, c, x, y);
+  block_cell(p, m, c, x, y);
+  if (block_kind(p, m, kStepThreads, bp.nbox_on, bp.nbox) == kFluid) {
+    if (c < m.lim) cell3_fluid<Q, S, TRT>(fin, fout, mac, p, x, y, m.bz);
+    return;
+  }
+  stage_pose(p, sp);
   CellForce cf;
   if (c < m.lim) cell3<Q, S, TRT>(fin, fout, mac, sp, x, y, m.bz, false, cf);
 }
@@ -132,8 +139,11 @@ __device__ __noinline__ void integrate_and_publish(BodyDyn *dyn, const double *f
   BodyPose np;
   np.body = body_pose(dyn->shape, dyn->st);
   int box[6];
-  if (!body_cell_box(np.body, dyn->q, dyn->nx, dyn->ny, dyn->nz, dyn->bounceback, dyn->swept_force, dyn->chi_eps,
-                     box, &np.swept, &np.swept_band, dyn->win)) {
+  const bool any = body_cell_box(np.body, dyn->q, dyn->nx, dyn->ny, dyn->nz, dyn->bounceback, dyn->swept_force,
+                                 dyn->chi_eps, box, &np.swept, &np.swept_band, dyn->win);
+  np.nbox_on = dyn->bounceback;
+  reach_box3(box, any, dyn->nx, dyn->ny, dyn->nz, np.nbox);
+  if (!any) {
     const float c[3] = {np.body.cx, np.body.cy, np.body.cz};
     const int len[3] = {dyn->nx, dyn->ny, dyn->nz};
     for (int a = 0; a < 3; ++a) {
@@ -141,34 +151,41 @@ __device__ __noinline__ void integrate_and_publish(BodyDyn *dyn, const double *f
       box[2 * a] = box[2 * a + 1] = v;
     }
   }
-  if (box_region(box, dyn->nx, dyn->ny, dyn->nz, dyn->cap, np.region)) dyn->overflow += 1;
+  if (force_box(box, dyn->nx, dyn->ny, dyn->nz, dyn->cap, np.box)) dyn->overflow += 1;
   *next = np;
 }
 
-// Free-body force pass over the blocks of the current force box (the
-// launch grid is the largest box; blocks past this step's box leave at
-// once and take no part in the reduction). The last block to finish sums
-// the partials and integrates the body.
+// Free-body force pass: the cells of the current force box as one run, one
+// per thread (the launch covers the largest box; blocks past this step's
+// cells leave at once and take no part in the reduction). The last block to
+// finish sums the partials and integrates the body, a chain that the step
+// waits for: with a block per 64 cells of a row of the grid the box of a
+// 16-cell body had a thousand partials, whose sum by one warp took most of
+// the pass; as one run it has about a hundred.
 template <int Q, typename S>
-__global__ void __launch_bounds__(kStepThreads)
+__global__ void __launch_bounds__(kForceThreads)
     d3_force_pass(const S *__restrict__ fin, const __grid_constant__ StepParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ StepParams sp;
+  const int *b = p.pose_in->box;
+  const int lx = b[1], ly = b[3], cells = lx * ly * b[5];
+  if ((int)blockIdx.x * kForceThreads >= cells) return;
+  const int lo[3] = {b[0], b[2], b[4]};
   stage_pose(p, sp);
-  const int rx = sp.rbx1 - sp.rbx0, ry = sp.rby1 - sp.rby0, rz = sp.rbz1 - sp.rbz0;
-  if ((int)blockIdx.x >= rx || (int)blockIdx.y >= ry || (int)blockIdx.z >= rz) return;
-  // blocks of the region, wrapped into the grid
-  const int nbx = (sp.nx + kStepThreads - 1) / kStepThreads;
-  int bx = sp.rbx0 + blockIdx.x, by = sp.rby0 + blockIdx.y, bz = sp.rbz0 + blockIdx.z;
-  bx -= bx >= nbx ? nbx : 0;
-  by -= by >= sp.ny ? sp.ny : 0;
-  bz -= bz >= sp.nz ? sp.nz : 0;
-  const int x = bx * kStepThreads + threadIdx.x;
-  CellForce cf;
-  if (x < sp.nx) cell3_force<Q, S>(fin, sp, x, by, bz, cf);
-  const int part = ((int)blockIdx.z * ry + (int)blockIdx.y) * rx + (int)blockIdx.x;
+  const int k = blockIdx.x * kForceThreads + threadIdx.x;
   ForceAcc acc;
-  acc.add(cf);
-  const bool last = reduce_force<kStepThreads>(acc, sp.partials, sp.counter, rx * ry * rz, part, sp.force_out);
+  if (k < cells) {
+    const int row = k / lx, pl = row / ly;
+    int x = lo[0] + k - row * lx, y = lo[1] + row - pl * ly, z = lo[2] + pl;
+    x -= x >= sp.nx ? sp.nx : 0;
+    y -= y >= sp.ny ? sp.ny : 0;
+    z -= z >= sp.nz ? sp.nz : 0;
+    CellForce cf;
+    cell3_force<Q, S>(fin, sp, x, y, z, cf);
+    acc.add(cf);
+  }
+  const int parts = (cells + kForceThreads - 1) / kForceThreads;
+  const bool last = reduce_force<kForceThreads>(acc, sp.partials, sp.counter, parts, blockIdx.x, sp.force_out);
   if (last && threadIdx.x == 0) integrate_and_publish(sp.dyn, sp.force_out, sp.pose_out);
 }
 
@@ -374,7 +391,7 @@ cudaError_t launch_step_kernel(int q, int storage, const void *f_in, void *f_out
   if (q != 9 && p.pose_in) {
     LBM_DISPATCH(q, storage, {
       auto run = [&](auto k) {
-        k<<<step_grid(p), kStepThreads, 0, st>>>((const S *)f_in, (S *)f_out, mac, p);
+        launch_pdl(step_grid(p), dim3(kStepThreads), st, k, (const S *)f_in, (S *)f_out, mac, p);
       };
       if constexpr (Q != 9) {
         if (p.trt_dw != 0.f) run(d3_step_free<Q, S, true>);
@@ -422,12 +439,10 @@ cudaError_t launch_step(int q, int storage, const void *f_in, void *f_out, float
   return cudaGetLastError();
 }
 
-cudaError_t launch_force_pass(int q, int storage, const void *f_in, const StepParams &p, const int cap[3],
-                              cudaStream_t st) {
+cudaError_t launch_force_pass(int q, int storage, const void *f_in, const StepParams &p, int parts, cudaStream_t st) {
   if (q == 9 || !p.pose_in || !p.pose_out || !p.dyn) return cudaErrorInvalidValue;
-  dim3 grid(cap[0], cap[1], cap[2]);
   LBM_DISPATCH(q, storage, {
-    if constexpr (Q != 9) d3_force_pass<Q, S><<<grid, kStepThreads, 0, st>>>((const S *)f_in, p);
+    if constexpr (Q != 9) launch_pdl(dim3(parts), dim3(kForceThreads), st, d3_force_pass<Q, S>, (const S *)f_in, p);
   });
 }
 

@@ -213,7 +213,7 @@ bool set_body_regions(const lbm_config &c, StepParams &p, bool force) {
 
 void set_force_blocks(const int box[6], StepParams &p) {
   int r[6];
-  box_region(box, p.nx, p.ny, p.nz, nullptr, r);
+  box_region(box, p.nx, p.ny, p.nz, r);
   if (p.flat) {  // no window, so the box lies in the grid
     r[0] = (int)(((int64_t)box[2] * p.nx + box[0]) / kStepThreads);
     r[1] = (int)(((int64_t)box[3] * p.nx + box[1]) / kStepThreads) + 1;

@@ -44,7 +44,7 @@ struct lbm_session {
   // Free body: two poses (by step parity) and the integrator state.
   bool free_body = false;
   int body_par = 0;
-  int cap[3] = {0, 0, 0};
+  int body_parts = 0;  // force-pass grid
   BodyPose *pose = nullptr;
   BodyDyn *dyn = nullptr;
   // A z-slab of the domain cfg describes (lbm_create_slab): planes
@@ -416,7 +416,7 @@ int lbm_step(lbm_session *s, int n) {
       fp.dyn = s->dyn;
       fp.force_on = 1;
       fp.write_mac = 0;
-      CK(s, launch_force_pass(s->q, s->storage, s->f[s->cur], fp, s->cap, s->stream));
+      CK(s, launch_force_pass(s->q, s->storage, s->f[s->cur], fp, s->body_parts, s->stream));
       StepParams sp = s->sp;
       sp.pose_in = s->pose + (1 - s->body_par);
       sp.force_on = 0;
@@ -504,15 +504,17 @@ int lbm_set_free_body(lbm_session *s, const lbm_body_state *state, const lbm_bod
   const double speed = vmax + 1.5 * omax * rc + 0.5;
   const double margin = c.use_bounceback ? 3.0 + speed : 8.0 * c.chi_eps + 2.0;
   const double cells = 2.0 * std::ceil(rc + margin) + 3.0;
-  const int nbx = (c.nx + kStepThreads - 1) / kStepThreads;
-  d.cap[0] = std::isfinite(cells) ? (int)std::min<double>(nbx, std::ceil(cells / kStepThreads) + 1) : nbx;
+  d.cap[0] = std::isfinite(cells) ? (int)std::min<double>(c.nx, cells) : c.nx;
   d.cap[1] = std::isfinite(cells) ? (int)std::min<double>(c.ny, cells) : c.ny;
   d.cap[2] = std::isfinite(cells) ? (int)std::min<double>(c.nz, cells) : c.nz;
   BodyPose p0{};
   p0.body = body_pose(c.body, st);
   int box[6];
-  if (!body_cell_box(p0.body, c.q, c.nx, c.ny, c.nz, c.use_bounceback, c.swept_force, c.chi_eps, box, &p0.swept,
-                     &p0.swept_band, c.window)) {
+  const bool any = body_cell_box(p0.body, c.q, c.nx, c.ny, c.nz, c.use_bounceback, c.swept_force, c.chi_eps, box,
+                                 &p0.swept, &p0.swept_band, c.window);
+  p0.nbox_on = c.use_bounceback ? 1 : 0;
+  reach_box3(box, any, c.nx, c.ny, c.nz, p0.nbox);
+  if (!any) {
     const float ctr[3] = {p0.body.cx, p0.body.cy, p0.body.cz};
     const int len[3] = {c.nx, c.ny, c.nz};
     for (int a = 0; a < 3; ++a) {
@@ -520,8 +522,8 @@ int lbm_set_free_body(lbm_session *s, const lbm_body_state *state, const lbm_bod
       box[2 * a] = box[2 * a + 1] = v;
     }
   }
-  box_region(box, c.nx, c.ny, c.nz, d.cap, p0.region);
-  const int need = d.cap[0] * d.cap[1] * d.cap[2];
+  force_box(box, c.nx, c.ny, c.nz, d.cap, p0.box);
+  const int need = (int)(((int64_t)d.cap[0] * d.cap[1] * d.cap[2] + kForceThreads - 1) / kForceThreads);
   if (int rc = grow_force_scratch(s, need)) return rc;
   if (!s->pose) {
     CK(s, cudaMalloc(&s->pose, 2 * sizeof(BodyPose)));
@@ -531,7 +533,7 @@ int lbm_set_free_body(lbm_session *s, const lbm_body_state *state, const lbm_bod
   CK(s, cudaMemcpyAsync(s->pose, &p0, sizeof(BodyPose), cudaMemcpyHostToDevice, s->stream));
   CK(s, cudaMemcpyAsync(s->dyn, &d, sizeof(BodyDyn), cudaMemcpyHostToDevice, s->stream));
   CK(s, cudaStreamSynchronize(s->stream));
-  for (int k = 0; k < 3; ++k) s->cap[k] = d.cap[k];
+  s->body_parts = need;
   s->body_par = 0;
   s->free_body = true;
   return LBM_OK;

@@ -115,7 +115,7 @@ int lbm_step_noalloc(const lbm_config *cfg, const void *f_in, void *f_out, float
     float band;
     lbm::body_cell_box(cfg->body, cfg->q, cfg->nx, cfg->ny, cfg->nz, cfg->use_bounceback, cfg->swept_force,
                        cfg->chi_eps, box, &swept, &band, cfg->q != 9 ? cfg->window : nullptr, false);
-    lbm::box_region(box, p.nx, p.ny, p.nz, nullptr, r);
+    lbm::box_region(box, p.nx, p.ny, p.nz, r);
     const int64_t parts = (int64_t)(r[1] - r[0]) * (r[3] - r[2]) * (r[5] - r[4]);
     lbm::force_cell_box(*cfg, p, box);
     if (parts <= kNoAllocMaxParts && lbm::force_parts(cfg->q, p) > kNoAllocMaxParts) {

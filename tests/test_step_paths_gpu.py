@@ -4,7 +4,8 @@ or topology selects, a cell gets the same bits.
 * 3D dense launch mappings (rows, or a plane's cells as one run) and block
   kinds, against the same domain in a batch, which updates one cell per
   thread by plain indices;
-* the D2Q9 reach box, against the batch, which evaluates the body everywhere.
+* the D2Q9 reach box, against the batch, which evaluates the body everywhere;
+* a free body that is pinned, against the prescribed pose.
 """
 import numpy as np
 import pytest
@@ -83,3 +84,26 @@ def test_2d_reach_box_equals_batch(lbm, body, bb, storage):
     f = dense_and_batch(lbm, 9, (130, 61, 1), 6, tau=0.6, storage=storage, has_body=1, use_bounceback=bb,
                         sponge_w=4.0, sponge_u=(0.04, 0.0, 0.0), body=dict(shape="ellipse", **body))
     assert abs(f[0]) > 0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("shape,bb", [("sphere", 1), ("spheroid", 1), ("roundbox", 1), ("spheroid", 0)])
+def test_pinned_free_body_equals_prescribed_pose(lbm, shape, bb, storage):
+    dims = (75, 30, 28)
+    n = int(np.prod(dims))
+    body = dict(shape=shape, centre=(22.3, 14.6, 13.9), a=5.0, b=4.0, c=3.0, r=1.0 if shape == "roundbox" else 0.0,
+                quat=(0.8, 0.6, 0.0, 0.0))
+    cfg = lbm.config_from(19, dims, tau=0.6, storage=storage, body=body, **dict(BODY, use_bounceback=bb))
+    out = []
+    for free in (False, True):
+        s = lbm.Solver(cfg)
+        mac = np.tile(np.array([1.0, 0.04, 0.0, 0.0], np.float32), (n, 1))
+        s.init_macro(mac)
+        if free:
+            s.set_free_body(lbm.body_state(cfg.body, 1.0), lbm.body_opts(pinned=1))
+        s.step(6)
+        out.append((s.read_f(), s.read_mac(), s.forces()))
+        s.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.allclose(out[0][2], out[1][2], rtol=1e-10, atol=1e-12 * np.abs(out[0][2]).max())
