@@ -74,6 +74,7 @@ struct StepParams {
   int defer_force;
   int prev_parts;
   const double *prev_partials;
+  int clear_ticket;        // the step zeroes `counter` first (no prev_parts)
   Pack pk;                 // 16-bit storage encoding
   // Multi-domain launches: the domain's first tile, and the tile range
   // [ft0, ft1) (relative to tile0) whose cells can see the body.

@@ -12,6 +12,7 @@ namespace lbm {
 template <int THREADS = kStepThreads, bool ROWS = false>
 __device__ __forceinline__ bool sum_previous(const StepParams &p) {
   const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  if (p.clear_ticket && b == 0 && threadIdx.x == 0) *p.counter = 0u;
   if ((int)(ROWS ? blockIdx.y : blockIdx.z) >= p.sum_layers) return false;
   if (b < sum_groups(p.prev_parts))
     sum_partials_grouped<THREADS>(p.prev_partials, p.prev_parts, p.groups, p.counter, p.force_out, b);

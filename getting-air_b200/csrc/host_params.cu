@@ -159,6 +159,7 @@ void fill_step_params(const lbm_config &c, int64_t n, int64_t base, StepParams &
   p.defer_force = 0;
   p.prev_parts = 0;
   p.prev_partials = nullptr;
+  p.clear_ticket = 0;
   p.sum_layers = 0;
   p.rot = 0;
   choose_step_map(c, p);

@@ -26,10 +26,11 @@
 //    torn down by cudaDeviceReset is followed by a fresh address, not a
 //    stale one; a graph captured before such a reset must not be replayed;
 //  * all calls on a device share the one array, which keeps the last call's
-//    contents. Each call clears the sum's ticket on its stream before the
-//    step (the only scratch that must start at zero; partials and group
-//    sums are written before they are read), so a sum that an earlier call
-//    left unfinished cannot skew a later one. Two calls whose kernels
+//    contents. Each call's step clears the sum's ticket before the sum runs
+//    (the only scratch that must start at zero; partials and group sums are
+//    written before they are read), so a sum that an earlier call left
+//    unfinished cannot skew a later one. (A memset of its own for those four
+//    bytes cost a third launch per call.) Two calls whose kernels
 //    overlap on the GPU still race on the array: serialise them (one stream,
 //    or events between streams);
 //  * force_out, when given, is always written on the stream: the body's
@@ -136,12 +137,11 @@ int lbm_step_noalloc(const lbm_config *cfg, const void *f_in, void *f_out, float
   p.counter = reinterpret_cast<unsigned int *>(p.groups + kMaxGroups * lbm::kForceSlots);
   p.force_out = force_out;
   p.write_mac = mac ? 1 : 0;
-  cudaError_t z = cudaSuccess;
-  if (p.force_on)
-    z = cudaMemsetAsync(p.counter, 0, sizeof(unsigned int), st);
-  else if (force_out)
-    z = cudaMemsetAsync(force_out, 0, lbm::kForceSlots * sizeof(double), st);
-  if (z != cudaSuccess) return nfail(LBM_ECUDA, std::string("clear: ") + cudaGetErrorString(z));
+  p.clear_ticket = p.force_on;
+  if (!p.force_on && force_out) {
+    const cudaError_t z = cudaMemsetAsync(force_out, 0, lbm::kForceSlots * sizeof(double), st);
+    if (z != cudaSuccess) return nfail(LBM_ECUDA, std::string("clear: ") + cudaGetErrorString(z));
+  }
   const cudaError_t e = lbm::launch_step(cfg->q, cfg->storage, f_in, f_out, mac, p, st);
   if (e != cudaSuccess) return nfail(LBM_ECUDA, std::string("step: ") + cudaGetErrorString(e));
   return LBM_OK;
