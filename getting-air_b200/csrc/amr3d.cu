@@ -2,8 +2,9 @@
 // macro-step and the session behind lbm_amr3d_*.
 //
 // One macro-step (main-3d.js:3219-3341, ?interface=explode):
-//   amr3_force     pool force on the tiles at time t (FP64, deterministic)
-//   amr3_explode   L0 (time t) -> every tile's ring, Chen et al. 2006: the
+//   amr3_explode   the pool force on the tiles at time t (FP64, deterministic;
+//                  amr3_force by itself with the penalty), and
+//                  L0 (time t) -> every tile's ring, Chen et al. 2006: the
 //                  populations of an unrefined L0 cell V whose target V + e_i
 //                  is covered, moved unchanged into V's eight fine cells
 //                  (plus the linear term orthogonal to e_i), and the
@@ -63,7 +64,8 @@ __device__ __forceinline__ bool interior(const Amr3Params &p, int j) { return j 
 struct TileCell {
   int slot, bx, by, bz, fx, fy, fz;
   int64_t cell;
-  int k;  // position in the tile's cell list (cell-list kernels)
+  int k;   // position in the tile's cell list (cell-list kernels)
+  int nb;  // the neighbour block it lies in (13: this tile's own)
 };
 
 // Tile kernels run one CTA per (fz, slot) with an FB x FB thread block, so a
@@ -78,31 +80,56 @@ __device__ __forceinline__ bool tile_cell(const Amr3Params &p, TileCell &t) {
   return true;
 }
 
-// The D3Q27 directions (D3Q19 their first 19), as a table in constant
-// memory for loops over a runtime direction index.
-struct DirTable {
-  signed char ex[27], ey[27], ez[27];
-};
-constexpr DirTable make_dirs() {
-  DirTable t{};
-  for (int i = 0; i < 27; ++i) {
-    t.ex[i] = (signed char)detail::ex27(i);
-    t.ey[i] = (signed char)detail::ey27(i);
-    t.ez[i] = (signed char)detail::ez27(i);
-  }
-  return t;
-}
-__constant__ DirTable c_dirs = make_dirs();
-
-// Cell-list kernels: one CTA of kListThreads per (chunk, slot) walking a
-// per-session list of the tile's cells -- the interior first, then the
-// ring -- so that a warp holds interior cells or ring cells, not both, and
-// a ring-only pass launches no interior threads. Sets up the CTA's
-// neighbour table; false for a thread with no cell (after the barrier).
+// Cell-list kernels: one CTA of kListThreads per (slot, chunk) of a
+// per-session list of the tile's cells: the interior first, then the ring
+// grouped by the neighbour block it lies in (faces, edges, corners), so that
+// a warp holds interior cells or ring cells of one neighbour.
+//
+// A ring cell inside a refined neighbour is dead: nothing reads it. Every
+// pull past the interior goes to that neighbour's own cells (DIRECT_GHOST),
+// the coalesce reads ring cells over unrefined L0 cells only, and explode
+// refills those at every macro-step. Two thirds of the ring cells of a
+// hierarchy of thousands of tiles are dead, so the explode and the substeps
+// run over a work list of the chunks that hold another cell (TileWork) and
+// skip the dead ones. What a caller reads back of the pool stays what it
+// was: the last substep of a call runs over every cell, and a dead cell's
+// value there depends on live cells -- and, through its links into the body,
+// on its own populations of the substep before. With a body at rest that is
+// as far as it goes (corr = 0: a bounced population whose opposite was pulled
+// comes from that pull, and a pair that both bounce is swapped by each
+// substep), so only the last macro-step's first substep updates the dead
+// cells with links (need), and one whose every link bounces keeps its value
+// (hold). A moving body's bounce depends on the whole history: then every
+// substep updates the cells of need. Where dead cells are read after all (the
+// penalty force's tile-clamped gather; the interp interface, whose ring
+// collides), and without the link table, every substep runs over every cell
+// (p.live = 0). Bound by instruction issue and the latency of the neighbour
+// gathers; per macro-step, together with the merged launches below, 2262
+// tiles around a box in 180^3: 660 -> 447 us; 160 tiles around a
+// sphere in 192x128x128, where the coarse step is most of it: 154 -> 139 us.
 constexpr int kListThreads = 128;
 
+// Work items (slot << 8 | chunk) of a launch; items NULL: a 2D grid of
+// (chunk, slot). count (dynamic hierarchies): the items in use of the grid.
+struct TileWork {
+  const uint32_t *items;
+  const int *count;
+};
+
+// The CTA's slot and chunk; false past the end of the list.
+__device__ __forceinline__ bool work_item(const TileWork &w, int block, int &slot, int &chunk) {
+  slot = blockIdx.y;
+  chunk = block;
+  if (!w.items) return true;
+  if (w.count && block >= __ldg(w.count)) return false;
+  const uint32_t it = __ldg(w.items + block);
+  slot = (int)(it >> 8);
+  chunk = (int)(it & 0xffu);
+  return true;
+}
+
+// Sets up the CTA's neighbour table for tile t.slot; false for a free slot.
 __device__ __forceinline__ bool list_tile(const Amr3Params &p, int *nb27, TileCell &t, bool as_base) {
-  t.slot = blockIdx.y;
   const int id = p.slot_to_block[t.slot];
   if (id < 0) return false;  // the whole CTA: a free slot
   t.bx = id % p.nbx; t.by = (id / p.nbx) % p.nby; t.bz = id / (p.nbx * p.nby);
@@ -123,16 +150,19 @@ __device__ __forceinline__ void list_at(const Amr3Params &p, const uint32_t *__r
                                         TileCell &t) {
   t.k = pos;
   const uint32_t c = __ldg(cells + pos);
-  t.fx = c & 0xff; t.fy = (c >> 8) & 0xff; t.fz = c >> 16;
+  t.fx = c & 0xff; t.fy = (c >> 8) & 0xff; t.fz = (c >> 16) & 0xff;
+  t.nb = c >> 24;
   t.cell = (int64_t)t.slot * p.T3 + (t.fz * p.FB + t.fy) * p.FB + t.fx;
 }
 
-__device__ __forceinline__ bool list_cell(const Amr3Params &p, const uint32_t *__restrict__ cells, int first,
-                                          int count, int *nb27, TileCell &t, bool as_base = false) {
-  if (!list_tile(p, nb27, t, as_base)) return false;
-  const int k = blockIdx.x * kListThreads + threadIdx.x;
-  if (k >= count) return false;
-  list_at(p, cells, first + k, t);
+// The thread's cell; false for a thread with none (after the barrier).
+__device__ __forceinline__ bool list_cell(const Amr3Params &p, const uint32_t *__restrict__ cells, const TileWork &w,
+                                          int *nb27, TileCell &t, bool as_base = false, int block = (int)blockIdx.x) {
+  int chunk;
+  if (!work_item(w, block, t.slot, chunk) || !list_tile(p, nb27, t, as_base)) return false;
+  const int k = chunk * kListThreads + threadIdx.x;
+  if (k >= p.T3) return false;
+  list_at(p, cells, k, t);
   return true;
 }
 
@@ -262,7 +292,7 @@ __global__ void __launch_bounds__(kListThreads)
                const unsigned char *__restrict__ only_new) {
   TileCell t;
   __shared__ int nb27[27];
-  if (!list_cell(p, cells, 0, p.T3, nb27, t)) return;
+  if (!list_cell(p, cells, {nullptr, nullptr}, nb27, t)) return;
   if (only_new && !only_new[t.slot]) return;
   links[t.cell] = link_code<Q>(p, t, phi3(tile_pos(p, t), p.c.body, p.c.win));
 }
@@ -273,16 +303,16 @@ __global__ void __launch_bounds__(kListThreads)
 __device__ __forceinline__ int nb_side(int r, int rb) { return r < 0 ? 0 : (r >= rb ? 2 : 1); }
 
 template <int Q>
-__global__ void __launch_bounds__(kListThreads)
-    amr3_explode(const float *__restrict__ fc, float *__restrict__ fp, const __grid_constant__ Amr3Params p,
-                 const uint32_t *__restrict__ cells, int first, int count) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
+__device__ __forceinline__ void explode_block(const float *__restrict__ fc, float *__restrict__ fp, const Amr3Params &p,
+                                              const uint32_t *__restrict__ cells, const TileWork &w, int block) {
   using L = Lattice<Q>;
   TileCell t;
   // the ring cells only; coverage of the L0 cells around the tile from the
   // neighbour table
   __shared__ int nb27[27];
-  if (!list_cell(p, cells, first, count, nb27, t)) return;
+  if (!list_cell(p, cells, w, nb27, t, false, block)) return;
+  // interior cells of a mixed chunk, and ring cells inside a covered L0 cell
+  if (t.nb == 13 || nb27[t.nb] >= 0) return;
   const int b[3] = {t.bx, t.by, t.bz};
   const int fi[3] = {t.fx, t.fy, t.fz};
   const int nf[3] = {2 * p.nx, 2 * p.ny, 2 * p.nz};
@@ -303,8 +333,6 @@ __global__ void __launch_bounds__(kListThreads)
   }
   auto sd = [&](int a, int e) { return (side[a] >> (2 * (e + 1))) & 3; };
   auto sf = [&](int a, int e) { return (side[a] >> (6 + 2 * (e + 1))) & 3; };
-  // A ring cell inside a covered L0 cell is never read (DIRECT_GHOST).
-  if (nb27[sd(2, 0) * 9 + sd(1, 0) * 3 + sd(0, 0)] >= 0) return;
   // L0 cells as 32-bit offsets (N < 2^31)
   const int vc = (int)ccell(p, v[0], v[1], v[2]);
   bool ok[3];
@@ -355,6 +383,139 @@ __global__ void __launch_bounds__(kListThreads)
   }
 }
 
+// ---- pool force (common_d3_force_pool.wgsl) -------------------------------
+// Interior cells of every tile at time t: momentum exchange with local rho_w
+// weighted by dx^2 = 1/4, the swept-cell term by dx^3 = 1/8, or the chi
+// penalty with a tile-clamped gather; FP64 partial per CTA, last-CTA sum.
+__host__ __device__ __forceinline__ int force_chunks(const Amr3Params &p) {
+  return (p.RB2 * p.RB2 * p.RB2 + kTileThreads - 1) / kTileThreads;
+}
+
+template <int Q>
+__device__ __forceinline__ void force_block(const float *__restrict__ fp, const Amr3Params &p,
+                                            const uint32_t *__restrict__ cells, int slot, int chunk) {
+  using L = Lattice<Q>;
+  const StepParams &c = p.c;
+  const int r3 = p.RB2 * p.RB2 * p.RB2;
+  const int k = chunk * kTileThreads + threadIdx.x;
+  CellForce cf;
+  const int id = p.slot_to_block[slot];
+  if (k < r3 && id >= 0) {
+    const int b[3] = {id % p.nbx, (id / p.nbx) % p.nby, id / (p.nbx * p.nby)};
+    // interior cell k (the cell list holds the interior first, z-, y-, x-major)
+    const uint32_t cl = __ldg(cells + k);
+    const int fx = cl & 0xff, fy = (cl >> 8) & 0xff, fz = (cl >> 16) & 0xff;
+    const int64_t cell = (int64_t)slot * p.T3 + (fz * p.FB + fy) * p.FB + fx;
+    const V3 pos = {f2c(fx, b[0] * p.rb), f2c(fy, b[1] * p.rb), f2c(fz, b[2] * p.rb)};
+    // With the link table and no swept-cell term, the cell's code says all
+    // the bounce-back force needs (0 <= phi < 1: near and not solid) and
+    // the distance is not evaluated.
+    const bool coded = c.bb && p.links && !c.swept;
+    const uint32_t code = coded ? __ldg(p.links + cell) : 0u;
+    const float phi = coded ? 0.5f : phi3(pos, c.body, c.win);
+    const V3 us = body_velocity3(pos, c.body, c.win);
+    float fbx = 0.f, fby = 0.f, fbz = 0.f, fsx = 0.f, fsy = 0.f, fsz = 0.f;
+    if (c.bb) {
+      if (coded ? (code & (kLinkNear | kLinkSolid)) == kLinkNear : (phi >= 0.f && phi < 1.0f)) {
+        float rhoW = 1.f;
+        if (c.rho_w_local && phi < 2.f) {
+          float s = 0.f;
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s += __ldg(fp + (int64_t)i * p.P + cell);
+          rhoW = s;
+        }
+        // the solid sources (the cell itself, phi >= 0 here, is not one)
+        uint32_t solid;
+        if (coded) {
+          solid = code & ((1u << Q) - 2u);
+        } else if (p.links) {
+          solid = __ldg(p.links + cell) & ((1u << Q) - 2u);
+        } else {
+          const TileCell t = {slot, b[0], b[1], b[2], fx, fy, fz, cell};
+          solid = link_code<Q>(p, t, phi) & ((1u << Q) - 2u);
+        }
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+          if (solid & (1u << i)) {
+            const float fo = __ldg(fp + (int64_t)L::opp(i) * p.P + cell);
+            const float corr =
+                2.f * L::w(i) * rhoW * ((float)L::ex(i) * us.x + (float)L::ey(i) * us.y + (float)L::ez(i) * us.z) * kInvCS2;
+            const float m = 2.f * fo + corr;
+            fbx += -(float)L::ex(i) * m;
+            fby += -(float)L::ey(i) * m;
+            fbz += -(float)L::ez(i) * m;
+          }
+        }
+      }
+      if (c.swept && fabsf(phi) < c.swept_band) {
+        const bool now = phi < 0.f;
+        if (now != (phi3_ahead(pos, c.body, 1.f, c.win) < 0.f)) {
+          float mcx = 0.f, mcy = 0.f, mcz = 0.f;
+#pragma unroll
+          for (int i = 0; i < Q; ++i) {
+            const float v = __ldg(fp + (int64_t)i * p.P + cell);
+            mcx += v * (float)L::ex(i); mcy += v * (float)L::ey(i); mcz += v * (float)L::ez(i);
+          }
+          if (!now) { fsx = mcx; fsy = mcy; fsz = mcz; }
+          else { fsx = -mcx; fsy = -mcy; fsz = -mcz; }
+        }
+      }
+    } else {
+      const float chi = chi_from_phi(phi, p.chi_eps_f);
+      if (chi >= 1e-6f) {
+        float rho = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+          const int sx = min(max(fx - L::ex(i), 0), p.FB - 1), sy = min(max(fy - L::ey(i), 0), p.FB - 1),
+                    sz = min(max(fz - L::ez(i), 0), p.FB - 1);
+          const float v = __ldg(fp + (int64_t)i * p.P + (int64_t)slot * p.T3 + (sz * p.FB + sy) * p.FB + sx);
+          rho += v;
+          mx += v * (float)L::ex(i); my += v * (float)L::ey(i); mz += v * (float)L::ez(i);
+        }
+        const float den = fmaxf(rho, 1e-6f);
+        fbx = -(rho * chi * (us.x - mx / den));
+        fby = -(rho * chi * (us.y - my / den));
+        fbz = -(rho * chi * (us.z - mz / den));
+      }
+    }
+    const float tx = fbx * 0.25f + fsx * 0.125f, ty = fby * 0.25f + fsy * 0.125f, tz = fbz * 0.25f + fsz * 0.125f;
+    const V3 r = body_delta(pos, c.body, c.win);
+    const float rx = r.x, ry = r.y, rz = r.z;
+    cf.fx = tx; cf.fy = ty; cf.fz = tz;
+    cf.tx = ry * tz - rz * ty;
+    cf.ty = rz * tx - rx * tz;
+    cf.tz = rx * ty - ry * tx;
+  }
+  ForceAcc acc;
+  acc.add(cf);
+  publish_force<kTileThreads>(acc, p.partials, slot * force_chunks(p) + chunk);
+}
+
+template <int Q>
+__global__ void __launch_bounds__(kTileThreads)
+    amr3_force(const float *__restrict__ fp, const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
+  force_block<Q>(fp, p, cells, blockIdx.y, blockIdx.x);
+}
+
+// The pool force and the explode in one launch: the first nforce CTAs take
+// the force of the tiles' interior (populations of time t), the rest the
+// explode's work list, which writes ring cells only. (As two launches of a
+// few microseconds each, one waited for the other's drain.)
+template <int Q>
+__global__ void __launch_bounds__(kListThreads)
+    amr3_explode(const float *__restrict__ fc, float *__restrict__ fp, const __grid_constant__ Amr3Params p,
+                 const uint32_t *__restrict__ cells, const TileWork w, int nforce) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
+  const int b = (int)blockIdx.x;
+  if (b < nforce) {
+    const int fch = force_chunks(p), slot = b / fch;
+    force_block<Q>(fp, p, cells, slot, b - slot * fch);
+    return;
+  }
+  explode_block<Q>(fc, fp, p, cells, w, b - nforce);
+}
+
 // ---- one pool substep ----------------------------------------------------
 // Population index i * P + cell, in 32 bits when every index of the pool
 // fits (W32: Q * P < 2^31, the usual case), so that an address is one
@@ -368,15 +529,16 @@ template <bool W32> struct PoolSink {
   __device__ __forceinline__ void put(int i, float v) { fo[(PoolIdx<W32>)i * n + cell] = v; }
 };
 
-template <int Q, bool W32>
-__device__ __forceinline__ void substep_cell(const float *__restrict__ fin, float *__restrict__ fout,
+template <int Q, bool W32, bool LIVE>
+__device__ __forceinline__ void substep_cell(const float *__restrict__ fin, float *fout,
                                              float4 *__restrict__ macp, const Amr3Params &p, const int *nbase,
-                                             const TileCell &t) {
+                                             const TileCell &t, bool need) {
   using L = Lattice<Q>;
   using I = PoolIdx<W32>;
   const I P = (I)p.P;
   const int cell = (int)t.cell;  // < P < 2^31
   const StepParams &c = p.c;
+  const bool dead = p.live && t.nb != 13 && nbase[t.nb] >= 0;
   const V3 pos = tile_pos(p, t);
   const bool bb = c.has_body && c.bb;
   float phi = 1e30f;  // the penalty's chi reads it; bounce-back reads the link code
@@ -387,7 +549,10 @@ __device__ __forceinline__ void substep_cell(const float *__restrict__ fin, floa
     else code = p.links ? __ldg(p.links + t.cell) : link_code<Q>(p, t, phi3(pos, c.body, c.win));
     us = body_velocity3(pos, c.body, c.win);
   }
-  const bool in_tile = interior(p, t.fx) && interior(p, t.fy) && interior(p, t.fz);
+  constexpr uint32_t kAll = (1u << Q) - 1u;
+  const bool hold = dead && p.resting && (code & kAll) == kAll;
+  if (LIVE && dead && (hold || !need || !(code & kAll))) return;
+  const bool in_tile = t.nb == 13;
   // A cell that collides inside the body (SOLID_EQ) is held at feq(1, u_body),
   // whatever it pulls: write that and skip the pull.
   if ((in_tile || p.collide_ring) && c.solid_eq && (code & kLinkSolid)) {
@@ -408,7 +573,7 @@ __device__ __forceinline__ void substep_cell(const float *__restrict__ fin, floa
     for (int i = 0; i < Q; ++i) s += __ldg(fin + (I)i * P + cell);
     rhoW = s;
   }
-  const uint32_t solid_links = code & ((1u << Q) - 1u);
+  const uint32_t solid_links = hold ? 0u : code & kAll;
   // The Q pull loads, addressed from the pull table (four directions per
   // 128-bit load of it) as 32-bit cell offsets from each plane's base, all
   // in flight together. A solid link then takes the cell's own opposite
@@ -427,7 +592,7 @@ __device__ __forceinline__ void substep_cell(const float *__restrict__ fin, floa
       if (i < Q) {
         const int nb = nbase[w[u] & 31u];
         const int off = nb >= 0 ? nb + (int)((w[u] >> 5) & 0x1fffu) : own + (int)(w[u] >> 18);
-        f[i] = __ldg(fin + (I)i * P + off);
+        f[i] = !LIVE && hold ? fout[(I)i * P + cell] : __ldg(fin + (I)i * P + off);
       }
     }
   }
@@ -480,16 +645,17 @@ __device__ __forceinline__ void substep_cell(const float *__restrict__ fin, floa
 // One thread per tile cell: CTAs of kListThreads over chunks of the tile's
 // cell list. (A CTA walking several chunks, so that the tile set-up is paid
 // once, held more registers and ran slower: other CTAs hide the set-up.)
-template <int Q, bool W32>
+template <int Q, bool W32, bool LIVE>
 __global__ void __launch_bounds__(kListThreads, Q == 19 ? (W32 ? 9 : 8) : 6)
-    amr3_substep(const float *__restrict__ fin, float *__restrict__ fout, float4 *__restrict__ macp,
-                 const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells, int count) {
+    amr3_substep(const float *__restrict__ fin, float *fout, float4 *__restrict__ macp,
+                 const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells, const TileWork w,
+                 int need) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
   TileCell t;
   // the tile's 26 same-level neighbours as pool cell bases, once per CTA
   __shared__ int nbase[27];
-  if (!list_cell(p, cells, 0, count, nbase, t, true)) return;
-  substep_cell<Q, W32>(fin, fout, macp, p, nbase, t);
+  if (!list_cell(p, cells, w, nbase, t, true)) return;
+  substep_cell<Q, W32, LIVE>(fin, fout, macp, p, nbase, t, need != 0);
 }
 
 // ---- coalesce -------------------------------------------------------------
@@ -510,13 +676,6 @@ __device__ __forceinline__ int local_in_tile(const Amr3Params &p, int g, int b, 
 // thousands of blocks one thread per cell (SUBS = 1) keeps its restriction
 // loop unrolled. The 3 x 3 x 3 neighbour blocks' slots come from a shared
 // table, so no coverage or slot lookup goes to global memory or divides.
-__device__ __forceinline__ int rel_block(int q, int b, int nb) {
-  int d = q - b;
-  if (d > 1) d -= nb;
-  if (d < -1) d += nb;
-  return d;
-}
-
 template <int Q, int SUBS>
 __global__ void __launch_bounds__(kMaxAmrRb * kMaxAmrRb * kMaxAmrRb)
     amr3_coalesce(const float *__restrict__ fp, float *__restrict__ fc, float4 *__restrict__ macc,
@@ -528,15 +687,19 @@ __global__ void __launch_bounds__(kMaxAmrRb * kMaxAmrRb * kMaxAmrRb)
   const int b[3] = {id % p.nbx, (id / p.nbx) % p.nby, id / (p.nbx * p.nby)};
   __shared__ int nb27[27];
   __shared__ signed char dir[3][27];
+  bool inner = true;
   for (int k = threadIdx.x; k < 27; k += blockDim.x) {
     const int dx = k % 3 - 1, dy = (k / 3) % 3 - 1, dz = k / 9 - 1;
     nb27[k] = p.block_slot[(wrapi(b[2] + dz, p.nbz) * p.nby + wrapi(b[1] + dy, p.nby)) * p.nbx +
                            wrapi(b[0] + dx, p.nbx)];
+    inner = inner && nb27[k] >= 0;
     dir[0][k] = (signed char)L::ex(k < Q ? k : 0);
     dir[1][k] = (signed char)L::ey(k < Q ? k : 0);
     dir[2][k] = (signed char)L::ez(k < Q ? k : 0);
   }
-  __syncthreads();
+  // a refined block among refined blocks has no population to restrict,
+  // only its cells' mac
+  if (__syncthreads_and(inner) && !p.write_mac) return;
   const int l = threadIdx.x / SUBS, sub = threadIdx.x % SUBS;
   // the cell's position within its block, per axis
   const int lc[3] = {l % p.rb, (l / p.rb) % p.rb, l / (p.rb * p.rb)};
@@ -745,6 +908,7 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
   asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
   const BlockMap m = block_map(sp, kStepThreads);
   const int c = m.c0 + threadIdx.x;
+  if (sum_previous(sp)) return;
   if (c >= m.lim) return;
   int x, y;
   block_cell(sp, m, c, x, y);
@@ -756,122 +920,6 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
   }
   CellForce cf;
   cell3<Q, float>(fin, fout, mac, sp, x, y, m.bz, false, cf);
-}
-
-// ---- pool force (common_d3_force_pool.wgsl) -------------------------------
-// Interior cells of every tile at time t: momentum exchange with local rho_w
-// weighted by dx^2 = 1/4, the swept-cell term by dx^3 = 1/8, or the chi
-// penalty with a tile-clamped gather; FP64 partial per CTA, last-CTA sum.
-template <int Q>
-__global__ void __launch_bounds__(kTileThreads)
-    amr3_force(const float *__restrict__ fp, const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
-  using L = Lattice<Q>;
-  const StepParams &c = p.c;
-  const int r3 = p.RB2 * p.RB2 * p.RB2;
-  const int k = blockIdx.x * kTileThreads + threadIdx.x;
-  CellForce cf;
-  const int slot = blockIdx.y;
-  const int id = p.slot_to_block[slot];
-  if (k < r3 && id >= 0) {
-    const int b[3] = {id % p.nbx, (id / p.nbx) % p.nby, id / (p.nbx * p.nby)};
-    // interior cell k (the cell list holds the interior first, z-, y-, x-major)
-    const uint32_t cl = __ldg(cells + k);
-    const int fx = cl & 0xff, fy = (cl >> 8) & 0xff, fz = cl >> 16;
-    const int64_t cell = (int64_t)slot * p.T3 + (fz * p.FB + fy) * p.FB + fx;
-    const V3 pos = {f2c(fx, b[0] * p.rb), f2c(fy, b[1] * p.rb), f2c(fz, b[2] * p.rb)};
-    // With the link table and no swept-cell term, the cell's code says all
-    // the bounce-back force needs (0 <= phi < 1: near and not solid) and
-    // the distance is not evaluated.
-    const bool coded = c.bb && p.links && !c.swept;
-    const uint32_t code = coded ? __ldg(p.links + cell) : 0u;
-    const float phi = coded ? 0.5f : phi3(pos, c.body, c.win);
-    const V3 us = body_velocity3(pos, c.body, c.win);
-    float fbx = 0.f, fby = 0.f, fbz = 0.f, fsx = 0.f, fsy = 0.f, fsz = 0.f;
-    if (c.bb) {
-      if (coded ? (code & (kLinkNear | kLinkSolid)) == kLinkNear : (phi >= 0.f && phi < 1.0f)) {
-        float rhoW = 1.f;
-        if (c.rho_w_local && phi < 2.f) {
-          float s = 0.f;
-#pragma unroll
-          for (int i = 0; i < Q; ++i) s += __ldg(fp + (int64_t)i * p.P + cell);
-          rhoW = s;
-        }
-        // the solid sources (the cell itself, phi >= 0 here, is not one)
-        uint32_t solid;
-        if (coded) {
-          solid = code & ((1u << Q) - 2u);
-        } else if (p.links) {
-          solid = __ldg(p.links + cell) & ((1u << Q) - 2u);
-        } else {
-          const TileCell t = {slot, b[0], b[1], b[2], fx, fy, fz, cell};
-          solid = link_code<Q>(p, t, phi) & ((1u << Q) - 2u);
-        }
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-          if (solid & (1u << i)) {
-            const float fo = __ldg(fp + (int64_t)L::opp(i) * p.P + cell);
-            const float corr =
-                2.f * L::w(i) * rhoW * ((float)L::ex(i) * us.x + (float)L::ey(i) * us.y + (float)L::ez(i) * us.z) * kInvCS2;
-            const float m = 2.f * fo + corr;
-            fbx += -(float)L::ex(i) * m;
-            fby += -(float)L::ey(i) * m;
-            fbz += -(float)L::ez(i) * m;
-          }
-        }
-      }
-      if (c.swept && fabsf(phi) < c.swept_band) {
-        const bool now = phi < 0.f;
-        if (now != (phi3_ahead(pos, c.body, 1.f, c.win) < 0.f)) {
-          float mcx = 0.f, mcy = 0.f, mcz = 0.f;
-#pragma unroll
-          for (int i = 0; i < Q; ++i) {
-            const float v = __ldg(fp + (int64_t)i * p.P + cell);
-            mcx += v * (float)L::ex(i); mcy += v * (float)L::ey(i); mcz += v * (float)L::ez(i);
-          }
-          if (!now) { fsx = mcx; fsy = mcy; fsz = mcz; }
-          else { fsx = -mcx; fsy = -mcy; fsz = -mcz; }
-        }
-      }
-    } else {
-      const float chi = chi_from_phi(phi, p.chi_eps_f);
-      if (chi >= 1e-6f) {
-        float rho = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-          const int sx = min(max(fx - L::ex(i), 0), p.FB - 1), sy = min(max(fy - L::ey(i), 0), p.FB - 1),
-                    sz = min(max(fz - L::ez(i), 0), p.FB - 1);
-          const float v = __ldg(fp + (int64_t)i * p.P + (int64_t)slot * p.T3 + (sz * p.FB + sy) * p.FB + sx);
-          rho += v;
-          mx += v * (float)L::ex(i); my += v * (float)L::ey(i); mz += v * (float)L::ez(i);
-        }
-        const float den = fmaxf(rho, 1e-6f);
-        fbx = -(rho * chi * (us.x - mx / den));
-        fby = -(rho * chi * (us.y - my / den));
-        fbz = -(rho * chi * (us.z - mz / den));
-      }
-    }
-    const float tx = fbx * 0.25f + fsx * 0.125f, ty = fby * 0.25f + fsy * 0.125f, tz = fbz * 0.25f + fsz * 0.125f;
-    const V3 r = body_delta(pos, c.body, c.win);
-    const float rx = r.x, ry = r.y, rz = r.z;
-    cf.fx = tx; cf.fy = ty; cf.fz = tz;
-    cf.tx = ry * tz - rz * ty;
-    cf.ty = rz * tx - rx * tz;
-    cf.tz = rx * ty - ry * tx;
-  }
-  ForceAcc acc;
-  acc.add(cf);
-  publish_force<kTileThreads>(acc, p.partials, blockIdx.y * gridDim.x + blockIdx.x);
-}
-
-// The pool force's partials summed in a fixed order (groups of kSumGroup,
-// then the groups), deterministic; a launch of its own, so that the force
-// CTAs publish their partials without a ticket and its fence.
-__global__ void __launch_bounds__(kSumGroup)
-    amr3_force_sum(const double *__restrict__ partials, int nparts, double *__restrict__ groups,
-                   unsigned int *__restrict__ counter, double *__restrict__ out) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
-  sum_partials_grouped<kSumGroup>(partials, nparts, groups, counter, out, blockIdx.x);
 }
 
 // ---- the refinement manager (common_d3_manage.wgsl) ------------------------
@@ -1103,6 +1151,78 @@ __global__ void __launch_bounds__(kManageThreads)
   }
 }
 
+// Per (chunk, slot): whether a ring cell has links into the body and is not
+// on hold (substep_cell).
+template <int Q>
+__global__ void __launch_bounds__(kListThreads)
+    amr3_need(const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells,
+              unsigned char *__restrict__ need) {
+  constexpr uint32_t kAll = (1u << Q) - 1u;
+  const int k = blockIdx.x * kListThreads + threadIdx.x, slot = blockIdx.y;
+  bool mine = false;
+  if (k < p.T3 && p.links && p.slot_to_block[slot] >= 0) {
+    const uint32_t c = __ldg(cells + k);
+    const int fx = c & 0xff, fy = (c >> 8) & 0xff, fz = (c >> 16) & 0xff;
+    const uint32_t code = p.links[(int64_t)slot * p.T3 + (fz * p.FB + fy) * p.FB + fx] & kAll;
+    mine = (c >> 24) != 13 && code && !(p.resting && code == kAll);
+  }
+  const int any = __syncthreads_or(mine);
+  if (threadIdx.x == 0) need[slot * gridDim.x + blockIdx.x] = any ? 1 : 0;
+}
+
+// The work lists, one CTA, after each change of the tiles or of the body: in
+// slot order, the chunks whose groups of cells (mask, one bit per neighbour
+// block, bit 13 the interior) hold a live one (the substeps'), those with a
+// live ring cell (explode's), and the substeps' with those that amr3_need
+// flagged; n their lengths.
+__global__ void __launch_bounds__(kManageThreads)
+    amr3_work(const int *__restrict__ block_slot, const int *__restrict__ slot_to_block,
+              const uint32_t *__restrict__ masks, int nch, int nbx, int nby, int nbz, int capacity,
+              const unsigned char *__restrict__ need, uint32_t *__restrict__ sub, uint32_t *__restrict__ expl,
+              uint32_t *__restrict__ with_need, int *__restrict__ n) {
+  __shared__ int sm[64];
+  int ns = 0, ne = 0, nw = 0;
+  for (int base = 0; base < capacity; base += kManageThreads) {
+    const int slot = base + threadIdx.x;
+    const int id = slot < capacity ? slot_to_block[slot] : -1;
+    uint32_t live = 0;  // the neighbours that hold no tile
+    if (id >= 0) {
+      const int bx = id % nbx, by = (id / nbx) % nby, bz = id / (nbx * nby);
+      for (int d = 0; d < 27; ++d) {
+        const int x = (bx + d % 3 - 1 + nbx) % nbx, y = (by + (d / 3) % 3 - 1 + nby) % nby,
+                  z = (bz + d / 9 - 1 + nbz) % nbz;
+        if (d != 13 && block_slot[(z * nby + y) * nbx + x] < 0) live |= 1u << d;
+      }
+    }
+    int cs = 0, ce = 0, cw = 0;
+    for (int c = 0; c < nch && id >= 0; ++c) {
+      const bool l = masks[c] & (live | 1u << 13);
+      cs += l;
+      ce += (masks[c] & live) != 0;
+      cw += l || need[slot * nch + c];
+    }
+    int ts, te, tw;
+    int rs = ns + block_scan(cs, sm, ts);
+    int re = ne + block_scan(ce, sm, te);
+    int rw = nw + block_scan(cw, sm, tw);
+    for (int c = 0; c < nch && id >= 0; ++c) {
+      const bool l = masks[c] & (live | 1u << 13);
+      const uint32_t item = (uint32_t)slot << 8 | c;
+      if (l) sub[rs++] = item;
+      if (masks[c] & live) expl[re++] = item;
+      if (l || need[slot * nch + c]) with_need[rw++] = item;
+    }
+    ns += ts;
+    ne += te;
+    nw += tw;
+  }
+  if (threadIdx.x == 0) {
+    n[0] = ns;
+    n[1] = ne;
+    n[2] = nw;
+  }
+}
+
 // ---- totals over the L0 mac ------------------------------------------------
 constexpr int kTotThreads = 256;
 __global__ void __launch_bounds__(kTotThreads)
@@ -1164,6 +1284,13 @@ struct lbm_amr3d {
   bool carved = false;          // device memory carved from a caller's block
   uint32_t *d_cells = nullptr;  // tile cells: interior (RB2^3) then ring, packed x | y << 8 | z << 16
   uint32_t *d_links = nullptr;  // bounce-back link code per pool cell (bounce-back bodies only)
+  // the work lists of the substeps and of explode (TileWork), their lengths
+  // on the device (dynamic) or in n_work, each chunk's groups of cells, and
+  // the chunks amr3_need flags
+  uint32_t *d_work[3] = {nullptr, nullptr, nullptr}, *d_masks = nullptr;
+  int *d_nwork = nullptr;
+  unsigned char *d_need = nullptr;
+  int n_work[3] = {0, 0, 0}, nch = 0;
   uint32_t *d_pulls = nullptr;  // substep pull sources per (direction, cell list position)
   int coalesce_subs = 1;        // threads per L0 cell in the coalesce
   float *d_block_q = nullptr;   // field criterion: per-block max Q (NULL = off)
@@ -1207,6 +1334,32 @@ cudaError_t launch_links(lbm_amr3d *a, const unsigned char *only_new) {
   AMR3_DISPATCH(a->q, amr3_links<Q><<<gl, kListThreads, 0, a->stream>>>(a->p, a->d_links, a->d_cells, only_new));
 }
 
+// The work lists for the current tiles and links.
+cudaError_t launch_work(lbm_amr3d *a) {
+  const Amr3Params &p = a->p;
+  const auto lists = [&] {
+    amr3_work<<<1, kManageThreads, 0, a->stream>>>(a->d_block_slot, a->d_slot_to_block, a->d_masks, a->nch, p.nbx, p.nby,
+                                                   p.nbz, a->capacity, a->d_need, a->d_work[0], a->d_work[1],
+                                                   a->d_work[2], a->d_nwork);
+  };
+  const dim3 g(a->nch, p.slots);
+  AMR3_DISPATCH(a->q, amr3_need<Q><<<g, kListThreads, 0, a->stream>>>(p, a->d_cells, a->d_need); lists());
+}
+
+// The same outside the manager's graph: a static hierarchy also learns its
+// lists' lengths, its launches' grids.
+int rebuild_work(lbm_amr3d *a) {
+  const bool bb = a->p.c.has_body && a->p.c.bb;
+  const lbm_body &b = a->p.c.body;
+  a->p.resting = bb && b.vx == 0.f && b.vy == 0.f && b.vz == 0.f && b.wx == 0.f && b.wy == 0.f && b.wz == 0.f;
+  a->p.live = a->cfg.iface != 1 && (!a->p.c.has_body || (bb && a->p.links)) ? 1 : 0;
+  ACK(a, launch_work(a));
+  if (a->dynamic) return LBM_OK;
+  ACK(a, cudaMemcpyAsync(a->n_work, a->d_nwork, sizeof(a->n_work), cudaMemcpyDeviceToHost, a->stream));
+  ACK(a, cudaStreamSynchronize(a->stream));
+  return LBM_OK;
+}
+
 // One decision of the manager before the macro-step from L0 parity `cp`
 // (main-3d.js:3247-3317): decide, drain the dying tiles into the time-t L0
 // buffer, free and grant slots, fill the new tiles from that buffer.
@@ -1242,6 +1395,7 @@ cudaError_t launch_manage(lbm_amr3d *a, int cp) {
                                            a->capacity);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = launch_links(a, a->d_slot_new)) != cudaSuccess) return e;
+  if ((e = launch_work(a)) != cudaSuccess) return e;
   return launch_interp(a, a->fc[cp], 0, a->d_slot_new);
 }
 
@@ -1263,6 +1417,8 @@ int coalesce_subs(const Amr3Params &p, int sms) {
   return subs;
 }
 
+// The macro-step's kernels are launched with launch_pdl (in a graph, a
+// programmatic edge) and wait at their first instruction.
 template <int Q>
 void launch_coalesce(cudaStream_t st, const float *fp, float *fc, float4 *macc, const float4 *macp,
                      const Amr3Params &p, int subs) {
@@ -1275,25 +1431,55 @@ void launch_coalesce(cudaStream_t st, const float *fp, float *fc, float4 *macc, 
   }
 }
 
-// A pool substep, with 32-bit population indices when the pool allows.
+// A pool substep, with 32-bit population indices when the pool allows, over
+// every cell, the live ones, or those and the dead ones with links.
+enum class Cells { kAll, kLive, kNeed };
 template <int Q>
-void launch_substep(dim3 gl, cudaStream_t st, const float *fin, float *fout, float4 *macp, const Amr3Params &p,
-                    const uint32_t *cells) {
-  if ((int64_t)Q * p.P <= INT32_MAX)
-    launch_pdl(gl, dim3(kListThreads), st, amr3_substep<Q, true>, fin, fout, macp, p, cells, p.T3);
-  else
-    launch_pdl(gl, dim3(kListThreads), st, amr3_substep<Q, false>, fin, fout, macp, p, cells, p.T3);
+void launch_substep(lbm_amr3d *a, cudaStream_t st, const float *fin, float *fout, const Amr3Params &p, Cells which) {
+  const bool live = which != Cells::kAll;
+  const int l = which == Cells::kNeed ? 2 : 0;
+  if (live && !a->n_work[l]) return;  // no tile
+  const dim3 g = live ? dim3(a->n_work[l]) : dim3(a->nch, p.slots);
+  const TileWork w = live ? TileWork{a->d_work[l], a->dynamic ? a->d_nwork + l : nullptr} : TileWork{nullptr, nullptr};
+  const uint32_t *cells = a->d_cells;
+  auto run = [&](auto k) {
+    launch_pdl(g, dim3(kListThreads), st, k, fin, fout, a->macp, p, cells, w, which == Cells::kNeed ? 1 : 0);
+  };
+  if ((int64_t)Q * p.P <= INT32_MAX) {
+    if (live) run(amr3_substep<Q, true, true>);
+    else run(amr3_substep<Q, true, false>);
+  } else {
+    if (live) run(amr3_substep<Q, false, true>);
+    else run(amr3_substep<Q, false, false>);
+  }
 }
 
-// The pool force at time t and its deterministic sum.
+// The pool force at time t as a launch of its own.
 template <int Q>
 void launch_pool_force(lbm_amr3d *a, const Amr3Params &p, cudaStream_t st) {
-  const int r3 = p.RB2 * p.RB2 * p.RB2;
-  const dim3 gf((r3 + kTileThreads - 1) / kTileThreads, p.slots);
-  launch_pdl(gf, dim3(kTileThreads), st, amr3_force<Q>, (const float *)a->fp[0], p, (const uint32_t *)a->d_cells);
-  const int parts = gf.x * gf.y;
-  launch_pdl(dim3(sum_groups(parts)), dim3(kSumGroup), st, amr3_force_sum, (const double *)a->partials, parts,
-             a->force_groups, a->counter, a->force_out);
+  launch_pdl(dim3(force_chunks(p), p.slots), dim3(kTileThreads), st, amr3_force<Q>, (const float *)a->fp[0], p,
+             (const uint32_t *)a->d_cells);
+}
+
+// The L0 step; with a body its first blocks sum the pool force's partials in
+// a fixed order (sum_partials_grouped), so the force CTAs publish them
+// without a ticket and no launch of its own adds them.
+template <int Q>
+void launch_coarse(lbm_amr3d *a, int cp, bool write_mac, cudaStream_t st) {
+  StepParams sp = a->sp;
+  sp.write_mac = write_mac ? 1 : 0;
+  if (a->p.slots && sp.has_body) {
+    sp.prev_parts = force_chunks(a->p) * a->p.slots;
+    sp.prev_partials = a->partials;
+    sp.groups = a->force_groups;
+    sp.counter = a->counter;
+    sp.force_out = a->force_out;
+  }
+  dim3 grid = step_grid(sp);
+  sp.sum_layers = sum_layers_for(sp, grid.x * grid.y);
+  grid.z += sp.sum_layers;
+  launch_pdl(grid, dim3(kStepThreads), st, amr3_coarse<Q>, (const float *)a->fc[cp], a->fc[1 - cp], a->macc,
+             sp, (const int *)a->d_block_slot, row_magic(a->p.rb), a->p.nbx, a->p.nby);
 }
 
 // One macro-step from L0 parity `cp`.
@@ -1307,29 +1493,22 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
     // ?interface=interp (main-3d.js:3343-3356): the L0 step first, then the
     // ring interpolated from L0 at t, two substeps with the ring collided,
     // and every tile restricted into L0's new buffer.
-    StepParams sp = a->sp;
-    sp.write_mac = write_mac ? 1 : 0;
-    const dim3 gs = step_grid(sp);
     const dim3 g = tile_grid(a);
-    const dim3 gl((p.T3 + kListThreads - 1) / kListThreads, p.slots);
     const int rb3 = p.rb * p.rb * p.rb;
     const dim3 gd((rb3 + kTileThreads - 1) / kTileThreads, p.slots);
-    const int r3 = p.RB2 * p.RB2 * p.RB2;
-    const dim3 gf((r3 + kTileThreads - 1) / kTileThreads, p.slots);
     const float tc = a->cfg.root.tau, tf = 2.f * tc - 0.5f;
     const float f2c_rescale = 2.f * (tc - 1.f) / (tf - 1.f);
     AMR3_DISPATCH(q, {
       if (p.c.has_body) launch_pool_force<Q>(a, p, st);
-      amr3_coarse<Q><<<gs, kStepThreads, 0, st>>>(a->fc[cp], a->fc[1 - cp], a->macc, sp, a->d_block_slot,
-                                                   row_magic(p.rb), p.nbx, p.nby);
+      launch_coarse<Q>(a, cp, write_mac, st);
       amr3_interp<Q><<<g, tile_block(a), 0, st>>>(a->fc[cp], a->fp[0], p, 1, nullptr);
       Amr3Params pa = p;
       pa.write_mac = 0;
       const int gc = (p.n_iface * rb3 + kTileThreads - 1) / kTileThreads;
       if (a->flux && gc) amr3_flux<Q><<<gc, kTileThreads, 0, st>>>(a->fp[0], a->flux, p, 0);
-      launch_substep<Q>(gl, st, a->fp[0], a->fp[1], a->macp, pa, a->d_cells);
+      launch_substep<Q>(a, st, a->fp[0], a->fp[1], pa, Cells::kAll);
       if (a->flux && gc) amr3_flux<Q><<<gc, kTileThreads, 0, st>>>(a->fp[1], a->flux, p, 1);
-      launch_substep<Q>(gl, st, a->fp[1], a->fp[0], a->macp, p, a->d_cells);
+      launch_substep<Q>(a, st, a->fp[1], a->fp[0], p, Cells::kAll);
       amr3_drain<Q><<<gd, kTileThreads, 0, st>>>(a->fp[0], a->fc[1 - cp], (float4 *)a->macc, p, nullptr,
                                                  f2c_rescale);
       if (a->flux && gc)
@@ -1337,18 +1516,25 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
     });
   }
   if (p.slots) {
-    const dim3 gl((p.T3 + kListThreads - 1) / kListThreads, p.slots);
+    // the last macro-step of a call leaves every cell up to date
+    const Cells most = p.resting || !p.c.has_body ? Cells::kLive : Cells::kNeed;
+    const Cells first = !p.live ? Cells::kAll : (write_mac ? Cells::kNeed : most);
+    const Cells second = !p.live || write_mac ? Cells::kAll : most;
     auto body = [&]() -> cudaError_t {
       AMR3_DISPATCH(q, {
-        if (p.c.has_body) launch_pool_force<Q>(a, p, st);
-        const int r3i = p.RB2 * p.RB2 * p.RB2, nring = p.T3 - r3i;
-        const dim3 gr((nring + kListThreads - 1) / kListThreads, p.slots);
-        launch_pdl(gr, dim3(kListThreads), st, amr3_explode<Q>, (const float *)a->fc[cp], a->fp[0], p,
-                   (const uint32_t *)a->d_cells, r3i, nring);
+        // the penalty's force gather reads ring cells, which the explode
+        // overwrites: a launch of its own before it
+        const bool joint = p.c.has_body && p.c.bb;
+        if (p.c.has_body && !joint) launch_pool_force<Q>(a, p, st);
+        const int nforce = joint ? force_chunks(p) * p.slots : 0;
+        if (a->n_work[1] + nforce)
+          launch_pdl(dim3(a->n_work[1] + nforce), dim3(kListThreads), st, amr3_explode<Q>, (const float *)a->fc[cp],
+                     a->fp[0], p, (const uint32_t *)a->d_cells,
+                     TileWork{a->d_work[1], a->dynamic ? a->d_nwork + 1 : nullptr}, nforce);
         Amr3Params pa = p;
         pa.write_mac = 0;
-        launch_substep<Q>(gl, st, a->fp[0], a->fp[1], a->macp, pa, a->d_cells);
-        launch_substep<Q>(gl, st, a->fp[1], a->fp[0], a->macp, p, a->d_cells);
+        launch_substep<Q>(a, st, a->fp[0], a->fp[1], pa, first);
+        launch_substep<Q>(a, st, a->fp[1], a->fp[0], p, second);
         if (p.n_iface)
           launch_coalesce<Q>(st, a->fp[0], a->fc[cp], (float4 *)a->macc, a->macp, p, a->coalesce_subs);
       });
@@ -1356,11 +1542,7 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
     e = body();
     if (e != cudaSuccess) return e;
   }
-  StepParams sp = a->sp;
-  sp.write_mac = write_mac ? 1 : 0;
-  const dim3 gs = step_grid(sp);
-  AMR3_DISPATCH(q, launch_pdl(gs, dim3(kStepThreads), st, amr3_coarse<Q>, (const float *)a->fc[cp], a->fc[1 - cp],
-                              a->macc, sp, (const int *)a->d_block_slot, row_magic(p.rb), p.nbx, p.nby));
+  AMR3_DISPATCH(q, launch_coarse<Q>(a, cp, write_mac, st));
 }
 
 void destroy_graphs(lbm_amr3d *a) {
@@ -1423,7 +1605,8 @@ void release(lbm_amr3d *a) {
                     (void *)a->counter, (void *)a->tot_counter, (void *)a->d_want, (void *)a->d_slot_new,
                     (void *)a->d_iface_flag, (void *)a->d_free_list, (void *)a->d_counts, (void *)a->flux,
                     (void *)a->d_block_q, (void *)a->d_cells, (void *)a->d_links, (void *)a->d_pulls,
-                    (void *)a->force_groups})
+                    (void *)a->force_groups, (void *)a->d_work[0], (void *)a->d_work[1], (void *)a->d_masks,
+                    (void *)a->d_nwork, (void *)a->d_need})
     if (!a->carved) cudaFree(ptr);
   if (a->host_out) cudaFreeHost(a->host_out);
   if (a->own) cudaStreamDestroy(a->own);
@@ -1470,7 +1653,7 @@ std::vector<uint32_t> pull_table(int q, int FB, int RB2, const std::vector<uint3
   const int G = kAmrGhost, n = (int)cl.size(), kw = pull_words(q);
   std::vector<uint32_t> t((size_t)kw * n, 0u);
   for (int k = 0; k < n; ++k) {
-    const int fi[3] = {(int)(cl[k] & 0xff), (int)((cl[k] >> 8) & 0xff), (int)(cl[k] >> 16)};
+    const int fi[3] = {(int)(cl[k] & 0xff), (int)((cl[k] >> 8) & 0xff), (int)((cl[k] >> 16) & 0xff)};
     for (int i = 0; i < q; ++i) {
       const int e[3] = {detail::ex27(i), detail::ey27(i), detail::ez27(i)};
       int o[3], sh[3], sc[3];
@@ -1488,6 +1671,24 @@ std::vector<uint32_t> pull_table(int q, int FB, int RB2, const std::vector<uint3
     }
   }
   return t;
+}
+
+// The tile's cells, x | y << 8 | z << 16 | neighbour block << 24: the
+// interior (neighbour 13), then the ring by the block it lies in, faces
+// before edges before corners; z-, y-, x-major within each.
+std::vector<uint32_t> tile_cells(int FB, int RB2) {
+  std::vector<uint32_t> by[27], out;
+  auto side = [&](int j) { return j < kAmrGhost ? 0 : (j < kAmrGhost + RB2 ? 1 : 2); };
+  for (int z = 0; z < FB; ++z)
+    for (int y = 0; y < FB; ++y)
+      for (int x = 0; x < FB; ++x) {
+        const int g = side(z) * 9 + side(y) * 3 + side(x);
+        by[g].push_back(x | (y << 8) | (z << 16) | (uint32_t)g << 24);
+      }
+  for (int rank = 0; rank <= 3; ++rank)
+    for (int g = 0; g < 27; ++g)
+      if ((g % 3 != 1) + (g / 3 % 3 != 1) + (g / 9 != 1) == rank) out.insert(out.end(), by[g].begin(), by[g].end());
+  return out;
 }
 
 // Builds the hierarchy with its device memory from `mem`; with mem.measure
@@ -1575,7 +1776,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
   p.linear = c->explode_linear ? 1 : 0;
   p.collide_ring = c->iface == 1 ? 1 : 0;
   fill_step_params(r, p.N, 0, a->sp);
-  a->sp.force_on = 0;
+  set_body_regions(r, a->sp, false);  // the reach box of the L0 step
   {
     StepParams tmp = a->sp;
     int box[6];
@@ -1593,6 +1794,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
   cudaError_t e;
   const bool live = !mem.measure;
   a->carved = mem.base != nullptr;
+  a->nch = (p.T3 + kListThreads - 1) / kListThreads;
   const size_t fcb = (size_t)a->q * p.N * sizeof(float), fpb = (size_t)a->q * p.P * sizeof(float);
   const int nfree = a->capacity - a->initial;
   const size_t nfl = (size_t)std::max(1, a->capacity);
@@ -1610,6 +1812,11 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
     if ((e = mem.take(&a->d_iface, std::max(p.n_iface, 1) * sizeof(int)))) return bail(e, "iface");
     if ((e = mem.take(&a->d_cells, (size_t)p.T3 * sizeof(uint32_t)))) return bail(e, "cell list");
     if ((e = mem.take(&a->d_pulls, (size_t)pull_words(a->q) * p.T3 * sizeof(uint32_t)))) return bail(e, "pull table");
+    for (auto *&w : a->d_work)
+      if ((e = mem.take(&w, (size_t)a->capacity * a->nch * sizeof(uint32_t)))) return bail(e, "work list");
+    if ((e = mem.take(&a->d_masks, a->nch * sizeof(uint32_t)))) return bail(e, "work list");
+    if ((e = mem.take(&a->d_nwork, 3 * sizeof(int)))) return bail(e, "work list");
+    if ((e = mem.take(&a->d_need, (size_t)a->capacity * a->nch))) return bail(e, "work list");
     if (r.has_body && r.use_bounceback && (e = mem.take(&a->d_links, (size_t)p.P * sizeof(uint32_t))))
       return bail(e, "link table");
     if (a->dynamic) {
@@ -1620,8 +1827,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
       if ((e = mem.take(&a->d_counts, 4 * sizeof(int)))) return bail(e, "counts");
       if (c->q_abs > 0 && (e = mem.take(&a->d_block_q, nb * sizeof(float)))) return bail(e, "block Q");
     }
-    const int r3 = p.RB2 * p.RB2 * p.RB2;
-    a->force_parts = std::max(1, ((r3 + kTileThreads - 1) / kTileThreads) * p.slots);
+    a->force_parts = std::max(1, force_chunks(p) * p.slots);
     if ((e = mem.take(&a->partials, (size_t)a->force_parts * kForceSlots * sizeof(double)))) return bail(e, "partials");
     if ((e = mem.take(&a->force_out, kForceSlots * sizeof(double)))) return bail(e, "force");
     if ((e = mem.take(&a->force_groups, (size_t)sum_groups(a->force_parts) * kForceSlots * sizeof(double))))
@@ -1647,18 +1853,16 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
   cudaMemcpyAsync(a->d_slot_to_block, a->slot_to_block.data(), a->capacity * sizeof(int), cudaMemcpyHostToDevice,
                   a->own);
   {
-    std::vector<uint32_t> cl;
-    cl.reserve(p.T3);
-    for (int pass = 0; pass < 2; ++pass)
-      for (int z = 0; z < p.FB; ++z)
-        for (int y = 0; y < p.FB; ++y)
-          for (int x = 0; x < p.FB; ++x) {
-            auto in = [&](int j) { return j >= kAmrGhost && j < kAmrGhost + p.RB2; };
-            if ((in(x) && in(y) && in(z)) == (pass == 0)) cl.push_back(x | (y << 8) | (z << 16));
-          }
+    const std::vector<uint32_t> cl = tile_cells(p.FB, p.RB2);
     cudaMemcpyAsync(a->d_cells, cl.data(), cl.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, a->own);
     const std::vector<uint32_t> pt = pull_table(a->q, p.FB, p.RB2, cl);
     cudaMemcpyAsync(a->d_pulls, pt.data(), pt.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, a->own);
+    // the work lists follow when the hierarchy is seeded; a dynamic one's grow
+    // up to every chunk of every slot
+    std::vector<uint32_t> masks(a->nch, 0u);
+    for (int k = 0; k < p.T3; ++k) masks[k / kListThreads] |= 1u << (cl[k] >> 24);
+    for (int &n : a->n_work) n = a->dynamic ? a->capacity * a->nch : 0;
+    cudaMemcpyAsync(a->d_masks, masks.data(), masks.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, a->own);
   }
   if (a->dynamic) {
     std::vector<unsigned char> flag(nb, 0);
@@ -1760,6 +1964,7 @@ int lbm_amr3d_init_macro(lbm_amr3d *a, const float *mac) {
     ACK(a, launch_init_eq(a->q, LBM_STORE_FP32, a->macc, a->fc[k], a->p.N, a->sp.pk, a->stream));
   ACK(a, launch_interp(a, a->fc[0], 0, nullptr));
   ACK(a, launch_links(a, nullptr));
+  if (int rc = rebuild_work(a)) return rc;
   ACK(a, launch_moments(a));
   ACK(a, cudaStreamSynchronize(a->stream));
   a->cp = 0;
@@ -1814,6 +2019,7 @@ int lbm_amr3d_set_body(lbm_amr3d *a, const lbm_body *body) {
   ACK(a, cudaStreamSynchronize(a->stream));
   a->cfg.root = r;
   a->sp.body = *body;
+  set_body_regions(r, a->sp, false);
   StepParams tmp = a->sp;
   int box[6];
   force_cell_box(r, tmp, box);
@@ -1821,8 +2027,9 @@ int lbm_amr3d_set_body(lbm_amr3d *a, const lbm_body *body) {
   a->sp.swept_band = tmp.swept_band;
   a->p.c = a->sp;
   destroy_graphs(a);
-  if (a->seeded) ACK(a, launch_links(a, nullptr));
-  return LBM_OK;
+  if (!a->seeded) return LBM_OK;
+  ACK(a, launch_links(a, nullptr));
+  return rebuild_work(a);
 }
 
 int lbm_amr3d_set_links(lbm_amr3d *a, int on) {
@@ -1830,8 +2037,9 @@ int lbm_amr3d_set_links(lbm_amr3d *a, int on) {
   ACK(a, cudaStreamSynchronize(a->stream));
   destroy_graphs(a);
   a->p.links = on ? a->d_links : nullptr;
-  if (a->seeded) ACK(a, launch_links(a, nullptr));
-  return LBM_OK;
+  if (!a->seeded) return LBM_OK;
+  ACK(a, launch_links(a, nullptr));
+  return rebuild_work(a);
 }
 
 int lbm_amr3d_links(const lbm_amr3d *a) { return a && a->p.links ? 1 : 0; }

@@ -37,6 +37,8 @@ struct Amr3Params {
   float chi_eps_f;              // the chi band on the fine level (CHI_EPS / 2)
   int linear;                   // linear explosion
   int collide_ring;             // interp interface: the ring collides (COLLIDE_RING = 1)
+  int live;                     // dead ring cells are skipped (TileWork, amr3d.cu)
+  int resting;                  // bounce-back body with no velocity
   int write_mac;
   double *partials;             // pool force: 8 doubles per force CTA
   unsigned int *counter;

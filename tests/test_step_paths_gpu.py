@@ -5,7 +5,9 @@ or topology selects, a cell gets the same bits.
   kinds, against the same domain in a batch, which updates one cell per
   thread by plain indices;
 * the D2Q9 reach box, against the batch, which evaluates the body everywhere;
-* a free body that is pinned, against the prescribed pose.
+* a free body that is pinned, against the prescribed pose;
+* 3D AMR macro-steps over the live chunks only, against single macro-steps,
+  whose last substep covers every tile cell.
 """
 import numpy as np
 import pytest
@@ -107,3 +109,28 @@ def test_pinned_free_body_equals_prescribed_pose(lbm, shape, bb, storage):
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
     assert np.allclose(out[0][2], out[1][2], rtol=1e-10, atol=1e-12 * np.abs(out[0][2]).max())
+
+
+@pytest.mark.parametrize("q,rb,dynamic,shape", [(19, 4, 0, "roundbox"), (27, 4, 0, "sphere"), (19, 2, 0, "sphere"),
+                                                (19, 3, 0, "roundbox"), (19, 4, 1, "sphere")])
+def test_amr3d_live_chunks_equal_whole_tiles(lbm, q, rb, dynamic, shape):
+    from getting_air_b200 import scenarios as sc
+    dims = (12 * rb, 8 * rb, 8 * rb)
+    kw = dict(tau=0.62, has_body=1, use_bounceback=1, sponge_w=4.0, sponge_u=(0.04, 0.0, 0.0),
+              body=dict(shape=shape, centre=(4.3 * rb, 4.0 * rb, 3.9 * rb), a=1.6 * rb, b=1.4 * rb, c=1.4 * rb,
+                        r=0.3 * rb if shape == "roundbox" else 0.0, v=(0.2 if dynamic else 0.0, 0.0, 0.0)))
+    runs = []
+    for single in (False, True):
+        a = lbm.Amr3D(lbm.amr3d_config(q, dims, refine="body", rb=rb, margin=2.0, dynamic=dynamic, manage_every=3,
+                                       slot_headroom=2.0, **kw))
+        a.init_macro(sc.uniform_macro(int(np.prod(dims)), (0.04, 0.0, 0.0)))
+        for _ in range(2):
+            for k in range(7 if single else 1):
+                a.step(1 if single else 7)
+            body = lbm.make_body(**dict(kw["body"], centre=(4.3 * rb + (3.0 if dynamic else 0.0), 4.0 * rb, 3.9 * rb)))
+            a.set_body(body)
+        runs.append(a.read_coarse() + a.read_pool() + (a.forces(), a.topology()["block_slot"]))
+        a.close()
+    for x, y in zip(*runs):
+        assert np.array_equal(x, y)
+    assert abs(runs[0][4][0]) > 0
