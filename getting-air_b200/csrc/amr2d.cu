@@ -24,6 +24,7 @@
 // the device), so the non-refine macro-step is topology-independent and is
 // replayed from a CUDA graph.
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -66,6 +67,23 @@ struct AmrParams {
 
 using L9 = Lattice<9>;
 
+// A population, through the read-only path (CG = false: the buffer does not
+// change during the kernel) or from L2 (CG: another block of this launch may
+// have written it; only amr_macro_loop).
+template <bool CG> __device__ __forceinline__ float ldf(const float *p) { return CG ? __ldcg(p) : __ldg(p); }
+
+// The slots of the 3 x 3 blocks around block (bx, by), by threads 0..8 (index
+// (dy + 1) * 3 + dx + 1); the caller synchronises.
+__device__ __forceinline__ void load_nb9(const AmrParams &p, int bx, int by, int *nb9) {
+  if (threadIdx.x < 9) {
+    const int k = threadIdx.x;
+    int x = bx + k % 3 - 1, y = by + k / 3 - 1;
+    x = x < 0 ? x + p.NBX : (x >= p.NBX ? x - p.NBX : x);
+    y = y < 0 ? y + p.NBY : (y >= p.NBY ? y - p.NBY : y);
+    nb9[k] = p.blockSlot[y * p.NBX + x];
+  }
+}
+
 __device__ __forceinline__ float feq9(float rho, float ux, float uy, int i) {
   const float eu = (float)L9::ex(i) * ux + (float)L9::ey(i) * uy;
   return L9::w(i) * rho * (1.f + 3.f * eu + 4.5f * eu * eu - 1.5f * (ux * ux + uy * uy));
@@ -84,7 +102,10 @@ __device__ __forceinline__ int64_t pcell(const AmrParams &p, int slot, int fx, i
 // Max |discrete curl| of the root velocity over each level-1 block's RB x RB
 // root cells (amr_criterion_pool.wgsl, GHOST == 0 branch). Every operation is
 // rounded on its own so the value is reproducible bit for bit.
+// Also clears the flags of newly granted slots for the round.
 __global__ void amr_criterion(const float4 *__restrict__ mac, const __grid_constant__ AmrParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < p.S; k += gridDim.x * blockDim.x) p.newly[k] = 0u;
   const int b = blockIdx.x;
   const int bx = b % p.NBX, by = b / p.NBX;
   float m = 0.f;
@@ -147,6 +168,7 @@ __device__ bool near_body_box(const AmrParams &p, float cx, float cy, float half
 // the body is within the margin of the block (now or lookahead steps on) or
 // the block's vorticity reaches the refine threshold.
 __global__ void amr_decide(const __grid_constant__ AmrParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
   const int pb = blockIdx.x * blockDim.x + threadIdx.x;
   if (pb >= p.PNX * p.PNY) return;
   const int bxP = pb % p.PNX, byP = pb / p.PNX;
@@ -170,6 +192,7 @@ __global__ void amr_decide(const __grid_constant__ AmrParams p) {
 constexpr int kManageThreads = 1024;
 
 __global__ void __launch_bounds__(kManageThreads) amr_coarsen_refine(const __grid_constant__ AmrParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
   __shared__ int sm[64];
   int count = p.counts[0];
   // coarsen: quads whose first block is no longer wanted
@@ -242,15 +265,12 @@ struct Sample {
   float rho, ux, uy, fneq[9];
 };
 
-__device__ __forceinline__ void sample_root(const AmrParams &p, const float *__restrict__ f0, int gx, int gy,
-                                            Sample &s) {
-  gx = ((gx % p.W) + p.W) % p.W;
-  gy = ((gy % p.H) + p.H) % p.H;
-  const int64_t cell = (int64_t)gy * p.W + gx;
+template <bool CG>
+__device__ __forceinline__ void sample_root(const AmrParams &p, const float *__restrict__ f0, unsigned cell, Sample &s) {
   float f[9], rho = 0.f, ux = 0.f, uy = 0.f;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
-    f[i] = __ldg(f0 + i * p.N0 + cell);
+    f[i] = ldf<CG>(f0 + i * p.N0 + cell);
     rho += f[i];
     ux += f[i] * (float)L9::ex(i);
     uy += f[i] * (float)L9::ey(i);
@@ -262,53 +282,72 @@ __device__ __forceinline__ void sample_root(const AmrParams &p, const float *__r
   for (int i = 0; i < 9; ++i) s.fneq[i] = f[i] - feq9(rho, ux, uy, i);
 }
 
-// Bilinear rho, u, fneq from the four root cells around the pool cell,
-// f = feq + 0.5 (tf-1)/(tc-1) fneq (common_interp.wgsl interpCoarseToFine).
-__device__ void interp_cell(const AmrParams &p, const float *__restrict__ f0, float *__restrict__ f1, int slot,
-                            int bx, int by, int fx, int fy) {
+// Where a pool cell is filled from: the four root cells around it with the
+// bilinear offsets, or (copy) a same-level neighbour's interior cell src[0].
+struct FillGeo {
+  unsigned cell, src[4];
+  float tx, ty;
+  bool copy;
+};
+
+__device__ __forceinline__ FillGeo interp_geo(const AmrParams &p, int slot, int bx, int by, int fx, int fy) {
+  FillGeo g;
   const float px = pool_pos(p, bx, fx), py = pool_pos(p, by, fy);
   const int x0 = (int)floorf(px), y0 = (int)floorf(py);
-  const float tx = px - (float)x0, ty = py - (float)y0;
-  Sample s00, s10, s01, s11;
-  sample_root(p, f0, x0, y0, s00);
-  sample_root(p, f0, x0 + 1, y0, s10);
-  sample_root(p, f0, x0, y0 + 1, s01);
-  sample_root(p, f0, x0 + 1, y0 + 1, s11);
-  const float w00 = (1.f - tx) * (1.f - ty), w10 = tx * (1.f - ty), w01 = (1.f - tx) * ty, w11 = tx * ty;
-  const float rho = w00 * s00.rho + w10 * s10.rho + w01 * s01.rho + w11 * s11.rho;
-  const float ux = w00 * s00.ux + w10 * s10.ux + w01 * s01.ux + w11 * s11.ux;
-  const float uy = w00 * s00.uy + w10 * s10.uy + w01 * s01.uy + w11 * s11.uy;
-  const int64_t cell = pcell(p, slot, fx, fy);
+  g.tx = px - (float)x0;
+  g.ty = py - (float)y0;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    const float fneq = w00 * s00.fneq[i] + w10 * s10.fneq[i] + w01 * s01.fneq[i] + w11 * s11.fneq[i];
-    f1[i * p.N1 + cell] = feq9(rho, ux, uy, i) + p.resc_c2f * fneq;
+  for (int k = 0; k < 4; ++k) {
+    const int gx = (((x0 + (k & 1)) % p.W) + p.W) % p.W, gy = (((y0 + (k >> 1)) % p.H) + p.H) % p.H;
+    g.src[k] = (unsigned)(gy * p.W + gx);
   }
+  g.cell = (unsigned)pcell(p, slot, fx, fy);
+  g.copy = false;
+  return g;
 }
 
 // One ring cell of tile `s` (block bx, by): the same-level neighbour's
 // interior cell when that neighbour is refined, else root interpolation.
-__device__ __forceinline__ void fill_ring_cell(const AmrParams &p, const float *__restrict__ f0,
-                                               float *__restrict__ f1, int s, int bx, int by, int fx, int fy) {
-  const int bxm = (bx + p.NBX - 1) % p.NBX, bxp = (bx + 1) % p.NBX;
-  const int bym = (by + p.NBY - 1) % p.NBY, byp = (by + 1) % p.NBY;
+__device__ __forceinline__ FillGeo ring_geo(const AmrParams &p, const int *nb9, int s, int bx, int by, int fx, int fy) {
   const int G = p.G, RB2 = p.RB2;
-  const bool inX = fx >= G && fx < G + RB2, inY = fy >= G && fy < G + RB2;
-  int ns, nfx = fx, nfy = fy;
-  if (inY && fx < G) { ns = p.blockSlot[by * p.NBX + bxm]; nfx = fx + RB2; }
-  else if (inY && fx >= G + RB2) { ns = p.blockSlot[by * p.NBX + bxp]; nfx = fx - RB2; }
-  else if (inX && fy < G) { ns = p.blockSlot[bym * p.NBX + bx]; nfy = fy + RB2; }
-  else if (inX && fy >= G + RB2) { ns = p.blockSlot[byp * p.NBX + bx]; nfy = fy - RB2; }
-  else if (fx < G && fy < G) { ns = p.blockSlot[bym * p.NBX + bxm]; nfx = fx + RB2; nfy = fy + RB2; }
-  else if (fx >= G + RB2 && fy < G) { ns = p.blockSlot[bym * p.NBX + bxp]; nfx = fx - RB2; nfy = fy + RB2; }
-  else if (fx < G && fy >= G + RB2) { ns = p.blockSlot[byp * p.NBX + bxm]; nfx = fx + RB2; nfy = fy - RB2; }
-  else { ns = p.blockSlot[byp * p.NBX + bxp]; nfx = fx - RB2; nfy = fy - RB2; }
-  if (ns >= 0) {
-    const int64_t dst = pcell(p, s, fx, fy), src = pcell(p, ns, nfx, nfy);
+  const int ox = fx < G ? -1 : (fx >= G + RB2 ? 1 : 0), oy = fy < G ? -1 : (fy >= G + RB2 ? 1 : 0);
+  const int ns = nb9[(oy + 1) * 3 + ox + 1];
+  if (ns < 0) return interp_geo(p, s, bx, by, fx, fy);
+  FillGeo g{};
+  g.cell = (unsigned)pcell(p, s, fx, fy);
+  g.src[0] = (unsigned)pcell(p, ns, fx - ox * RB2, fy - oy * RB2);
+  g.copy = true;
+  return g;
+}
+
+// Bilinear rho, u, fneq from the four root cells around the pool cell,
+// f = feq + 0.5 (tf-1)/(tc-1) fneq (common_interp.wgsl interpCoarseToFine);
+// or the neighbour's cell.
+template <bool CG>
+__device__ __forceinline__ void fill_cell(const AmrParams &p, const FillGeo &g, const float *__restrict__ f0,
+                                          float *f1) {
+  if (g.copy) {
+    float v[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) f1[i * p.N1 + dst] = f1[i * p.N1 + src];
-  } else {
-    interp_cell(p, f0, f1, s, bx, by, fx, fy);
+    for (int i = 0; i < 9; ++i) v[i] = __ldcg(f1 + i * p.N1 + g.src[0]);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) f1[i * p.N1 + g.cell] = v[i];
+    return;
+  }
+  const float tx = g.tx, ty = g.ty;
+  Sample s00, s10, s01, s11;
+  sample_root<CG>(p, f0, g.src[0], s00);
+  sample_root<CG>(p, f0, g.src[1], s10);
+  sample_root<CG>(p, f0, g.src[2], s01);
+  sample_root<CG>(p, f0, g.src[3], s11);
+  const float w00 = (1.f - tx) * (1.f - ty), w10 = tx * (1.f - ty), w01 = (1.f - tx) * ty, w11 = tx * ty;
+  const float rho = w00 * s00.rho + w10 * s10.rho + w01 * s01.rho + w11 * s11.rho;
+  const float ux = w00 * s00.ux + w10 * s10.ux + w01 * s01.ux + w11 * s11.ux;
+  const float uy = w00 * s00.uy + w10 * s10.uy + w01 * s01.uy + w11 * s11.uy;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    const float fneq = w00 * s00.fneq[i] + w10 * s10.fneq[i] + w01 * s01.fneq[i] + w11 * s11.fneq[i];
+    f1[i * p.N1 + g.cell] = feq9(rho, ux, uy, i) + p.resc_c2f * fneq;
   }
 }
 
@@ -316,6 +355,8 @@ __device__ __forceinline__ void fill_ring_cell(const AmrParams &p, const float *
 // interpolation); mode 1: every cell of the tiles activated this round.
 __global__ void __launch_bounds__(kChunk)
     amr_fill(const float *__restrict__ f0, float *__restrict__ f1, int mode, const __grid_constant__ AmrParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
+  __shared__ int nb9[9];
   const int n = p.counts[1];
   const int FB2 = p.FB * p.FB, nch = (FB2 + kChunk - 1) / kChunk;
   for (int w = blockIdx.x; w < n * nch; w += gridDim.x) {
@@ -324,55 +365,59 @@ __global__ void __launch_bounds__(kChunk)
     if (mode == 1 && !p.newly[s]) continue;
     const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
     const int G = p.G, RB2 = p.RB2, FB = p.FB;
+    __syncthreads();
+    load_nb9(p, bx, by, nb9);
+    __syncthreads();
     for (int c = c0 + threadIdx.x; c < c1; c += kChunk) {
       const int fx = c % FB, fy = c / FB;
       const bool inX = fx >= G && fx < G + RB2, inY = fy >= G && fy < G + RB2;
       if (mode == 1) {
-        interp_cell(p, f0, f1, s, bx, by, fx, fy);
+        fill_cell<false>(p, interp_geo(p, s, bx, by, fx, fy), f0, f1);
         continue;
       }
       if (inX && inY) continue;
-      fill_ring_cell(p, f0, f1, s, bx, by, fx, fy);
+      fill_cell<false>(p, ring_geo(p, nb9, s, bx, by, fx, fy), f0, f1);
     }
   }
 }
 
-// One pool substep (amr_step1.wgsl stepCell): DIRECT_GHOST pull (a source
-// past the tile interior comes from the same-level neighbour's interior when
-// that neighbour is refined, else from this tile's ring), BGK + Guo at
-// tau_f with the chi penalty on this level's band, sponge, SOLID_EQ. Every
-// cell of the tile, ring included, collides (COLLIDE_RING = 1).
-__device__ __forceinline__ void substep_cell(const AmrParams &p, const float *__restrict__ fin,
-                                             float *__restrict__ fout, float2 *__restrict__ vel1, int s, int bx,
-                                             int by, int fx, int fy) {
+// What a pool cell's substep needs beyond populations, constant while the
+// tiles and the body are: the source of each pull, the body's band and
+// velocity there, the links that bounce back, the sponge weight.
+enum : unsigned { kGeoRing = 1u << 16, kGeoSolid = 1u << 17 };
+
+struct SubGeo {
+  unsigned cell, src[9];  // pool cells (fewer than 2^32 of 9 planes fit any GPU)
+  unsigned flags;         // bits 0-8: solid links; kGeoRing, kGeoSolid (phi < 0)
+  float usx, usy, chi, sw;
+};
+
+// DIRECT_GHOST pull (amr_step1.wgsl stepCell): a source past the tile
+// interior comes from the same-level neighbour's interior when that neighbour
+// is refined, else from this tile's ring.
+__device__ __forceinline__ SubGeo sub_geo(const AmrParams &p, const int *nb9, int s, int bx, int by, int fx, int fy) {
+  SubGeo g;
   const float Wf = (float)p.W, Hf = (float)p.H;
-  const int bxm = (bx + p.NBX - 1) % p.NBX, bxp = (bx + 1) % p.NBX;
-  const int bym = (by + p.NBY - 1) % p.NBY, byp = (by + 1) % p.NBY;
   const int G = p.G, RB2 = p.RB2, FB = p.FB;
   const int offX = fx <= G ? -1 : (fx + 1 >= G + RB2 ? 1 : 0);
   const int offY = fy <= G ? -1 : (fy + 1 >= G + RB2 ? 1 : 0);
-  const int cxb = offX > 0 ? bxp : (offX < 0 ? bxm : bx);
-  const int cyb = offY > 0 ? byp : (offY < 0 ? bym : by);
-  const int nbrX = offX ? p.blockSlot[by * p.NBX + cxb] : -1;
-  const int nbrY = offY ? p.blockSlot[cyb * p.NBX + bx] : -1;
-  const int nbrXY = (offX && offY) ? p.blockSlot[cyb * p.NBX + cxb] : -1;
-  const int64_t cell = pcell(p, s, fx, fy);
+  const int nbrX = offX ? nb9[4 + offX] : -1;
+  const int nbrY = offY ? nb9[4 + 3 * offY] : -1;
+  const int nbrXY = (offX && offY) ? nb9[4 + 3 * offY + offX] : -1;
+  g.cell = (unsigned)pcell(p, s, fx, fy);
   const float px = pool_pos(p, bx, fx), py = pool_pos(p, by, fy);
   float wx = fmodf(px, Wf); if (wx < 0.f) wx += Wf;
   float wy = fmodf(py, Hf); if (wy < 0.f) wy += Hf;
   const float rx = wrap_delta(px - p.body.cx, Wf), ry = wrap_delta(py - p.body.cy, Hf);
-  const float usx = p.body.vx - p.body.wz * ry, usy = p.body.vy + p.body.wz * rx;
+  g.usx = p.body.vx - p.body.wz * ry;
+  g.usy = p.body.vy + p.body.wz * rx;
   const float phi = phi2(px, py, p.body, Wf, Hf);
   const bool near = p.bb && phi < 2.0f;  // a link is at most sqrt(2)/2 root cells long here
-  float f[9];
+  g.flags = 0u;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     const int ex = L9::ex(i), ey = L9::ey(i);
-    if (near && phi2(pool_pos(p, bx, fx - ex), pool_pos(p, by, fy - ey), p.body, Wf, Hf) < 0.f) {
-      const float corr = 2.f * L9::w(i) * ((float)ex * usx + (float)ey * usy) * kInvCS2;
-      f[i] = __ldg(fin + L9::opp(i) * p.N1 + cell) + corr;
-      continue;
-    }
+    if (near && phi2(pool_pos(p, bx, fx - ex), pool_pos(p, by, fy - ey), p.body, Wf, Hf) < 0.f) g.flags |= 1u << i;
     int sx = fx - ex, sy = fy - ey, src = s;
     const int ox = (sx < G || sx >= G + RB2) ? offX : 0;
     const int oy = (sy < G || sy >= G + RB2) ? offY : 0;
@@ -380,7 +425,33 @@ __device__ __forceinline__ void substep_cell(const AmrParams &p, const float *__
     if (ns >= 0) { src = ns; sx -= ox * RB2; sy -= oy * RB2; }
     sx = min(max(sx, 0), FB - 1);
     sy = min(max(sy, 0), FB - 1);
-    f[i] = __ldg(fin + i * p.N1 + pcell(p, src, sx, sy));
+    g.src[i] = (unsigned)pcell(p, src, sx, sy);
+  }
+  g.chi = p.bb ? 0.f : chi_from_phi(phi, p.eps_f);
+  const float dx = fminf(wx, Wf - 1.0f - wx), dy = fminf(wy, Hf - 1.0f - wy);
+  g.sw = sponge_weight(fminf(dx, dy), p.sponge_w);
+  if (!(fx >= G && fx < G + RB2 && fy >= G && fy < G + RB2)) g.flags |= kGeoRing;
+  if (phi < 0.f) g.flags |= kGeoSolid;
+  return g;
+}
+
+// One pool substep of one cell: BGK + Guo at tau_f with the chi penalty on
+// this level's band, sponge, SOLID_EQ. Every cell of the tile, ring included,
+// collides (COLLIDE_RING = 1). vel1 NULL: the velocity is not written.
+template <bool CG>
+__device__ __forceinline__ void sub_update(const AmrParams &p, const SubGeo &g, const float *__restrict__ fin,
+                                           float *__restrict__ fout, float2 *__restrict__ vel1) {
+  float f[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    const bool solid = (g.flags >> i) & 1u;
+    f[i] = ldf<CG>(fin + (solid ? L9::opp(i) : i) * p.N1 + (solid ? g.cell : g.src[i]));
+  }
+  if (g.flags & 0x1ffu) {
+#pragma unroll
+    for (int i = 0; i < 9; ++i)
+      if ((g.flags >> i) & 1u)
+        f[i] = __fmaf_rn(2.f * L9::w(i) * ((float)L9::ex(i) * g.usx + (float)L9::ey(i) * g.usy), kInvCS2, f[i]);
   }
   float rho = 0.f, uxs = 0.f, uys = 0.f;
 #pragma unroll
@@ -392,28 +463,26 @@ __device__ __forceinline__ void substep_cell(const AmrParams &p, const float *__
   const float den = fmaxf(rho, 1e-6f);
   uxs /= den;
   uys /= den;
-  const float chi = p.bb ? 0.f : chi_from_phi(phi, p.eps_f);
-  const float Fx = rho * chi * (usx - uxs) + p.fx;
-  const float Fy = rho * chi * (usy - uys) + p.fy;
+  const float Fx = rho * g.chi * (g.usx - uxs) + p.fx;
+  const float Fy = rho * g.chi * (g.usy - uys) + p.fy;
   const float ux = uxs + Fx / (2.0f * den), uy = uys + Fy / (2.0f * den);
   const float usq = ux * ux + uy * uy;
-  vel1[cell] = make_float2(ux, uy);
-  if (p.explode && !(fx >= G && fx < G + RB2 && fy >= G && fy < G + RB2)) {
+  if (vel1) vel1[g.cell] = make_float2(ux, uy);
+  if (p.explode && (g.flags & kGeoRing)) {
     // explode/coalesce: the ring advects without colliding (COLLIDE_RING = 0)
 #pragma unroll
-    for (int i = 0; i < 9; ++i) fout[i * p.N1 + cell] = f[i];
+    for (int i = 0; i < 9; ++i) fout[i * p.N1 + g.cell] = f[i];
     return;
   }
-  const float dx = fminf(wx, Wf - 1.0f - wx), dy = fminf(wy, Hf - 1.0f - wy);
-  const float sw = sponge_weight(fminf(dx, dy), p.sponge_w);
-  const bool solid = p.solid_eq && p.bb && phi < 0.f;
+  const float sw = g.sw;
+  const bool solid = p.solid_eq && p.bb && (g.flags & kGeoSolid);
   const float omg = p.omega_f, sfac = 1.0f - 0.5f * omg;
 #pragma unroll
   for (int i = 0; i < 9; ++i) {
     const float exf = (float)L9::ex(i), eyf = (float)L9::ey(i), w = L9::w(i);
     float o;
     if (solid) {
-      o = feq9(1.0f, usx, usy, i);
+      o = feq9(1.0f, g.usx, g.usy, i);
     } else {
       const float eu = exf * ux + eyf * uy;
       const float fe = w * rho * (1.f + 3.f * eu + 4.5f * eu * eu - 1.5f * usq);
@@ -422,25 +491,31 @@ __device__ __forceinline__ void substep_cell(const AmrParams &p, const float *__
       const float fc = f[i] - omg * (f[i] - fe) + Si;
       o = fc * (1.0f - sw) + p.ftarget[i] * sw;
     }
-    fout[i * p.N1 + cell] = o;
+    fout[i * p.N1 + g.cell] = o;
   }
 }
 
 __global__ void __launch_bounds__(kChunk)
     amr_substep(const float *__restrict__ fin, float *__restrict__ fout, float2 *__restrict__ vel1,
                 const __grid_constant__ AmrParams p) {
+  __shared__ int nb9[9];
   const int n = p.counts[1];
   const int FB2 = p.FB * p.FB, nch = (FB2 + kChunk - 1) / kChunk;
   for (int w = blockIdx.x; w < n * nch; w += gridDim.x) {
     const int k = w / nch, c0 = (w % nch) * kChunk, c1 = min(c0 + kChunk, FB2);
     const int s = p.activeList[k];
     const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-    for (int c = c0 + threadIdx.x; c < c1; c += kChunk) substep_cell(p, fin, fout, vel1, s, bx, by, c % p.FB, c / p.FB);
+    __syncthreads();
+    load_nb9(p, bx, by, nb9);
+    __syncthreads();
+    for (int c = c0 + threadIdx.x; c < c1; c += kChunk)
+      sub_update<false>(p, sub_geo(p, nb9, s, bx, by, c % p.FB, c / p.FB), fin, fout, vel1);
   }
 }
 
 // 4-child restriction into the root (common_average.wgsl averageCell): root
 // cell c (of RB x RB) of tile s's block.
+template <bool CG>
 __device__ __forceinline__ void average_cell(const AmrParams &p, const float *__restrict__ f1, float *__restrict__ f0,
                                              int s, int bx, int by, int c) {
   const int lx = c % p.RB, ly = c / p.RB;
@@ -456,7 +531,7 @@ __device__ __forceinline__ void average_cell(const AmrParams &p, const float *__
     float f[9], rho = 0.f, ux = 0.f, uy = 0.f;
 #pragma unroll
     for (int i = 0; i < 9; ++i) {
-      f[i] = __ldg(f1 + i * p.N1 + ch[q]);
+      f[i] = ldf<CG>(f1 + i * p.N1 + ch[q]);
       rho += f[i];
       ux += f[i] * (float)L9::ex(i);
       uy += f[i] * (float)L9::ey(i);
@@ -482,13 +557,15 @@ __global__ void __launch_bounds__(64)
   for (int k = blockIdx.x; k < n; k += gridDim.x) {
     const int s = p.activeList[k];
     const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-    for (int c = threadIdx.x; c < p.RB * p.RB; c += 64) average_cell(p, f1, f0, s, bx, by, c);
+    for (int c = threadIdx.x; c < p.RB * p.RB; c += 64) average_cell<false>(p, f1, f0, s, bx, by, c);
   }
 }
 
 // Finest-level force (amr_force1.wgsl forceCell): this thread's share of
-// the interior cells of tile s (cells threadIdx.x, + kPoolThreads, ...),
-// momentum exchange or penalty weighted by dx = 1/2.
+// the interior cells of tile s (cells threadIdx.x, + kPoolThreads, ...; none
+// from thread kPoolThreads on), momentum exchange or penalty weighted by
+// dx = 1/2.
+template <bool CG>
 __device__ __forceinline__ void force_tile_acc(const AmrParams &p, const float *__restrict__ f1, int s, int bx, int by,
                                                ForceAcc &acc) {
   const float Wf = (float)p.W, Hf = (float)p.H;
@@ -506,7 +583,7 @@ __device__ __forceinline__ void force_tile_acc(const AmrParams &p, const float *
         for (int i = 0; i < 9; ++i) {
           const int ex = L9::ex(i), ey = L9::ey(i);
           if (phi2(pool_pos(p, bx, fx - ex), pool_pos(p, by, fy - ey), p.body, Wf, Hf) < 0.f) {
-            const float fo = __ldg(f1 + L9::opp(i) * p.N1 + cell);
+            const float fo = ldf<CG>(f1 + L9::opp(i) * p.N1 + cell);
             const float corr = 2.f * L9::w(i) * ((float)ex * usx + (float)ey * usy) * kInvCS2;
             fxb += -(float)ex * (2.f * fo + corr) * 0.5f;
             fyb += -(float)ey * (2.f * fo + corr) * 0.5f;
@@ -532,7 +609,7 @@ __device__ __forceinline__ void force_tile_acc(const AmrParams &p, const float *
               if (ns >= 0) src = pcell(p, ns, sx0 - ox * p.RB2, sy0 - oy * p.RB2);
             }
           }
-          const float v = __ldg(f1 + i * p.N1 + src);
+          const float v = ldf<CG>(f1 + i * p.N1 + src);
           rho += v;
           ux += v * (float)L9::ex(i);
           uy += v * (float)L9::ey(i);
@@ -553,6 +630,17 @@ __device__ __forceinline__ void force_tile_acc(const AmrParams &p, const float *
   }
 }
 
+// Whether any of this thread's cells in force_tile_acc can add to the force.
+__device__ __forceinline__ bool force_tile_near(const AmrParams &p, int bx, int by) {
+  bool any = false;
+  for (int c = threadIdx.x; c < p.RB2 * p.RB2; c += kPoolThreads) {
+    const float phi = phi2(pool_pos(p, bx, p.G + c % p.RB2), pool_pos(p, by, p.G + c / p.RB2), p.body, (float)p.W,
+                           (float)p.H);
+    any = any || (p.bb ? phi >= 0.f && phi < 2.0f : chi_from_phi(phi, p.eps_f) >= 1e-6f);
+  }
+  return any;
+}
+
 // The force of every active tile: one FP64 partial per tile and a
 // deterministic last-block sum.
 __global__ void __launch_bounds__(kPoolThreads)
@@ -566,161 +654,275 @@ __global__ void __launch_bounds__(kPoolThreads)
     const int s = p.activeList[k];
     const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
     ForceAcc acc;
-    force_tile_acc(p, f1, s, bx, by, acc);
+    force_tile_acc<false>(p, f1, s, bx, by, acc);
     reduce_force<kPoolThreads>(acc, p.partials, p.counter, n, k, p.force_out);
     __syncthreads();
   }
 }
 
-// ---- the interp macro-step as one cooperative launch -----------------------
-// The six launches of a macro-step (force, ring fill, root step, two
-// substeps, restriction) are latency-bound: 64 tiles are 25,600 pool cells,
-// and each launch mostly waits on a chain of dependent loads and on its own
-// start and drain. Here one launch of resident blocks runs them as phases
-// separated by grid barriers:
-//   0  force partials of every tile | ring fill | root step   (independent)
-//   1  force sum (block 0) | substep a -> b
-//   2  substep b -> a
-//   3  restriction into the root
-// Every cell goes through the same device function as in the separate
-// kernels (fill_ring_cell, cell2, substep_cell, average_cell,
+// ---- interp macro-steps in one cooperative launch ---------------------------
+// A macro-step on a few dozen tiles is latency: 64 tiles are 25,600 pool
+// cells and the root's populations stay in L2, while each of the six kernels
+// (force, ring fill, root step, two substeps, restriction) waits on its own
+// start, a chain of dependent loads and its drain. One launch of resident
+// blocks runs all macro-steps up to the next refine round instead, each as
+// three phases between grid barriers:
+//   0  force partials and ring fill of the block's tiles | root step, part 1
+//   1  substep a -> b of its tiles | force sum | root step, part 2
+//   2  substep b -> a of its tiles, then their restriction into the root
+// Block b owns tiles b, b + grid, ... throughout (their neighbour slots are
+// looked up once), so the restriction follows its tile's substep without a
+// grid barrier; the root is stepped by the blocks without tiles when those
+// are at least half. Within a macro-step every phase reads only what the
+// barrier before it completed.
+// Every cell goes through the same device functions as in the separate
+// kernels (ring_geo, fill_cell, cell2_core, sub_geo, sub_update, average_cell,
 // force_tile_acc, the same block tree and fixed-order partial sum), so the
-// result is theirs to the bit. 256-thread blocks: the force tree must see
-// amr_force's thread mapping.
+// result is theirs to the bit. The root's mac and the pool's velocity, which
+// each macro-step overwrites, are written by the launch's last one.
+// All populations are read from L2 (ldf<true>): other blocks of the launch
+// write them.
+// Bound by latency: three barriers and three chains of dependent L2 loads a
+// macro-step. 1024x256 root, per macro-step with the refine
+// rounds: 38.8 us as one launch per macro-step with five phases and the
+// geometry worked out in each, 20.3 us in this form (the same with one block
+// per SM).
+
+constexpr int kMacroThreads = 512;
+constexpr int kKeptRing = 256;
+constexpr int kMacroSteps = 32;  // macro-steps of one launch at most
 
 struct MacroArgs {
-  const float *f0in;
-  float *f0out;
+  float *f0[2];  // root buffers: the first macro-step reads f0[0]
   float *mac;
   float *f1a, *f1b;
   float2 *vel1;
-  unsigned *bar;  // arrivals, generation
+  unsigned *bar;  // arrivals, zero at launch
   int *bar_err;
-  unsigned nblocks;
+  int steps;
 };
 
-// About a second of polling (2^22 waits of ~256 ns) before a barrier gives
-// up, flags the error and lets its block go on: the launch then ends (its
-// result void, reported by lbm_amr2d_sync as LBM_ETIMEDOUT) instead of
-// holding the GPU. A cooperative launch has every block resident, so a
-// healthy barrier releases within microseconds.
-constexpr unsigned long long kBarrierSpins = 1ull << 22;
+// About a second of polling before a barrier gives up, flags the error and
+// its block leaves; every other block then leaves at its next poll. The
+// launch then ends (its result void, reported by lbm_amr2d_sync as
+// LBM_ETIMEDOUT) instead of holding the GPU. A cooperative launch has every
+// block resident, so a healthy barrier releases within microseconds.
+constexpr unsigned kBarrierSpins = 1u << 21;
 
-__device__ __forceinline__ void grid_barrier(unsigned *bar, int *err, unsigned nblocks) {
+// Waits until every block has arrived `round` times; false after a timeout.
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, int *err, unsigned round, int *ok) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned *gen = bar + 1;
-    const unsigned g = *gen;
+    *ok = 1;
+    const unsigned target = round * gridDim.x;
     __threadfence();
-    if (atomicAdd(bar, 1u) == nblocks - 1) {
-      atomicExch(bar, 0u);  // re-armed before the release
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      unsigned long long spins = 0;
-      while (*gen == g) {
-        if (++spins > kBarrierSpins) {
-          atomicExch(err, 1);
-          break;
-        }
-        __nanosleep(256);
+    atomicAdd(bar, 1u);
+    unsigned spins = 0, seen;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+      if ((int)(seen - target) >= 0) break;
+      if (++spins > kBarrierSpins || (spins % 1024u == 0u && *(volatile int *)err)) {
+        atomicExch(err, 1);
+        *ok = 0;
+        break;
       }
     }
     __threadfence();
   }
   __syncthreads();
+  return *ok != 0;
 }
 
-__global__ void __launch_bounds__(kPoolThreads)
-    amr_macro_fused(const __grid_constant__ AmrParams p, const __grid_constant__ StepParams rp,
-                    const __grid_constant__ MacroArgs m) {
-  __shared__ double sm[kForceSlots * (kPoolThreads / 32)];
-  const int n = p.counts[1];
-  const int FB = p.FB, FB2 = FB * FB, nch = (FB2 + kPoolThreads - 1) / kPoolThreads;
-  const int nroot = (int)((p.N0 + kPoolThreads - 1) / kPoolThreads);
-  // 0: force partials (time t, pool), ring fill (from the root at t), root step
-  for (int w = blockIdx.x; w < n + n * nch + nroot; w += gridDim.x) {
-    if (w < n) {
-      const int s = p.activeList[w];
-      const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
+// Ring cell r of a tile as (fx, fy): the two rows below the interior, the two
+// cells on either side of each interior row, the two rows above.
+__device__ __forceinline__ void ring_cell(const AmrParams &p, int r, int &fx, int &fy) {
+  const int FB = p.FB, G = p.G, low = G * FB, mid = p.RB2 * 2 * G;
+  if (r < low) {
+    fy = r / FB;
+    fx = r - fy * FB;
+  } else if (r < low + mid) {
+    const int q = r - low, w = q % (2 * G);
+    fy = G + q / (2 * G);
+    fx = w < G ? w : w + p.RB2;
+  } else {
+    const int q = r - low - mid;
+    fy = G + p.RB2 + q / FB;
+    fx = q % FB;
+  }
+}
+
+__global__ void __launch_bounds__(kMacroThreads, 2)
+    amr_macro_loop(const __grid_constant__ AmrParams p, const __grid_constant__ StepParams rp,
+                   const __grid_constant__ MacroArgs m) {
+  __shared__ double sm[kForceSlots * (kMacroThreads / 32)];
+  __shared__ int nb9[9];
+  __shared__ int ok;
+  const int n = p.counts[1], tid = threadIdx.x, G = (int)gridDim.x;
+  const int FB = p.FB, FB2 = FB * FB, nring = FB2 - p.RB2 * p.RB2, RR = p.RB * p.RB;
+  // the block's first tile: its slot, block and neighbours for all steps
+  int s = 0, bx = 0, by = 0;
+  auto tile = [&](int k) {
+    s = p.activeList[k];
+    const int bid = p.slotToBlock[s];
+    by = bid / p.NBX;
+    bx = bid - by * p.NBX;
+    __syncthreads();
+    load_nb9(p, bx, by, nb9);
+    __syncthreads();
+  };
+  const bool many = n > G;  // more tiles than blocks: looked up per phase
+  // With one tile per block whose cells fit its threads, what the tile's cells
+  // need beyond populations (SubGeo, FillGeo: the body's distance, tanh,
+  // modulo and divisions) is worked out once per launch.
+  const bool kept = !many && FB2 <= kMacroThreads && nring <= kKeptRing;
+  __shared__ unsigned g_src[9][kMacroThreads], g_flags[kMacroThreads], r_src[4][kKeptRing];
+  __shared__ float g_f[4][kMacroThreads], r_t[2][kKeptRing];
+  __shared__ unsigned char r_copy[kKeptRing];
+  bool force = true;  // whether this thread's force cells can feel the body
+  if (!many && (int)blockIdx.x < n) {
+    tile(blockIdx.x);
+    if (kept && tid < FB2) {
+      const SubGeo g = sub_geo(p, nb9, s, bx, by, tid % FB, tid / FB);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) g_src[i][tid] = g.src[i];
+      g_flags[tid] = g.flags;
+      g_f[0][tid] = g.usx;
+      g_f[1][tid] = g.usy;
+      g_f[2][tid] = g.chi;
+      g_f[3][tid] = g.sw;
+    }
+    if (kept && tid < nring) {
+      int fx, fy;
+      ring_cell(p, tid, fx, fy);
+      const FillGeo g = ring_geo(p, nb9, s, bx, by, fx, fy);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r_src[k][tid] = g.src[k];
+      r_t[0][tid] = g.tx;
+      r_t[1][tid] = g.ty;
+      r_copy[tid] = g.copy;
+    }
+    if (kept) force = force_tile_near(p, bx, by);
+  }
+  // (each thread reads back what it wrote)
+  auto substep = [&](const float *fin, float *fout, float2 *vel1) {
+    if (kept) {
+      if (tid >= FB2) return;
+      SubGeo g;
+      g.cell = (unsigned)((int64_t)s * FB2 + tid);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) g.src[i] = g_src[i][tid];
+      g.flags = g_flags[tid];
+      g.usx = g_f[0][tid];
+      g.usy = g_f[1][tid];
+      g.chi = g_f[2][tid];
+      g.sw = g_f[3][tid];
+      sub_update<true>(p, g, fin, fout, vel1);
+      return;
+    }
+    for (int c = tid; c < FB2; c += kMacroThreads)
+      sub_update<true>(p, sub_geo(p, nb9, s, bx, by, c % FB, c / FB), fin, fout, vel1);
+  };
+  // the root's cells over the blocks without tiles, or over all of them
+  const int w0 = 2 * n <= G ? n : 0, workers = G - w0, me = (int)blockIdx.x - w0;
+  const int half = (int)(p.N0 / 2);
+  auto root = [&](const float *f0in, float *f0out, float *mac, int c0, int c1) {
+    if (me < 0) return;
+    for (int c = c0 + me * kMacroThreads + tid; c < c1; c += workers * kMacroThreads) {
+      const int y = c / p.W, x = c - y * p.W;
+      CellForce cf;
+      cell2<CgFloat>((const CgFloat *)f0in, (CgFloat *)f0out, mac, rp, x, y, false, cf);
+    }
+  };
+  unsigned round = 0;
+  for (int step = 0; step < m.steps; ++step) {
+    const float *f0in = m.f0[step & 1];
+    float *f0out = m.f0[1 - (step & 1)];
+    const bool last = step == m.steps - 1;
+    float *mac = last ? m.mac : nullptr;
+    for (int k = blockIdx.x; k < n; k += G) {
+      if (many) tile(k);
+      // the force first: the penalty's gather reads the ring cells that the
+      // fill overwrites. The tree of kPoolThreads threads (the others add
+      // zeros), or zeros directly where no cell contributes.
       ForceAcc acc;
-      force_tile_acc(p, m.f1a, s, bx, by, acc);
-      double v[kForceSlots];
+      if (tid < kPoolThreads && force) force_tile_acc<true>(p, m.f1a, s, bx, by, acc);
+      const bool mine = acc.v[0] != 0.0 || acc.v[1] != 0.0 || acc.v[5] != 0.0 || acc.bad != 0.0;
+      double *part = p.partials + (int64_t)k * kForceSlots;
+      if (__syncthreads_or(mine)) {
+        double v[kForceSlots];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) v[k] = acc.v[k];
-      v[6] = acc.bad;
-      v[7] = 0.0;
-      block_sum<kForceSlots, kPoolThreads>(v, sm);
-      if (threadIdx.x == 0)
+        for (int j = 0; j < 6; ++j) v[j] = acc.v[j];
+        v[6] = acc.bad;
+        v[7] = 0.0;
+        block_sum<kForceSlots, kMacroThreads>(v, sm);
+        if (tid == 0)
 #pragma unroll
-        for (int k = 0; k < kForceSlots; ++k) p.partials[(int64_t)w * kForceSlots + k] = v[k];
+          for (int j = 0; j < kForceSlots; ++j) part[j] = v[j];
+      } else if (tid < kForceSlots) {
+        part[tid] = 0.0;
+      }
+      for (int r = tid; r < nring; r += kMacroThreads) {
+        int fx, fy;
+        ring_cell(p, r, fx, fy);
+        FillGeo g;
+        if (kept) {
+          g.cell = (unsigned)pcell(p, s, fx, fy);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) g.src[j] = r_src[j][r];
+          g.tx = r_t[0][r];
+          g.ty = r_t[1][r];
+          g.copy = r_copy[r];
+        } else {
+          g = ring_geo(p, nb9, s, bx, by, fx, fy);
+        }
+        fill_cell<true>(p, g, f0in, m.f1a);
+      }
+    }
+    root(f0in, f0out, mac, 0, half);
+    if (!grid_barrier(m.bar, m.bar_err, ++round, &ok)) return;
+    if ((int)blockIdx.x == G - 1) {
+      if (n == 0) {
+        if (tid < 4) p.force_out[tid] = 0.0;
+      } else if (tid < 32) {
+        sum_partials_warp<kForceSlots>(p.partials, n, p.force_out);
+      }
+    }
+    for (int k = blockIdx.x; k < n; k += G) {
+      if (many) tile(k);
+      substep(m.f1a, m.f1b, nullptr);
+    }
+    root(f0in, f0out, mac, half, (int)p.N0);
+    if (!grid_barrier(m.bar, m.bar_err, ++round, &ok)) return;
+    for (int k = blockIdx.x; k < n; k += G) {
+      if (many) tile(k);
+      substep(m.f1b, m.f1a, last ? m.vel1 : nullptr);
       __syncthreads();
-    } else if (w < n + n * nch) {
-      const int k = (w - n) / nch, c = ((w - n) % nch) * kPoolThreads + threadIdx.x;
-      if (c < FB2) {
-        const int s = p.activeList[k];
-        const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-        const int fx = c % FB, fy = c / FB;
-        const bool inX = fx >= p.G && fx < p.G + p.RB2, inY = fy >= p.G && fy < p.G + p.RB2;
-        if (!(inX && inY)) fill_ring_cell(p, m.f0in, m.f1a, s, bx, by, fx, fy);
-      }
-    } else {
-      const int c = (w - n - n * nch) * kPoolThreads + threadIdx.x;
-      if (c < p.N0) {
-        CellForce cf;
-        cell2<float>(m.f0in, m.f0out, m.mac, rp, c % p.W, c / p.W, false, cf);
-      }
+      for (int c = tid; c < RR; c += kMacroThreads) average_cell<true>(p, m.f1a, f0out, s, bx, by, c);
     }
-  }
-  grid_barrier(m.bar, m.bar_err, m.nblocks);
-  // 1: the force of this macro-step, and substep a -> b
-  if (blockIdx.x == 0) {
-    if (n == 0) {
-      if (threadIdx.x < 4) p.force_out[threadIdx.x] = 0.0;
-    } else if (threadIdx.x < 32) {
-      sum_partials_warp<kForceSlots>(p.partials, n, p.force_out);
-    }
-  }
-  for (int w = blockIdx.x; w < n * nch; w += gridDim.x) {
-    const int k = w / nch, c = (w % nch) * kPoolThreads + threadIdx.x;
-    if (c >= FB2) continue;
-    const int s = p.activeList[k];
-    const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-    substep_cell(p, m.f1a, m.f1b, m.vel1, s, bx, by, c % FB, c / FB);
-  }
-  grid_barrier(m.bar, m.bar_err, m.nblocks);
-  // 2: substep b -> a
-  for (int w = blockIdx.x; w < n * nch; w += gridDim.x) {
-    const int k = w / nch, c = (w % nch) * kPoolThreads + threadIdx.x;
-    if (c >= FB2) continue;
-    const int s = p.activeList[k];
-    const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-    substep_cell(p, m.f1b, m.f1a, m.vel1, s, bx, by, c % FB, c / FB);
-  }
-  grid_barrier(m.bar, m.bar_err, m.nblocks);
-  // 3: restriction of the pool into the root at t + 1
-  const int RR = p.RB * p.RB, nrr = (RR + kPoolThreads - 1) / kPoolThreads;
-  for (int w = blockIdx.x; w < n * nrr; w += gridDim.x) {
-    const int k = w / nrr, c = (w % nrr) * kPoolThreads + threadIdx.x;
-    if (c >= RR) continue;
-    const int s = p.activeList[k];
-    const int bid = p.slotToBlock[s], bx = bid % p.NBX, by = bid / p.NBX;
-    average_cell(p, m.f1a, m.f0out, s, bx, by, c);
+    if (!last && !grid_barrier(m.bar, m.bar_err, ++round, &ok)) return;
   }
 }
 
-// Blocks of the fused macro-step's cooperative launch on the current device
-// (every one resident), or 0 where it cannot run: the explode interface, or
-// a device without cooperative launches.
+// Blocks of the fused macro-steps' cooperative launch on the current device
+// (every one resident, two per SM at most), or 0 where it cannot run: the
+// explode interface, or a device without cooperative launches.
 int fused_blocks(const AmrParams &p) {
   int dev = 0, sms = 0, coop = 0, per_sm = 0;
   if (p.explode || cudaGetDevice(&dev) != cudaSuccess) return 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  const bool ok = coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, amr_macro_fused, kPoolThreads, 0) ==
+  const bool ok = coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, amr_macro_loop, kMacroThreads, 0) ==
                               cudaSuccess;
   cudaGetLastError();
-  return ok ? per_sm * sms : 0;
+  return ok ? std::min(per_sm, 2) * sms : 0;
+}
+
+// (ux, uy) of the root's mac, for the host (half the bytes, and no pass over
+// them there).
+__global__ void __launch_bounds__(256)
+    root_velocity(const float4 *__restrict__ mac, float2 *__restrict__ vel, int64_t n) {
+  const int64_t c = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (c < n) vel[c] = make_float2(mac[c].y, mac[c].z);
 }
 
 // ---- explode / coalesce interface ------------------------------------------------
@@ -860,7 +1062,7 @@ struct lbm_amr2d {
   float *f0[2] = {nullptr, nullptr};
   float4 *mac = nullptr;
   float *f1[2] = {nullptr, nullptr};
-  float2 *vel1 = nullptr;
+  float2 *vel1 = nullptr, *vel0 = nullptr;
   int cur = 0;
   int64_t step = 0;
   cudaStream_t own = nullptr, stream = nullptr;
@@ -868,7 +1070,7 @@ struct lbm_amr2d {
   double *host = nullptr;
   int *host_counts = nullptr;
   int grid_slots = 0;
-  // the fused macro-step: resident blocks of one cooperative launch (0: off)
+  // the fused macro-steps: resident blocks of one cooperative launch (0: off)
   // and its grid barrier's state and timeout flag
   int fused_grid = 0;
   unsigned *bar = nullptr;
@@ -899,7 +1101,7 @@ void release_amr(lbm_amr2d *a) {
   for (auto &g : a->graph)
     if (g) cudaGraphExecDestroy(g);
   cudaFree(a->f0[0]); cudaFree(a->f0[1]); cudaFree(a->mac);
-  cudaFree(a->f1[0]); cudaFree(a->f1[1]); cudaFree(a->vel1);
+  cudaFree(a->f1[0]); cudaFree(a->f1[1]); cudaFree(a->vel1); cudaFree(a->vel0);
   AmrParams &p = a->p;
   cudaFree(p.blockSlot); cudaFree(p.slotToBlock); cudaFree(p.parentSlot); cudaFree(p.freeList);
   cudaFree(p.counts); cudaFree(p.activeList); cudaFree(p.want); cudaFree(p.newly); cudaFree(p.crit);
@@ -933,6 +1135,15 @@ int validate_amr(const lbm_amr2d_config *c, std::string &why) {
   return LBM_OK;
 }
 
+// The root level is a dense D2Q9 domain stepped by the dense kernel's update.
+void root_config(const lbm_amr2d_config &c, lbm_config &rc) {
+  lbm_config_default(&rc, 9, c.nx, c.ny, 1);
+  rc.tau = c.tau; rc.force[0] = c.force[0]; rc.force[1] = c.force[1];
+  rc.has_body = 1; rc.use_bounceback = c.use_bounceback; rc.solid_eq = c.solid_eq; rc.chi_eps = c.k_eps;
+  rc.sponge_w = c.sponge_w; rc.sponge_u[0] = c.sponge_u[0]; rc.sponge_u[1] = c.sponge_u[1];
+  rc.body = c.body;
+}
+
 int macro_launches(lbm_amr2d *a, cudaStream_t st, int from) {
   AmrParams &p = a->p;
   const int g = a->grid_slots;
@@ -951,23 +1162,6 @@ int macro_launches(lbm_amr2d *a, cudaStream_t st, int from) {
     ACK(a, cudaGetLastError());
     return LBM_OK;
   }
-  if (a->fused_grid > 0) {
-    StepParams rp = a->root;
-    rp.write_mac = 1;
-    const MacroArgs m{a->f0[from], a->f0[1 - from], (float *)a->mac, a->f1[0], a->f1[1], a->vel1, a->bar,
-                      a->bar_err, (unsigned)a->fused_grid};
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(a->fused_grid);
-    lc.blockDim = dim3(kPoolThreads);
-    lc.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    ACK(a, cudaLaunchKernelEx(&lc, amr_macro_fused, p, rp, m));
-    return LBM_OK;
-  }
   amr_force<<<g, kPoolThreads, 0, st>>>(a->f1[0], p);
   amr_fill<<<g, kChunk, 0, st>>>(a->f0[from], a->f1[0], 0, p);
   StepParams rp = a->root;
@@ -981,15 +1175,34 @@ int macro_launches(lbm_amr2d *a, cudaStream_t st, int from) {
   return LBM_OK;
 }
 
+// k fused macro-steps from the current buffer.
+int macro_loop(lbm_amr2d *a, int k) {
+  StepParams rp = a->root;
+  rp.write_mac = 1;
+  const MacroArgs m{{a->f0[a->cur], a->f0[1 - a->cur]}, (float *)a->mac, a->f1[0], a->f1[1], a->vel1, a->bar,
+                    a->bar_err, k};
+  ACK(a, cudaMemsetAsync(a->bar, 0, sizeof(unsigned), a->stream));
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(a->fused_grid);
+  lc.blockDim = dim3(kMacroThreads);
+  lc.stream = a->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  ACK(a, cudaLaunchKernelEx(&lc, amr_macro_loop, a->p, rp, m));
+  return LBM_OK;
+}
+
 int refine_round(lbm_amr2d *a) {
   AmrParams &p = a->p;
   cudaStream_t st = a->stream;
-  ACK(a, cudaMemsetAsync(p.newly, 0, p.S * sizeof(unsigned), st));
-  amr_criterion<<<p.NBX * p.NBY, 64, 0, st>>>(a->mac, p);
-  ACK(a, cudaMemsetAsync(p.want, 0, (size_t)p.NBX * p.NBY * sizeof(unsigned), st));
-  amr_decide<<<(p.PNX * p.PNY + 127) / 128, 128, 0, st>>>(p);
-  amr_coarsen_refine<<<1, kManageThreads, 0, st>>>(p);
-  amr_fill<<<a->grid_slots, kChunk, 0, st>>>(a->f0[a->cur], a->f1[0], 1, p);
+  // (decide writes every want flag)
+  launch_pdl(dim3(p.NBX * p.NBY), dim3(64), st, amr_criterion, (const float4 *)a->mac, p);
+  launch_pdl(dim3((p.PNX * p.PNY + 127) / 128), dim3(128), st, amr_decide, p);
+  launch_pdl(dim3(1), dim3(kManageThreads), st, amr_coarsen_refine, p);
+  launch_pdl(dim3(a->grid_slots), dim3(kChunk), st, amr_fill, (const float *)a->f0[a->cur], a->f1[0], 1, p);
   ACK(a, cudaGetLastError());
   return LBM_OK;
 }
@@ -1006,12 +1219,6 @@ int build_graph(lbm_amr2d *a, int from) {
   if (e == cudaSuccess && rc == LBM_OK) e = cudaGraphInstantiate(&a->graph[from], g, 0);
   if (g) cudaGraphDestroy(g);
   cudaStreamDestroy(cs);
-  if ((rc || e != cudaSuccess) && a->fused_grid > 0) {
-    // a cooperative kernel node this driver will not capture: the six launches
-    cudaGetLastError();
-    a->fused_grid = 0;
-    return build_graph(a, from);
-  }
   if (rc) return rc;
   if (e != cudaSuccess) return afail(a, LBM_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
   return LBM_OK;
@@ -1077,15 +1284,10 @@ int lbm_amr2d_create(const lbm_amr2d_config *cfg, lbm_amr2d **out) {
     const float eu = (float)ex * p.sux + (float)ey * p.suy;
     p.ftarget[i] = Lattice<9>::w(i) * (1.0f + 3.0f * eu + 4.5f * eu * eu - 1.5f * (p.sux * p.sux + p.suy * p.suy));
   }
-  // The root level is a dense D2Q9 domain stepped by the dense kernel.
   lbm_config rc;
-  lbm_config_default(&rc, 9, c.nx, c.ny, 1);
-  rc.tau = c.tau; rc.force[0] = c.force[0]; rc.force[1] = c.force[1];
-  rc.has_body = 1; rc.use_bounceback = c.use_bounceback; rc.solid_eq = c.solid_eq; rc.chi_eps = c.k_eps;
-  rc.sponge_w = c.sponge_w; rc.sponge_u[0] = c.sponge_u[0]; rc.sponge_u[1] = c.sponge_u[1];
-  rc.body = c.body;
+  root_config(c, rc);
   fill_step_params(rc, p.N0, 0, a->root);
-  a->root.force_on = 0;  // the body force is measured on the finest level
+  set_body_regions(rc, a->root, false);  // the body force is measured on the finest level
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1101,7 +1303,7 @@ int lbm_amr2d_create(const lbm_amr2d_config *cfg, lbm_amr2d **out) {
   if ((e = cudaStreamCreateWithFlags(&a->own, cudaStreamNonBlocking))) return bail(e, "stream");
   a->stream = a->own;
   AM(a->f0[0], 9 * p.N0 * 4); AM(a->f0[1], 9 * p.N0 * 4); AM(a->mac, p.N0 * 16);
-  AM(a->f1[0], 9 * p.N1 * 4); AM(a->f1[1], 9 * p.N1 * 4); AM(a->vel1, p.N1 * 8);
+  AM(a->f1[0], 9 * p.N1 * 4); AM(a->f1[1], 9 * p.N1 * 4); AM(a->vel1, p.N1 * 8); AM(a->vel0, p.N0 * 8);
   AM(p.blockSlot, p.NBX * p.NBY * 4); AM(p.slotToBlock, p.S * 4); AM(p.parentSlot, p.S * 4);
   AM(p.freeList, (p.S / 4) * 4); AM(p.counts, 2 * 4); AM(p.activeList, p.S * 4);
   AM(p.want, p.NBX * p.NBY * 4); AM(p.newly, p.S * 4); AM(p.crit, p.NBX * p.NBY * 4);
@@ -1164,14 +1366,12 @@ int lbm_amr2d_read_root(lbm_amr2d *a, float *f, float *vel) {
   if (!a) return LBM_EINVAL;
   const AmrParams &p = a->p;
   if (f) ACK(a, cudaMemcpyAsync(f, a->f0[a->cur], 9 * p.N0 * 4, cudaMemcpyDeviceToHost, a->stream));
-  std::vector<float4> m;
   if (vel) {
-    m.resize(p.N0);
-    ACK(a, cudaMemcpyAsync(m.data(), a->mac, p.N0 * 16, cudaMemcpyDeviceToHost, a->stream));
+    root_velocity<<<(int)((p.N0 + 255) / 256), 256, 0, a->stream>>>(a->mac, a->vel0, p.N0);
+    ACK(a, cudaGetLastError());
+    ACK(a, cudaMemcpyAsync(vel, a->vel0, p.N0 * 8, cudaMemcpyDeviceToHost, a->stream));
   }
   ACK(a, cudaStreamSynchronize(a->stream));
-  if (vel)
-    for (int64_t k = 0; k < p.N0; ++k) { vel[2 * k] = m[k].y; vel[2 * k + 1] = m[k].z; }
   return LBM_OK;
 }
 
@@ -1187,11 +1387,24 @@ int lbm_amr2d_read_pool(lbm_amr2d *a, float *f, float *vel) {
 int lbm_amr2d_step(lbm_amr2d *a, int n) {
   if (!a) return LBM_EINVAL;
   if (n < 0) return afail(a, LBM_EINVAL, "step count must be >= 0");
-  for (int k = 0; k < n; ++k) {
-    if (a->cfg.auto_refine && a->step % a->cfg.refine_every == 0) {
+  for (int k = 0; k < n;) {
+    const int64_t every = a->cfg.refine_every;
+    if (a->cfg.auto_refine && a->step % every == 0) {
       int rc = refine_round(a);
       if (rc) return rc;
     }
+    if (a->fused_grid > 0) {
+      // up to the next refine round
+      int64_t run = std::min<int64_t>(n - k, kMacroSteps);
+      if (a->cfg.auto_refine) run = std::min(run, every - a->step % every);
+      int rc = macro_loop(a, (int)run);
+      if (rc) return rc;
+      a->step += run;
+      a->cur = (a->cur + (int)run) & 1;
+      k += (int)run;
+      continue;
+    }
+    ++k;
     ++a->step;
     if (!a->graph[a->cur]) {
       int rc = build_graph(a, a->cur);
@@ -1350,6 +1563,11 @@ int lbm_amr2d_set_body(lbm_amr2d *a, const lbm_body *body) {
   a->cfg.body = *body;
   a->p.body = *body;
   a->root.body = *body;
+  {
+    lbm_config rc;
+    root_config(a->cfg, rc);
+    set_body_regions(rc, a->root, false);
+  }
   for (auto &g : a->graph)
     if (g) { cudaGraphExecDestroy(g); g = nullptr; }
   return LBM_OK;

@@ -7,7 +7,9 @@ or topology selects, a cell gets the same bits.
 * the D2Q9 reach box, against the batch, which evaluates the body everywhere;
 * a free body that is pinned, against the prescribed pose;
 * 3D AMR macro-steps over the live chunks only, against single macro-steps,
-  whose last substep covers every tile cell.
+  whose last substep covers every tile cell;
+* the fused 2D AMR macro-steps with more tiles than blocks, against the six
+  launches.
 """
 import numpy as np
 import pytest
@@ -134,3 +136,23 @@ def test_amr3d_live_chunks_equal_whole_tiles(lbm, q, rb, dynamic, shape):
     for x, y in zip(*runs):
         assert np.array_equal(x, y)
     assert abs(runs[0][4][0]) > 0
+
+
+@pytest.mark.parametrize("bounceback", [0, 1])
+def test_fused_2d_macro_steps_with_more_tiles_than_blocks(lbm, bounceback):
+    from getting_air_b200 import scenarios as sc
+    s = sc.cylinder_amr(W=512, H=256, r=14.0, centre=(150.0, 128.0), u0=0.08, re=100.0, bounceback=bool(bounceback))
+    out = []
+    for fused in (True, False):
+        a = lbm.Amr2D(lbm.amr2d_config(512, 256, refine_margin=100.0, **s["kw"]))
+        a.set_fused(fused)
+        assert a.fused == fused
+        a.write_root(s["f"], s["vel"])
+        a.step(5)
+        a.step(16)
+        a.sync()
+        out.append(a.read_root() + a.read_pool() + (a.forces(), a.topology()["active"]))
+        a.close()
+    assert len(out[0][5]) > 2 * 148
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
