@@ -94,6 +94,13 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
   }
 }
 
+// c / nx by multiplication where the host found it exact (row_magic): the
+// lean kernel's two divisions a cell were 70.3 -> 68.8 us per step of 64
+// domains (4.9 M cells).
+__device__ __forceinline__ int row_of(unsigned c, int nx, unsigned magic) {
+  return magic ? (int)__umulhi(c, magic) : (int)c / nx;
+}
+
 // The fluid tiles of a D2Q9 batch (cell2_fluid). Without the bounce-back
 // and force code the update fits 64 registers, and 1024 resident
 // threads per SM keep more loads in flight: the loop is memory-latency
@@ -122,8 +129,8 @@ __global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1024 : 768) / THREA
     for (int c = td.y + threadIdx.x; c < end; c += 2 * THREADS) {
       const int c2 = c + THREADS;
       const bool two = c2 < end;
-      const int x = c % nx, r = c / nx;
-      const int x2 = two ? c2 % nx : 0, r2 = two ? c2 / nx : 0;
+      const int r = row_of((unsigned)c, nx, sp.magic), x = c - r * nx;
+      const int r2 = two ? row_of((unsigned)c2, nx, sp.magic) : 0, x2 = two ? c2 - r2 * nx : 0;
       float f[9], g[9];
       gather2<S>(fin + sp.base, sp, x, r, f);
       if (two) gather2<S>(fin + sp.base, sp, x2, r2, g);
