@@ -1757,15 +1757,23 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
     return afail(nullptr, LBM_ENOMEM, "pool of more than 2^31 cells");
   }
   // interface blocks: covered, or a covered block among the 26 neighbours
-  for (int id = 0; id < nb; ++id) {
-    const int bx = id % p.nbx, by = (id / p.nbx) % p.nby, bz = id / (p.nbx * p.nby);
-    bool keep = false;
-    for (int d = 0; d < 27 && !keep; ++d) {
-      const int nx_ = ((bx + d % 3 - 1) % p.nbx + p.nbx) % p.nbx, ny_ = ((by + (d / 3) % 3 - 1) % p.nby + p.nby) % p.nby,
-                nz_ = ((bz + d / 9 - 1) % p.nbz + p.nbz) % p.nbz;
-      keep = a->block_slot[(nz_ * p.nby + ny_) * p.nbx + nx_] >= 0;
+  // (marked from the covered ones: most blocks are far from any, and this runs
+  // for every size query, submission and creation)
+  {
+    std::vector<uint8_t> keep(nb, 0);
+    auto near3 = [](int v, int n, int out[3]) {
+      for (int k = 0; k < 3; ++k) out[k] = ((v + k - 1) % n + n) % n;
+    };
+    for (int id : a->slot_to_block) {
+      if (id < 0) continue;
+      int x[3], y[3], z[3];
+      near3(id % p.nbx, p.nbx, x);
+      near3((id / p.nbx) % p.nby, p.nby, y);
+      near3(id / (p.nbx * p.nby), p.nbz, z);
+      for (int d = 0; d < 27; ++d) keep[(z[d / 9] * p.nby + y[d / 3 % 3]) * p.nbx + x[d % 3]] = 1;
     }
-    if (keep) a->iface.push_back(id);
+    for (int id = 0; id < nb; ++id)
+      if (keep[id]) a->iface.push_back(id);
   }
   p.n_iface = (int)a->iface.size();
   if (a->dynamic) p.n_iface = nb;  // every block, filtered by the device's interface flags

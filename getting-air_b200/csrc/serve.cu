@@ -37,6 +37,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -44,6 +45,7 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include "../../include/lbm.h"
 #include "cell_update.cuh"
@@ -174,10 +176,46 @@ struct Arena {
   }
 };
 
+// A caller's seed, kept from submission to admission: 16 bytes per cell. On
+// 2 MiB boundaries with huge pages asked for, where it is large: in fresh
+// 4 KiB pages the copy of a few million cells was mostly page faults (30 MB:
+// 15 ms).
+class Seed {
+ public:
+  Seed() = default;
+  Seed(Seed &&o) noexcept : p_(o.p_) { o.p_ = nullptr; }
+  Seed &operator=(const Seed &) = delete;
+  ~Seed() { clear(); }
+  // A copy of n floats; false without memory.
+  bool copy(const float *src, int64_t n) {
+    clear();
+    constexpr size_t kHuge = size_t(2) << 20;
+    const size_t bytes = (size_t)n * sizeof(float);
+    if (bytes < 2 * kHuge) {
+      p_ = (float *)std::malloc(bytes);
+    } else {
+      const size_t whole = (bytes + kHuge - 1) / kHuge * kHuge;
+      p_ = (float *)std::aligned_alloc(kHuge, whole);
+      if (p_) madvise(p_, whole, MADV_HUGEPAGE);  // advice: its failure changes nothing
+    }
+    if (!p_) return false;
+    std::memcpy(p_, src, bytes);
+    return true;
+  }
+  void clear() {
+    std::free(p_);
+    p_ = nullptr;
+  }
+  const float *data() const { return p_; }
+
+ private:
+  float *p_ = nullptr;
+};
+
 struct Request {
   int64_t id = 0;
   lbm_config cfg{};
-  std::vector<float> mac_seed;  // empty: uniform freestream at sponge_u
+  Seed mac_seed;                // none: uniform freestream at sponge_u
   int steps = 0;
   int enq = 0;                  // steps enqueued (complete once retired)
   double t_submit = 0, t_admit = 0, t_done = 0;
@@ -361,7 +399,7 @@ int admit_amr(lbm_server *s, Request &r, bool &ok) {
   lbm_amr3d_set_stream(r.amr, r.own);
   const int64_t n = request_cells(r);
   std::vector<float> seed;
-  const float *src = r.mac_seed.empty() ? nullptr : r.mac_seed.data();
+  const float *src = r.mac_seed.data();
   if (!src) {
     const lbm_config &c = r.cfg;
     const float ux = c.sponge_u[0], uy = c.sponge_u[1], uz = c.sponge_u[2];
@@ -375,7 +413,6 @@ int admit_amr(lbm_server *s, Request &r, bool &ok) {
   rc = lbm_amr3d_init_macro(r.amr, src);
   if (rc) return sfail(s, rc, lbm_amr3d_last_error(r.amr));
   r.mac_seed.clear();
-  r.mac_seed.shrink_to_fit();
   r.state = 1;
   r.t_admit = now_s(s);
   ok = true;
@@ -435,7 +472,7 @@ int admit(lbm_server *s, Request &r, bool &ok) {
   // request's own): a pageable copy waits for its stream and returns once
   // the host buffer is staged, so neither waits for a tick in flight.
   const Pack pk = make_pack(r.cfg);
-  if (!r.mac_seed.empty()) {
+  if (r.mac_seed.data()) {
     cudaStream_t us = r.kind == 2 ? r.own : s->upload;
     cudaError_t e = cudaMemcpyAsync(r.mac, r.mac_seed.data(), n * 16, cudaMemcpyHostToDevice, us);
     if (!e) e = launch_init_eq(r.cfg.q, r.cfg.storage, r.mac, r.f[0], n, pk, us);
@@ -455,7 +492,6 @@ int admit(lbm_server *s, Request &r, bool &ok) {
   SCK(s, cudaMemsetAsync(r.counter, 0, 4, st));
   SCK(s, cudaMemsetAsync(r.force_out, 0, kForceSlots * 8, st));
   r.mac_seed.clear();
-  r.mac_seed.shrink_to_fit();
   r.state = 1;
   r.t_admit = now_s(s);
   ok = true;
@@ -749,7 +785,8 @@ int lbm_server_submit(lbm_server *s, int64_t id, const lbm_config *cfg, const fl
   r.cfg = *cfg;
   r.steps = steps;
   r.t_submit = now_s(s);
-  if (mac) r.mac_seed.assign(mac, mac + 4 * (int64_t)cfg->nx * cfg->ny * cfg->nz);
+  if (mac && !r.mac_seed.copy(mac, 4 * (int64_t)cfg->nx * cfg->ny * cfg->nz))
+    return sfail(s, LBM_ENOMEM, "no host memory for the seed");
   s->reqs.emplace(id, std::move(r));
   s->queue.push_back(id);
   return LBM_OK;
@@ -782,7 +819,7 @@ int lbm_server_submit_amr3d(lbm_server *s, int64_t id, const lbm_amr3d_config *c
   r.cfg = cfg->root;
   r.steps = steps;
   r.t_submit = now_s(s);
-  if (mac) r.mac_seed.assign(mac, mac + 4 * request_cells(r));
+  if (mac && !r.mac_seed.copy(mac, 4 * request_cells(r))) return sfail(s, LBM_ENOMEM, "no host memory for the seed");
   s->reqs.emplace(id, std::move(r));
   s->queue.push_back(id);
   return LBM_OK;
@@ -860,10 +897,9 @@ int lbm_server_read(lbm_server *s, int64_t id, float *f, float *mac) {
   Request &r = it->second;
   const int64_t n = (int64_t)r.cfg.nx * r.cfg.ny * r.cfg.nz;
   if (r.kind == 1) {
-    // the L0 level: f of the current time level and the mac
-    const int64_t qn = (int64_t)r.cfg.q * n;
-    std::vector<float> fb(f ? 0 : qn), mb(mac ? 0 : 4 * n);
-    const int rc = lbm_amr3d_read_coarse(r.amr, f ? f : fb.data(), mac ? mac : mb.data());
+    // the L0 level: f of the current time level and the mac (what is NULL is
+    // not read: the populations are 5 to 7 times the field's bytes)
+    const int rc = lbm_amr3d_read_coarse(r.amr, f, mac);
     if (rc) return sfail(s, rc, lbm_amr3d_last_error(r.amr));
     return LBM_OK;
   }
