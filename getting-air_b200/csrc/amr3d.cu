@@ -486,9 +486,7 @@ __device__ __forceinline__ void force_block(const float *__restrict__ fp, const 
     cf.ty = rz * tx - rx * tz;
     cf.tz = rx * ty - ry * tx;
   }
-  ForceAcc acc;
-  acc.add(cf);
-  publish_force<kTileThreads>(acc, p.partials, slot * force_chunks(p) + chunk);
+  publish_force<kTileThreads>(cf, p.partials, slot * force_chunks(p) + chunk);
 }
 
 template <int Q>

@@ -76,7 +76,8 @@ __device__ __forceinline__ void stage_pose(const StepParams &p, StepParams &sp) 
 //             FP32             FP16             BF16
 //   D3Q19  107.1 -> 102.6   106.6 -> 98.7    106.6 -> 99.4
 //   D3Q27  153.9 -> 146.2   154.3 -> 136.0   154.6 -> 135.6
-// and a D3Q19 FP32 sphere in 64^3 13.1 -> 9.9. (Two cells a thread in packed
+// and a D3Q19 FP32 sphere in 64^3 13.1 -> 9.9 (8.3 with publish_force's short
+// sum). (Two cells a thread in packed
 // arithmetic, and planes staged by bulk copies, both ran slower: more
 // registers, so fewer warps to hide the gather.)
 template <int Q, typename S, bool TRT>
@@ -95,11 +96,7 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
   }
   CellForce cf;
   if (c < m.lim) cell3<Q, S, TRT>(fin, fout, mac, p, x, y, m.bz, m.region, cf);
-  if (m.region) {
-    ForceAcc acc;
-    acc.add(cf);
-    publish_force<kStepThreads>(acc, p.partials, m.part);
-  }
+  if (m.region) publish_force<kStepThreads>(cf, p.partials, m.part);
 }
 
 // The step of a free body: the pose comes from the device (written by the
@@ -196,7 +193,8 @@ __global__ void __launch_bounds__(kForceThreads)
 // which outside its reach box (for a penalty body where chi is not 0) is not
 // evaluated. us per step before (every cell general, no programmatic launch)
 // and after: 512^2 FP32 12.4 -> 6.5, FP16 12.3 -> 7.5, 1000x600 16.4 -> 8.4,
-// 200x150 10.3 -> 5.7, 2048x1024 34.2 -> 31.4. (64 registers: at 40, 512^2
+// 200x150 10.3 -> 5.7, 2048x1024 34.2 -> 31.4; with publish_force's short sum
+// 5.0, 5.9, 8.2, 4.0 and 31.7. (64 registers: at 40, 512^2
 // takes 7.2 and 2048x1024, bound by HBM, 27.1. Two cells a thread: 8.5 and 46.)
 template <typename S>
 __global__ void __launch_bounds__(kStepThreads, kStepMinBlocks)
@@ -221,9 +219,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepMinBlocks)
   if (x < p.nx) cell2<S>(fin, fout, mac, p, x, by, region, cf);
   if (region) {
     const int rx = p.rbx1 - p.rbx0;
-    ForceAcc acc;
-    acc.add(cf);
-    publish_force<kStepThreads>(acc, p.partials, (by - p.rby0) * rx + (bx - p.rbx0));
+    publish_force<kStepThreads>(cf, p.partials, (by - p.rby0) * rx + (bx - p.rbx0));
   }
 }
 
