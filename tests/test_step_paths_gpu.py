@@ -156,3 +156,39 @@ def test_fused_2d_macro_steps_with_more_tiles_than_blocks(lbm, bounceback):
     assert len(out[0][5]) > 2 * 148
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("q,dims", [(19, (40, 24, 22)), (9, (70, 40, 1))])
+def test_force_counts_nonfinite_cells(lbm, q, dims):
+    """Non-finite contributions are dropped and counted, in a block's partial
+    (one cell per thread) as in the batch's running sums."""
+    import torch
+    body = dict(shape="sphere" if q == 19 else "ellipse", a=5.0, b=5.0,
+                centre=(14.0, 12.0, 11.0) if q == 19 else (30.0, 20.0, 0.0))
+    cfg = lbm.config_from(q, dims, tau=0.6, body=body, **BODY)
+    s, b = lbm.Solver(cfg), lbm.Batch([cfg])
+    n = int(np.prod(dims))
+    mac = np.tile(np.array([1.0, 0.04, 0.0, 0.0], np.float32), (n, 1))
+    s.init_macro(mac)
+    f = np.array(s.read_f())
+    # fluid cells beside the body, whole columns of them
+    x = np.arange(n) % dims[0]
+    f.reshape(q, n)[:, x == (20 if q == 19 else 36)] = np.nan
+    f.reshape(q, n)[:, x == (8 if q == 19 else 24)] = np.inf
+    f.reshape(q, n)[:, x == (19 if q == 19 else 35)] = np.nan
+    s.write_f(f)
+    b.write_f(0, f)
+    din = torch.tensor(f, device="cuda")
+    dout, force = torch.empty_like(din), torch.zeros(8, dtype=torch.float64, device="cuda")
+    lbm.step_noalloc(cfg, din.data_ptr(), dout.data_ptr(), None, force.data_ptr(),
+                     torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    s.step(1)
+    b.step(1)
+    g, h, k = s.forces(), b.forces()[0], force.cpu().numpy()
+    assert np.isfinite(g).all() and np.array_equal(g, k[:6])
+    # FP64 sums of the same cell contributions, differently grouped
+    assert np.allclose(g, h, rtol=1e-10, atol=1e-12 * np.abs(h).max())
+    assert k[6] > 0 and k[6] == int(k[6]) and k[7] == 0
+    s.close()
+    b.close()
