@@ -1562,7 +1562,6 @@ int lbm_amr2d_set_body(lbm_amr2d *a, const lbm_body *body) {
   ACK(a, cudaStreamSynchronize(a->stream));
   a->cfg.body = *body;
   a->p.body = *body;
-  a->root.body = *body;
   {
     lbm_config rc;
     root_config(a->cfg, rc);

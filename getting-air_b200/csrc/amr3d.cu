@@ -2024,7 +2024,6 @@ int lbm_amr3d_set_body(lbm_amr3d *a, const lbm_body *body) {
   if (validate_config(&r, why)) return afail(a, LBM_EINVAL, why);
   ACK(a, cudaStreamSynchronize(a->stream));
   a->cfg.root = r;
-  a->sp.body = *body;
   set_body_regions(r, a->sp, false);
   StepParams tmp = a->sp;
   int box[6];

@@ -138,8 +138,7 @@ void fill_step_params(const lbm_config &c, int64_t n, int64_t base, StepParams &
     p.ftarget[i] = lattice_weight(c.q, i) * (1.0f + 3.0f * eu + 4.5f * eu * eu - 1.5f * ufar);
   }
   p.pk = make_pack(c);
-  p.body = c.body;
-  p.ball2 = ball_square(c.body.a);
+  set_body_params(c.body, p);
   p.win = Win{};
   if (c.q != 9) {
     const int len[3] = {c.nx, c.ny, c.nz};
@@ -163,6 +162,11 @@ void fill_step_params(const lbm_config &c, int64_t n, int64_t base, StepParams &
   p.sum_layers = 0;
   p.rot = 0;
   choose_step_map(c, p);
+}
+
+void set_body_params(const lbm_body &b, StepParams &p) {
+  p.body = b;
+  p.ball2 = ball_square(b.a);
 }
 
 bool force_cell_box(const lbm_config &c, StepParams &p, int box[6]) {
@@ -198,6 +202,7 @@ bool reach_box2(const lbm_config &c, const int fbox[6], bool any, int box[6]) {
 }
 
 bool set_body_regions(const lbm_config &c, StepParams &p, bool force) {
+  set_body_params(c.body, p);
   int box[6];
   const bool any = force_cell_box(c, p, box);
   p.nbox_on = 0;

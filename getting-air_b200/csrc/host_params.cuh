@@ -20,16 +20,20 @@ int validate_config(const lbm_config *c, std::string &why);
 // regions are left for the caller.
 void fill_step_params(const lbm_config &c, int64_t n, int64_t base, StepParams &p);
 
+// The body of `p` and what the kernels keep of its shape (p.ball2). The only
+// place that sets either: fill_step_params and set_body_regions go through it.
+void set_body_params(const lbm_body &b, StepParams &p);
+
 // Cell box [x0,x1]x[y0,y1]x[z0,z1] (inclusive) outside which no cell can
 // contribute to the body force; also sets p.swept / p.swept_band. Returns
 // false when the body has no cell in the domain (force off).
 bool force_cell_box(const lbm_config &c, StepParams &p, int box[6]);
 
-// The body's regions of a dense step, from force_cell_box(): the reach box
-// p.nbox of a 3D bounce-back body (cells outside it are beyond every link,
-// so the step skips the SDF there; an empty box when the body has no cell
-// in the domain), and with `force` the launch blocks that reduce the force
-// (p.rb*). Returns p.force_on.
+// The body c.body and its regions of a dense step, from force_cell_box(): the
+// reach box p.nbox of a 3D bounce-back body (cells outside it are beyond
+// every link, so the step skips the SDF there; an empty box when the body has
+// no cell in the domain), and with `force` the launch blocks that reduce the
+// force (p.rb*). Returns p.force_on.
 bool set_body_regions(const lbm_config &c, StepParams &p, bool force);
 
 // The force region (p.rb*) of the cell box under the launch mapping of p.
