@@ -60,13 +60,12 @@ __device__ __forceinline__ int block_kind(const StepParams &p, int lo, int hi, i
 struct BlockMap {
   int c0, lim;        // first cell and end: of row by, or (flat) of the plane
   int by, bz, zg;     // row (row mapping), stored plane, the domain's plane
-  bool region;        // takes part in the force reduction, as
-  int part;           // this partial
+  int part;           // the block's force partial, or -1
+  bool region;        // takes part in the force reduction
 };
 
 // bz skips a slab's ghost plane below; zg is the domain's plane, which the
-// force region and the block kind are in. The region is read modulo the
-// grid (it can cross a windowed seam; a slab's is its own share, no seam).
+// force region (region_part) and the block kind are in.
 __device__ __forceinline__ BlockMap block_map(const StepParams &p, int bcells) {
   BlockMap m;
   m.by = blockIdx.y;
@@ -77,13 +76,8 @@ __device__ __forceinline__ BlockMap block_map(const StepParams &p, int bcells) {
   m.zg = m.bz + p.zoff;
   m.c0 = blockIdx.x * bcells;
   m.lim = p.flat ? p.nx * p.ny : p.nx;
-  int dx = (int)blockIdx.x - p.rbx0, dy = m.by - p.rby0, dz = m.zg - p.rbz0;
-  dx += dx < 0 ? (int)gridDim.x : 0;
-  dy += dy < 0 ? (int)gridDim.y : 0;
-  dz += (dz < 0 && p.zlo == 0) ? p.nzg : 0;
-  const int rx = p.rbx1 - p.rbx0, ry = p.rby1 - p.rby0, rz = p.rbz1 - p.rbz0;
-  m.region = p.force_on && dx < rx && dy < ry && dz < rz;
-  m.part = (dz * ry + dy) * rx + dx;
+  m.part = region_part(p, blockIdx.x, m.by, m.zg, gridDim.x, gridDim.y);
+  m.region = m.part >= 0;
   return m;
 }
 

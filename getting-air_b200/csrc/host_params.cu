@@ -1,4 +1,5 @@
 // Host-side parameter translation shared by every form of the solver.
+#include <algorithm>
 #include <cmath>
 
 #include "host_params.cuh"
@@ -215,6 +216,17 @@ bool set_body_regions(const lbm_config &c, StepParams &p, bool force) {
   if (!p.force_on) return false;
   set_force_blocks(box, p);
   return true;
+}
+
+void set_slab(int z0, int nzl, StepParams &p) {
+  p.nz = nzl + 2;
+  p.zoff = z0 - 1;
+  p.zlo = 1;
+  if (p.force_on) {
+    p.rbz0 = std::max(p.rbz0, z0);
+    p.rbz1 = std::min(p.rbz1, z0 + nzl);
+    if (p.rbz0 >= p.rbz1) p.force_on = 0;
+  }
 }
 
 void set_force_blocks(const int box[6], StepParams &p) {

@@ -36,6 +36,12 @@ bool force_cell_box(const lbm_config &c, StepParams &p, int box[6]);
 // force (p.rb*). Returns p.force_on.
 bool set_body_regions(const lbm_config &c, StepParams &p, bool force);
 
+// Turns the parameters of a whole domain into those of its slab of planes
+// [z0, z0 + nzl): stored plane z is domain plane z + z0 - 1 (p.nzg stays the
+// domain's), and the force region is the slab's own share of the domain's
+// (slabs take no window, so no seam).
+void set_slab(int z0, int nzl, StepParams &p);
+
 // The force region (p.rb*) of the cell box under the launch mapping of p.
 void set_force_blocks(const int box[6], StepParams &p);
 

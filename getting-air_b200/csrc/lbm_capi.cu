@@ -126,18 +126,7 @@ void fill_params(lbm_session *s) {
   p.counter = s->force_counter;
   p.force_out = s->force_out;
   set_force_region(s);  // in the whole domain's planes
-  if (!s->slab) return;
-  // a slab: stored plane z is domain plane z + z0 - 1; its force region is
-  // its own share of the domain's (slabs take no window, so no seam)
-  p.nz = s->nzl + 2;
-  p.zoff = s->z0 - 1;
-  p.nzg = s->cfg.nz;
-  p.zlo = 1;
-  if (p.force_on) {
-    p.rbz0 = std::max(p.rbz0, s->z0);
-    p.rbz1 = std::min(p.rbz1, s->z0 + s->nzl);
-    if (p.rbz0 >= p.rbz1) p.force_on = 0;
-  }
+  if (s->slab) set_slab(s->z0, s->nzl, p);
 }
 
 // Copies between the caller's array of the session's cells (Q planes of

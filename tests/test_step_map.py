@@ -1,0 +1,114 @@
+"""The launch mapping of the dense 3D step, on the CPU: the host functions the
+kernels and the sessions share, compiled into a small program.
+
+For every domain, body and slab, the launch blocks of the force region have
+the partials 0 .. force_parts - 1, each exactly once, and every cell of the
+body's force box lies in one of them: a block outside must write no partial,
+and a step reads as many as it has blocks.
+"""
+import subprocess
+
+import pytest
+
+PROGRAM = r"""
+#include <cstdio>
+#include <string>
+#include <vector>
+#include "host_params.cuh"
+using namespace lbm;
+
+static int fail(const lbm_config &c, const char *what, int z0, int nzl) {
+  std::printf("%s: %d x %d x %d, body %g at %g %g %g, slab %d + %d\n", what, c.nx, c.ny, c.nz, c.body.a, c.body.cx,
+              c.body.cy, c.body.cz, z0, nzl);
+  return 1;
+}
+
+// slab: planes [z0, z0 + nzl) of the domain (nzl 0: all of it)
+static int check(const lbm_config &c, int z0, int nzl) {
+  std::string why;
+  if (validate_config(&c, why)) return fail(c, why.c_str(), z0, nzl);
+  StepParams p{};
+  fill_step_params(c, (int64_t)c.nx * c.ny * c.nz, 0, p);
+  set_body_regions(c, p, true);
+  if (nzl) set_slab(z0, nzl, p);
+  const dim3 g = step_grid(p);
+  const int parts = p.force_on ? force_parts(c.q, p) : 0;
+  std::vector<int> seen(parts, 0);
+  int box[6];
+  StepParams t = p;
+  const bool any = force_cell_box(c, t, box);
+  const int len[3] = {c.nx, c.ny, c.nz};
+  auto inside = [&](int a, int v) {
+    int d = (v - box[2 * a]) % len[a];
+    return (d < 0 ? d + len[a] : d) <= box[2 * a + 1] - box[2 * a];
+  };
+  for (int z = 0; z < (int)g.z; ++z)
+    for (int y = 0; y < (int)g.y; ++y)
+      for (int x = 0; x < (int)g.x; ++x) {
+        const int zg = z + p.zlo + p.zoff, part = region_part(p, x, y, zg, g.x, g.y);
+        if (part < -1 || part >= parts) return fail(c, "partial out of range", z0, nzl);
+        if (part >= 0 && seen[part]++) return fail(c, "partial twice", z0, nzl);
+        bool hit = false;  // a cell of the force box in the block
+        const int first = x * kStepThreads, lim = p.flat ? c.nx * c.ny : c.nx;
+        for (int k = first; k < first + kStepThreads && k < lim; ++k) {
+          const int cx = p.flat ? k % c.nx : k, cy = p.flat ? k / c.nx : y;
+          hit = hit || (any && inside(0, cx) && inside(1, cy) && inside(2, zg));
+        }
+        if (hit && part < 0) return fail(c, "force cell without a partial", z0, nzl);
+      }
+  for (int k = 0; k < parts; ++k)
+    if (!seen[k]) return fail(c, "partial without a block", z0, nzl);
+  return 0;
+}
+
+int main() {
+  const int dims[][3] = {{40, 24, 26}, {64, 20, 30}, {128, 12, 17}, {130, 30, 9}, {7, 9, 40}, {192, 5, 3}};
+  const float at[][3] = {{0.33f, 0.5f, 0.5f}, {0.05f, 0.1f, 0.95f}, {0.9f, 0.9f, 0.02f}, {0.5f, 0.5f, 0.75f}, {0.5f, 3.0f, 0.5f}};
+  int n = 0;
+  for (auto &d : dims)
+    for (auto &f : at)
+      for (float a : {1.0f, 3.2f, 6.0f})
+        for (int kind = 0; kind < 4; ++kind) {
+          lbm_config c;
+          lbm_config_default(&c, 19, d[0], d[1], d[2]);
+          c.has_body = 1;
+          c.use_bounceback = kind != 1;
+          c.body.a = a; c.body.b = 0.7f * a; c.body.c = 1.2f * a; c.body.r = 0.1f * a;
+          c.body.shape = kind == 2 ? LBM_SHAPE_ROUNDBOX : LBM_SHAPE_SPHERE;
+          c.body.cx = f[0] * d[0]; c.body.cy = f[1] * d[1]; c.body.cz = f[2] * d[2];
+          if (kind == 3) {
+            c.window[2] = 1;
+            c.sponge_w = 2.0f;
+          }
+          if (check(c, 0, 0)) return 1;
+          ++n;
+          if (kind == 3) continue;  // a slab takes no window
+          for (int R = 1; R <= 4 && R <= d[2]; ++R)
+            for (int k = 0; k < R; ++k) {
+              const int z0 = d[2] * k / R, z1 = d[2] * (k + 1) / R;
+              if (check(c, z0, z1 - z0)) return 1;
+              ++n;
+            }
+        }
+  std::printf("ok %d\n", n);
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def program(lbm, tmp_path_factory):
+    from getting_air_b200 import build
+    d = tmp_path_factory.mktemp("step_map")
+    (d / "map.cu").write_text(PROGRAM)
+    exe = d / "map"
+    subprocess.run([build._nvcc(), "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-ffp-contract=off",
+                    "-I", str(build.CSRC), "-o", str(exe), str(d / "map.cu"), str(build.CSRC / "host_params.cu"),
+                    str(build.LIB), "-Xlinker", f"-rpath={build.LIB.parent}"], check=True)
+    return exe
+
+
+def test_force_region_blocks_have_the_partials_once(program):
+    r = subprocess.run([str(program)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.startswith("ok")
