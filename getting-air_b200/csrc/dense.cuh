@@ -120,21 +120,23 @@ LBM_HD unsigned row_magic(int nx) { return (unsigned)(((1ull << 32) + (unsigned)
 constexpr int kStepThreads = LBM_STEP_THREADS;
 constexpr int kStepMinBlocks = LBM_STEP_MIN_BLOCKS;
 
-inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
-
 // The launch blocks of the dense step grid (kStepThreads cells along x, one
 // row per block in y and z) that cover an inclusive cell box: per axis the
-// first block, wrapped into the grid, and first + count, read modulo the
-// grid -- the box of a windowed axis can cross the periodic seam. A box as
-// long as the grid covers all of it.
+// first block and first + count, read modulo the grid -- the box of a windowed
+// axis can cross the periodic seam (where its cells, not its blocks, wrap: the
+// last block of a row may hold fewer cells). A box as long as the axis, or
+// whose two ends share a block, covers all of it.
 inline void box_region(const int box[6], int nx, int ny, int nz, int r[6]) {
   const int unit[3] = {kStepThreads, 1, 1};
-  const int nb[3] = {(nx + kStepThreads - 1) / kStepThreads, ny, nz};
+  const int len[3] = {nx, ny, nz};
   for (int a = 0; a < 3; ++a) {
-    const int b0 = floor_div(box[2 * a], unit[a]), b1 = floor_div(box[2 * a + 1], unit[a]);
-    int first = b0 % nb[a], count = b1 - b0 + 1;
-    if (first < 0) first += nb[a];
-    if (count >= nb[a]) { first = 0; count = nb[a]; }
+    const int nb = (len[a] + unit[a] - 1) / unit[a], cells = box[2 * a + 1] - box[2 * a] + 1;
+    int lo = box[2 * a] % len[a];
+    if (lo < 0) lo += len[a];
+    const int hi = lo + cells - 1;
+    int first = lo / unit[a];
+    int count = (hi < len[a] ? hi / unit[a] : nb + (hi - len[a]) / unit[a]) - first + 1;
+    if (cells >= len[a] || count >= nb) { first = 0; count = nb; }
     r[2 * a] = first;
     r[2 * a + 1] = first + count;
   }

@@ -62,7 +62,7 @@ static int check(const lbm_config &c, int z0, int nzl) {
 }
 
 int main() {
-  const int dims[][3] = {{40, 24, 26}, {64, 20, 30}, {128, 12, 17}, {130, 30, 9}, {7, 9, 40}, {192, 5, 3}};
+  const int dims[][3] = {{40, 24, 26}, {64, 20, 30}, {128, 12, 17}, {130, 30, 9}, {7, 9, 40}, {192, 5, 3}, {100, 10, 12}};
   const float at[][3] = {{0.33f, 0.5f, 0.5f}, {0.05f, 0.1f, 0.95f}, {0.9f, 0.9f, 0.02f}, {0.5f, 0.5f, 0.75f}, {0.5f, 3.0f, 0.5f}};
   int n = 0;
   for (auto &d : dims)
@@ -77,7 +77,7 @@ int main() {
           c.body.shape = kind == 2 ? LBM_SHAPE_ROUNDBOX : LBM_SHAPE_SPHERE;
           c.body.cx = f[0] * d[0]; c.body.cy = f[1] * d[1]; c.body.cz = f[2] * d[2];
           if (kind == 3) {
-            c.window[2] = 1;
+            c.window[0] = c.window[2] = 1;
             c.sponge_w = 2.0f;
           }
           if (check(c, 0, 0)) return 1;

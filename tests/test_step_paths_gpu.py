@@ -5,6 +5,8 @@ or topology selects, a cell gets the same bits.
   kinds, against the same domain in a batch, which updates one cell per
   thread by plain indices;
 * the D2Q9 reach box, against the batch, which evaluates the body everywhere;
+* a moving window whose rows are no whole number of launch blocks, the body on
+  either side of the seam, against the oracle;
 * a free body that is pinned, against the prescribed pose;
 * 3D AMR macro-steps over the live chunks only, against single macro-steps,
   whose last substep covers every tile cell;
@@ -88,6 +90,25 @@ def test_2d_reach_box_equals_batch(lbm, body, bb, storage):
     f = dense_and_batch(lbm, 9, (130, 61, 1), 6, tau=0.6, storage=storage, has_body=1, use_bounceback=bb,
                         sponge_w=4.0, sponge_u=(0.04, 0.0, 0.0), body=dict(shape="ellipse", **body))
     assert abs(f[0]) > 0
+
+
+@pytest.mark.parametrize("nx,cx", [(100, 1.3), (100, 97.7), (130, 8.25), (130, 126.6), (70, 69.9)])
+def test_windowed_force_across_a_ragged_seam(lbm, oracle, nx, cx):
+    dims = (nx, 24, 22)
+    rng = np.random.RandomState(2)
+    mac = np.empty((int(np.prod(dims)), 4), np.float32)
+    mac[:, 0] = 1 + 0.01 * (rng.rand(len(mac)) - 0.5)
+    mac[:, 1:] = 0.04 * (rng.rand(len(mac), 3) - 0.5)
+    f0 = oracle.init_eq(19, mac, fp32=True)
+    cfg = lbm.config_from(19, dims, tau=0.6, has_body=1, use_bounceback=1, sponge_w=4.0, window="x", win_anchor=(30, 0, 0),
+                          body=dict(shape="sphere", centre=(cx, 11.5, 11.0), a=6.0, v=(0.1, 0.0, 0.0)))
+    s = lbm.Solver(cfg)
+    s.write_f(f0.astype(np.float32))
+    s.step(3)
+    g = s.forces()
+    s.close()
+    o = oracle.run(cfg, f0, 3)[2][-1, :6]
+    assert np.abs(g - o).max() <= 1e-4 * max(np.abs(o).max(), 1e-3)  # the bound of the seam test at whole blocks
 
 
 @pytest.mark.parametrize("storage", ["fp32", "fp16"])
