@@ -1815,7 +1815,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
     if ((e = mem.take(&a->macp, (size_t)p.P * 16))) return bail(e, "pool mac");
     if ((e = mem.take(&a->d_block_slot, nb * sizeof(int)))) return bail(e, "block_slot");
     if ((e = mem.take(&a->d_slot_to_block, a->capacity * sizeof(int)))) return bail(e, "slots");
-    if ((e = mem.take(&a->d_iface, std::max(p.n_iface, 1) * sizeof(int)))) return bail(e, "iface");
+    if ((e = mem.take(&a->d_iface, std::max<size_t>(a->iface.size(), 1) * sizeof(int)))) return bail(e, "iface");
     if ((e = mem.take(&a->d_cells, (size_t)p.T3 * sizeof(uint32_t)))) return bail(e, "cell list");
     if ((e = mem.take(&a->d_pulls, (size_t)pull_words(a->q) * p.T3 * sizeof(uint32_t)))) return bail(e, "pull table");
     for (auto *&w : a->d_work)
@@ -1889,8 +1889,9 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
       a->q_hold = (float)(qr * std::exp2(-2.0 * (double)c->q_hyst));
     }
   }
-  if (p.n_iface)
-    cudaMemcpyAsync(a->d_iface, a->iface.data(), p.n_iface * sizeof(int), cudaMemcpyHostToDevice, a->own);
+  // (a dynamic one's launches cover every block and read the flags instead)
+  if (!a->dynamic && p.n_iface)
+    cudaMemcpyAsync(a->d_iface, a->iface.data(), a->iface.size() * sizeof(int), cudaMemcpyHostToDevice, a->own);
   if ((e = cudaMemsetAsync(a->counter, 0, sizeof(unsigned int), a->own))) return bail(e, "counter");
   if ((e = cudaMemsetAsync(a->force_out, 0, kForceSlots * sizeof(double), a->own))) return bail(e, "force");
   if ((e = cudaMemsetAsync(a->tot_counter, 0, sizeof(unsigned int), a->own))) return bail(e, "totals");

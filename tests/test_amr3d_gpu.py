@@ -556,3 +556,20 @@ def test_amr3d_mid_size_hierarchies_match_oracle(lbm, oracle, dims, radius):
     assert np.abs(g - of[-1, :6]).max() <= 1e-3 * scale, (g, of[-1, :6])
     a.close()
     o.close()
+
+
+def test_dynamic_hierarchy_of_many_blocks(lbm):
+    """A dynamic hierarchy whose blocks outnumber its interface blocks by far
+    (262,144 and some hundred): it is created, steps and refines as a small
+    one does."""
+    from getting_air_b200 import scenarios as sc
+    dims = (128, 128, 128)
+    body = dict(shape="sphere", centre=(32.0, 32.0, 32.0), a=4.0, v=(0.05, 0.0, 0.0))
+    cfg = lbm.amr3d_config(19, dims, refine="body", rb=2, margin=2.0, dynamic=1, manage_every=2, max_slots=2000, tau=0.62,
+                           has_body=1, use_bounceback=1, sponge_w=4.0, body=body)
+    a = lbm.Amr3D(cfg)
+    a.init_macro(sc.uniform_macro(int(np.prod(dims)), (0.03, 0.0, 0.0)))
+    a.step(4)
+    assert a.pool_stats()["decisions"] == 2
+    assert np.isfinite(a.forces()).all() and abs(a.forces()[0]) > 0
+    a.close()
