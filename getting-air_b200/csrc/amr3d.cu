@@ -1279,7 +1279,7 @@ struct lbm_amr3d {
   unsigned char *d_want = nullptr, *d_slot_new = nullptr, *d_iface_flag = nullptr;
   int *d_free_list = nullptr, *d_counts = nullptr;
   cudaGraphExec_t manage_graph[2] = {nullptr, nullptr};
-  bool carved = false;          // device memory carved from a caller's block
+  std::vector<void *> owned;    // device allocations (none where carved from a caller's block)
   uint32_t *d_cells = nullptr;  // tile cells: interior (RB2^3) then ring, packed x | y << 8 | z << 16
   uint32_t *d_links = nullptr;  // bounce-back link code per pool cell (bounce-back bodies only)
   // the work lists of the substeps and of explode (TileWork), their lengths
@@ -1583,10 +1583,15 @@ struct DevCarve {
   char *base = nullptr;
   size_t cap = 0, used = 0;
   bool measure = false;
+  std::vector<void *> *owned = nullptr;  // where own allocations are noted
   template <class T> cudaError_t take(T **ptr, size_t bytes) {
     const size_t b = (bytes + 255) & ~size_t(255);
     if (measure) { *ptr = nullptr; used += b; return cudaSuccess; }
-    if (!base) return cudaMalloc(ptr, bytes);
+    if (!base) {
+      const cudaError_t e = cudaMalloc(ptr, bytes);
+      if (e == cudaSuccess) owned->push_back(*ptr);
+      return e;
+    }
     if (used + b > cap) return cudaErrorMemoryAllocation;
     *ptr = reinterpret_cast<T *>(base + used);
     used += b;
@@ -1597,15 +1602,7 @@ struct DevCarve {
 void release(lbm_amr3d *a) {
   if (a->stream) cudaStreamSynchronize(a->stream);
   destroy_graphs(a);
-  for (auto *ptr : {(void *)a->fc[0], (void *)a->fc[1], (void *)a->fp[0], (void *)a->fp[1], (void *)a->macc,
-                    (void *)a->macp, (void *)a->d_block_slot, (void *)a->d_slot_to_block, (void *)a->d_iface,
-                    (void *)a->partials, (void *)a->force_out, (void *)a->tot_partials, (void *)a->tot_out,
-                    (void *)a->counter, (void *)a->tot_counter, (void *)a->d_want, (void *)a->d_slot_new,
-                    (void *)a->d_iface_flag, (void *)a->d_free_list, (void *)a->d_counts, (void *)a->flux,
-                    (void *)a->d_block_q, (void *)a->d_cells, (void *)a->d_links, (void *)a->d_pulls,
-                    (void *)a->force_groups, (void *)a->d_work[0], (void *)a->d_work[1], (void *)a->d_masks,
-                    (void *)a->d_nwork, (void *)a->d_need})
-    if (!a->carved) cudaFree(ptr);
+  for (void *ptr : a->owned) cudaFree(ptr);
   if (a->host_out) cudaFreeHost(a->host_out);
   if (a->own) cudaStreamDestroy(a->own);
 
@@ -1799,7 +1796,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
   };
   cudaError_t e;
   const bool live = !mem.measure;
-  a->carved = mem.base != nullptr;
+  mem.owned = &a->owned;
   a->nch = (p.T3 + kListThreads - 1) / kListThreads;
   const size_t fcb = (size_t)a->q * p.N * sizeof(float), fpb = (size_t)a->q * p.P * sizeof(float);
   const int nfree = a->capacity - a->initial;

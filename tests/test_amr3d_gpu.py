@@ -573,3 +573,19 @@ def test_dynamic_hierarchy_of_many_blocks(lbm):
     assert a.pool_stats()["decisions"] == 2
     assert np.isfinite(a.forces()).all() and abs(a.forces()[0]) > 0
     a.close()
+
+
+def test_closed_hierarchies_give_their_memory_back(lbm):
+    """A hierarchy's lists grow with its slots: 0.6 MB each here, of which a
+    dozen closed hierarchies must hold none."""
+    import torch
+    body = dict(shape="sphere", centre=(32.0, 32.0, 32.0), a=4.0)
+    cfg = lbm.amr3d_config(19, (128, 128, 128), refine="body", rb=2, margin=2.0, dynamic=1, max_slots=40000, tau=0.62,
+                           has_body=1, use_bounceback=1, sponge_w=4.0, body=body)
+    free = []
+    for _ in range(13):
+        a = lbm.Amr3D(cfg)
+        a.close()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < 4 << 20, free
