@@ -1474,8 +1474,8 @@ void launch_coarse(lbm_amr3d *a, int cp, bool write_mac, cudaStream_t st) {
     sp.force_out = a->force_out;
   }
   dim3 grid = step_grid(sp);
-  sp.sum_layers = sum_layers_for(sp, grid.x * grid.y);
-  grid.z += sp.sum_layers;
+  if (!add_sum_layers(sp, grid, false))
+    launch_force_sum(a->partials, force_chunks(a->p) * a->p.slots, a->force_groups, a->counter, a->force_out, st);
   launch_pdl(grid, dim3(kStepThreads), st, amr3_coarse<Q>, (const float *)a->fc[cp], a->fc[1 - cp], a->macc,
              sp, (const int *)a->d_block_slot, row_magic(a->p.rb), a->p.nbx, a->p.nby);
 }

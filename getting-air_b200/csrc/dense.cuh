@@ -171,6 +171,21 @@ LBM_HD int region_part(const StepParams &p, int bx, int by, int zg, int gx, int 
 inline int sum_layers_for(const StepParams &p, unsigned layer) {
   return p.prev_parts ? (int)((sum_groups(p.prev_parts) + layer - 1) / layer) : 0;
 }
+// Puts the blocks that sum p.prev_parts in front of a step's launch grid: rows
+// in front of a D2Q9 grid (rows = true), layers in front of a 3D one. False,
+// and the sum taken out of `p`, where the grid has no room for them: the sum
+// is a launch of its own then (launch_force_sum).
+inline bool add_sum_layers(StepParams &p, dim3 &grid, bool rows) {
+  unsigned &along = rows ? grid.y : grid.z;
+  const int layers = sum_layers_for(p, rows ? grid.x : grid.x * grid.y);
+  if (along + (unsigned)layers > 65535u) {
+    p.sum_layers = p.prev_parts = 0;
+    return false;
+  }
+  p.sum_layers = layers;
+  along += layers;
+  return true;
+}
 // Launch grid of a dense 3D step (without the sum layers).
 inline dim3 step_grid(const StepParams &p) {
   const int nz = p.nz - 2 * p.zlo;
@@ -205,6 +220,10 @@ inline cudaError_t launch_pdl(dim3 g, dim3 b, cudaStream_t st, void (*k)(K...), 
 // storage: 0 fp32, 1 fp16 offset, 2 bf16 offset
 cudaError_t launch_step(int q, int storage, const void *f_in, void *f_out, float *mac,
                         const StepParams &p, cudaStream_t st);
+// The sum of `parts` force partials (sum_partials_grouped) as a launch of its
+// own, for a step that no following launch sums.
+void launch_force_sum(const double *partials, int parts, double *groups, unsigned int *counter, double *out,
+                      cudaStream_t st);
 // Free-body force pass: the cells near the body (pose p.pose_in), FP64
 // force/torque into p.force_out, then the body integrated into p.pose_out.
 // `parts` is the launch grid (the largest box's cells, kForceThreads a block).

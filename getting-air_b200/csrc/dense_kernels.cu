@@ -381,6 +381,11 @@ int grid_for(int64_t n, int threads) {
 
 }  // namespace
 
+void launch_force_sum(const double *partials, int parts, double *groups, unsigned int *counter, double *out,
+                      cudaStream_t st) {
+  launch_pdl(dim3(sum_groups(parts)), dim3(kStepThreads), st, force_finish, partials, parts, groups, counter, out);
+}
+
 namespace {
 cudaError_t launch_step_kernel(int q, int storage, const void *f_in, void *f_out, float *mac, const StepParams &p,
                                cudaStream_t st) {
@@ -399,19 +404,10 @@ cudaError_t launch_step_kernel(int q, int storage, const void *f_in, void *f_out
   dim3 grid = step_grid(p);
   if (q == 9) grid = dim3((p.nx + kStepThreads - 1) / kStepThreads, p.ny, 1);
   if (p.force_on) r.rot = q == 9 ? p.rby0 : std::max(0, p.rbz0 - p.zoff - p.zlo);
-  if (p.prev_parts) {
-    // The sum's blocks: rows in front of a D2Q9 grid, layers in front of a 3D
-    // one. (A whole plane in front of a D2Q9 grid is mostly blocks that start
-    // and leave, 0.4 ns each: 2048x1024 took 49 us per step, 34 without it.)
-    unsigned &along = q == 9 ? grid.y : grid.z;
-    r.sum_layers = sum_layers_for(p, q == 9 ? grid.x : grid.x * grid.y);
-    if (along + r.sum_layers > 65535u) {  // no room for them: a launch of their own
-      r.sum_layers = r.prev_parts = 0;
-      launch_pdl(dim3(sum_groups(p.prev_parts)), dim3(kStepThreads), st, force_finish, p.prev_partials, p.prev_parts,
-                 p.groups, p.counter, p.force_out);
-    }
-    along += r.sum_layers;
-  }
+  // (A whole plane in front of a D2Q9 grid is mostly blocks that start and
+  // leave, 0.4 ns each: 2048x1024 took 49 us per step, 34 without it.)
+  if (!add_sum_layers(r, grid, q == 9))
+    launch_force_sum(p.prev_partials, p.prev_parts, p.groups, p.counter, p.force_out, st);
   LBM_DISPATCH(q, storage, {
     auto run = [&](auto k) { launch_pdl(grid, dim3(kStepThreads), st, k, (const S *)f_in, (S *)f_out, mac, r); };
     if constexpr (Q == 9) run(d2_step<S>);
@@ -429,9 +425,7 @@ cudaError_t launch_step(int q, int storage, const void *f_in, void *f_out, float
   if (p.prev_parts && (!p.prev_partials || !p.groups || !p.counter || !p.force_out)) return cudaErrorInvalidValue;
   const cudaError_t e = launch_step_kernel(q, storage, f_in, f_out, mac, p, st);
   if (e != cudaSuccess || !p.force_on || p.defer_force) return e;
-  const int parts = force_parts(q, p);
-  launch_pdl(dim3(sum_groups(parts)), dim3(kStepThreads), st, force_finish, (const double *)p.partials, parts,
-             p.groups, p.counter, p.force_out);
+  launch_force_sum(p.partials, force_parts(q, p), p.groups, p.counter, p.force_out, st);
   return cudaGetLastError();
 }
 

@@ -589,3 +589,23 @@ def test_closed_hierarchies_give_their_memory_back(lbm):
         torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[-1] < 4 << 20, free
+
+
+def test_deep_l0_grid_sums_the_pool_force_apart(lbm):
+    """An L0 grid so deep (65,532 planes) that the launch has no room for the
+    layers of blocks that sum the pool force: the same force, to the bit, as
+    on a shorter domain, whose other end the flow cannot have reached."""
+    from getting_air_b200 import scenarios as sc
+    out = []
+    for nz in (65532, 4000):
+        dims = (12, 12, nz)
+        want = np.zeros((nz // 4, 3, 3), np.uint8)
+        want[:17] = 1  # 153 tiles: 612 partials in 10 groups, 4 layers of 3 blocks
+        a = lbm.Amr3D(lbm.amr3d_config(19, dims, refine="list", rb=4, tau=0.62, has_body=1, use_bounceback=1,
+                                       body=dict(shape="sphere", centre=(5.8, 6.1, 30.3), a=3.0)),
+                      block_want=want.ravel())
+        a.init_macro(sc.uniform_macro(int(np.prod(dims)), (0.0, 0.0, 0.04)))
+        a.step(2)
+        out.append(a.forces())
+        a.close()
+    assert np.array_equal(*out) and abs(out[0][2]) > 0
