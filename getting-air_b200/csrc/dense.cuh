@@ -152,17 +152,20 @@ LBM_HD int sum_groups(int nparts) { return nparts <= kSumOne ? 1 : (nparts + kSu
 inline int force_parts(int q, const StepParams &p) {
   return (p.rbx1 - p.rbx0) * (p.rby1 - p.rby0) * (q == 9 ? 1 : p.rbz1 - p.rbz0);
 }
-// The partial of launch block (bx, by) of the domain's plane zg in a dense 3D
-// step of gx * gy blocks a plane, or -1 outside the force region. The region is
+// Whether launch block (bx, by) of the domain's plane zg, in a dense 3D step of
+// gx * gy blocks a plane, is in the force region, and its partial. The region is
 // read modulo the grid, as it can cross a windowed seam. A slab's, its own
 // share of the domain's planes, has no seam: a plane below it wraps past it.
-LBM_HD int region_part(const StepParams &p, int bx, int by, int zg, int gx, int gy) {
+// (`part` means nothing outside the region. Returning -1 there instead of a
+// separate truth value made the 256x128x128 FP16 step 0.7 % slower.)
+LBM_HD bool region_part(const StepParams &p, int bx, int by, int zg, int gx, int gy, int &part) {
   int dx = bx - p.rbx0, dy = by - p.rby0, dz = zg - p.rbz0;
   dx += dx < 0 ? gx : 0;
   dy += dy < 0 ? gy : 0;
   dz += dz < 0 ? p.nzg : 0;
   const int rx = p.rbx1 - p.rbx0, ry = p.rby1 - p.rby0, rz = p.rbz1 - p.rbz0;
-  return p.force_on && dx < rx && dy < ry && dz < rz ? (dz * ry + dy) * rx + dx : -1;
+  part = (dz * ry + dy) * rx + dx;
+  return p.force_on && dx < rx && dy < ry && dz < rz;
 }
 // The blocks that sum the previous step's force take no cells: a sum is a
 // chain of loads, a block tree, a fence and a ticket of some microseconds, and

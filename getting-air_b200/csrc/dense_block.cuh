@@ -60,8 +60,8 @@ __device__ __forceinline__ int block_kind(const StepParams &p, int lo, int hi, i
 struct BlockMap {
   int c0, lim;        // first cell and end: of row by, or (flat) of the plane
   int by, bz, zg;     // row (row mapping), stored plane, the domain's plane
-  int part;           // the block's force partial, or -1
-  bool region;        // takes part in the force reduction
+  bool region;        // takes part in the force reduction, as
+  int part;           // this partial
 };
 
 // bz skips a slab's ghost plane below; zg is the domain's plane, which the
@@ -76,8 +76,7 @@ __device__ __forceinline__ BlockMap block_map(const StepParams &p, int bcells) {
   m.zg = m.bz + p.zoff;
   m.c0 = blockIdx.x * bcells;
   m.lim = p.flat ? p.nx * p.ny : p.nx;
-  m.part = region_part(p, blockIdx.x, m.by, m.zg, gridDim.x, gridDim.y);
-  m.region = m.part >= 0;
+  m.region = region_part(p, blockIdx.x, m.by, m.zg, gridDim.x, gridDim.y, m.part);
   return m;
 }
 

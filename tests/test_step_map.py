@@ -45,16 +45,18 @@ static int check(const lbm_config &c, int z0, int nzl) {
   for (int z = 0; z < (int)g.z; ++z)
     for (int y = 0; y < (int)g.y; ++y)
       for (int x = 0; x < (int)g.x; ++x) {
-        const int zg = z + p.zlo + p.zoff, part = region_part(p, x, y, zg, g.x, g.y);
-        if (part < -1 || part >= parts) return fail(c, "partial out of range", z0, nzl);
-        if (part >= 0 && seen[part]++) return fail(c, "partial twice", z0, nzl);
+        const int zg = z + p.zlo + p.zoff;
+        int part;
+        const bool region = region_part(p, x, y, zg, g.x, g.y, part);
+        if (region && (part < 0 || part >= parts)) return fail(c, "partial out of range", z0, nzl);
+        if (region && seen[part]++) return fail(c, "partial twice", z0, nzl);
         bool hit = false;  // a cell of the force box in the block
         const int first = x * kStepThreads, lim = p.flat ? c.nx * c.ny : c.nx;
         for (int k = first; k < first + kStepThreads && k < lim; ++k) {
           const int cx = p.flat ? k % c.nx : k, cy = p.flat ? k / c.nx : y;
           hit = hit || (any && inside(0, cx) && inside(1, cy) && inside(2, zg));
         }
-        if (hit && part < 0) return fail(c, "force cell without a partial", z0, nzl);
+        if (hit && !region) return fail(c, "force cell without a partial", z0, nzl);
       }
   for (int k = 0; k < parts; ++k)
     if (!seen[k]) return fail(c, "partial without a block", z0, nzl);
