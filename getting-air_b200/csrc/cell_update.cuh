@@ -580,8 +580,7 @@ __device__ __forceinline__ unsigned solid_links(const StepParams &p, const V3 &p
 
 // What the body and the walls mean for a cell: its distance, the body's
 // velocity there, whether it is held at the body's state (SOLID_EQ), and the
-// links to patch. Decided before the gather is issued: a body's links may
-// take a call, which would have to save the populations in flight.
+// links to patch.
 struct Geom3 {
   float phi;
   V3 us;
@@ -589,8 +588,9 @@ struct Geom3 {
   bool in_solid;
 };
 
-// (x, y, z): the cell in the domain's own coordinates.
-template <int Q>
+// (x, y, z): the cell in the domain's own coordinates. LINKS = false: of a
+// domain without a bounce-back body.
+template <int Q, bool LINKS>
 __device__ __forceinline__ Geom3 classify3(const StepParams &p, int x, int y, int z) {
   using L = Lattice<Q>;
   const int nx = p.nx, ny = p.ny, nz = p.nzg;
@@ -608,7 +608,7 @@ __device__ __forceinline__ Geom3 classify3(const StepParams &p, int x, int y, in
     g.phi = phi3(pos, p.body, p.win);
     g.us = body_velocity3(pos, p.body, p.win);
   }
-  const bool bbody = p.has_body && p.bb;
+  const bool bbody = LINKS && p.has_body && p.bb;
   // A cell held at the body's state uses nothing it pulls, so its links need
   // no patch. For the others a link reaches a solid source only from within
   // |e| <= sqrt(3) of the surface, as a signed distance is 1-Lipschitz.
@@ -632,7 +632,7 @@ __device__ __forceinline__ Geom3 classify3(const StepParams &p, int x, int y, in
 // Everything after the pull gather, for one cell: bounce-back patches,
 // moments, forcing, collision into `sink`, mac, force. `fi` is the domain's
 // base in the input arena (own-cell loads of the bounce-back patches).
-template <int Q, typename S, class Sink, bool TRT = false>
+template <int Q, typename S, class Sink, bool TRT = false, bool LINKS = true>
 __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[Q], float *__restrict__ mac,
                                            const StepParams &p, const Geom3 &g, int x, int y, int z, bool force,
                                            CellForce &cf, Sink &sink) {
@@ -647,8 +647,8 @@ __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[
   const V3 pos = {(float)x, (float)y, (float)z};
   const float phi = g.phi;
   const V3 us = g.us;
-  const unsigned solid = g.solid, wall = g.wall;
-  const bool bbody = p.has_body && p.bb, in_solid = g.in_solid;
+  const unsigned solid = LINKS ? g.solid : 0u, wall = g.wall;
+  const bool bbody = LINKS && p.has_body && p.bb, in_solid = LINKS && g.in_solid;
   float fbx = 0.f, fby = 0.f, fbz = 0.f;
 
   // 1b. Bounce-back links, all classified already (classify3): the cell's own
@@ -804,26 +804,40 @@ __device__ __forceinline__ void gather3(const S *__restrict__ fi, const StepPara
 
 // TRT: the collision is the two-relaxation-time one; callers pass
 // p.trt_dw != 0 (see collide_store).
-template <int Q, typename S, bool TRT = false>
+// LINKS: the domain may have a bounce-back body. Its links are decided before
+// the gather is issued, as they may take a call, which would have to save the
+// populations in flight. Without one (a penalty body, whose distance every
+// cell takes) the gather comes first and hides the distance; and without the
+// call the update does not spill at the step's 64 registers.
+template <int Q, typename S, bool TRT = false, bool LINKS = true>
 __device__ __forceinline__ void cell3(const S *__restrict__ fin, S *__restrict__ fout,
                                       float *__restrict__ mac, const StepParams &p, int x, int y,
                                       int z, bool force, CellForce &cf) {
   const S *fi = fin + p.base;
-  const Geom3 g = classify3<Q>(p, x, y, z + p.zoff);
+  Geom3 g;
+  if (LINKS) g = classify3<Q, true>(p, x, y, z + p.zoff);
   float f[Q];
   gather3<Q, S>(fi, p, x, y, z, f);
+  if (!LINKS) g = classify3<Q, false>(p, x, y, z + p.zoff);
   MemSink<S> sink{fout + p.base, p.n, (z * p.ny + y) * p.nx + x, p.pk};
-  cell3_core<Q, S, MemSink<S>, TRT>(fi, f, mac, p, g, x, y, z, force, cf, sink);
+  cell3_core<Q, S, MemSink<S>, TRT, LINKS>(fi, f, mac, p, g, x, y, z, force, cf, sink);
 }
 
-// cell3 with the collision picked from the launch's parameters (a
-// warp-uniform branch), for kernels that do not instantiate per collision.
+// cell3 with the collision and the kind of body picked from the domain's
+// parameters (warp-uniform branches), for kernels that do not instantiate per
+// collision.
 template <int Q, typename S>
 __device__ __forceinline__ void cell3_any(const S *__restrict__ fin, S *__restrict__ fout,
                                           float *__restrict__ mac, const StepParams &p, int x, int y,
                                           int z, bool force, CellForce &cf) {
-  if (p.trt_dw != 0.f) cell3<Q, S, true>(fin, fout, mac, p, x, y, z, force, cf);
-  else cell3<Q, S, false>(fin, fout, mac, p, x, y, z, force, cf);
+  const bool links = p.has_body && p.bb;
+  if (p.trt_dw != 0.f) {
+    if (links) cell3<Q, S, true, true>(fin, fout, mac, p, x, y, z, force, cf);
+    else cell3<Q, S, true, false>(fin, fout, mac, p, x, y, z, force, cf);
+  } else {
+    if (links) cell3<Q, S, false, true>(fin, fout, mac, p, x, y, z, force, cf);
+    else cell3<Q, S, false, false>(fin, fout, mac, p, x, y, z, force, cf);
+  }
 }
 
 // A cell that only fluid can reach: no body link within reach (or no body),
@@ -868,7 +882,7 @@ template <int Q, typename S>
 __device__ __forceinline__ void cell3_force(const S *__restrict__ fin, const StepParams &p, int x, int y, int z,
                                             CellForce &cf) {
   const S *fi = fin + p.base;
-  const Geom3 g = classify3<Q>(p, x, y, z + p.zoff);
+  const Geom3 g = classify3<Q, true>(p, x, y, z + p.zoff);
   float f[Q];
   gather3<Q, S>(fi, p, x, y, z, f);
   NullSink sink;

@@ -33,7 +33,7 @@ __device__ __forceinline__ bool span_hits(int lo, int hi, int a, int len, int n)
 // cell3_fluid, for blocks that take no part in the force reduction, have no
 // cell within reach of a bounce-back body (or no body), touch no wall and
 // are not windowed. Penalty bodies reach every cell through chi and always
-// take kGeneral. (A third kind without the sponge blend, for blocks beyond
+// take kGeneral (the dense step has a kernel of its own for them). (A third kind without the sponge blend, for blocks beyond
 // the sponge band, had fewer instructions per update but a slower step: a
 // third hot copy of the update raised instruction-fetch and memory stalls.)
 enum BlockKind { kGeneral = 0, kFluid = 1 };

@@ -65,6 +65,17 @@ def test_body_domain_equals_batch(lbm, q, trt, dims, storage):
     assert abs(f[0]) > 0
 
 
+@pytest.mark.parametrize("storage", ["fp32", "bf16"])
+@pytest.mark.parametrize("q,trt,dims,shape", [(19, 0, (66, 24, 22), "sphere"), (27, 0, (64, 26, 24), "roundbox"),
+                                              (19, 1, (100, 21, 20), "spheroid"), (27, 1, (3, 4, 5), "sphere")])
+def test_penalty_domain_equals_batch(lbm, q, trt, dims, shape, storage):
+    body = dict(shape=shape, centre=(dims[0] / 3.0, dims[1] / 2.0, dims[2] / 2.0), a=4.0, b=3.0, c=3.0,
+                r=1.0 if shape == "roundbox" else 0.0, quat=(0.96, 0.28, 0.0, 0.0), v=(0.01, 0.0, 0.0))
+    f = dense_and_batch(lbm, q, dims, 5, tau=0.58, storage=storage, trt=trt, trt_lambda=0.1875, wall=(0, 1, 0),
+                        body=body, **dict(BODY, use_bounceback=0))
+    assert abs(f[0]) > 0
+
+
 @pytest.mark.parametrize("storage", ["fp32", "fp16"])
 def test_walls_and_body_at_the_edge_equal_batch(lbm, storage):
     body = dict(shape="roundbox", centre=(3.0, 20.5, 2.0), a=4.0, b=3.0, c=3.0, r=1.0, quat=(0.96, 0.28, 0.0, 0.0))
