@@ -897,8 +897,9 @@ __global__ void __launch_bounds__(kTileThreads)
 
 // ---- L0 step, skipping covered blocks ------------------------------------
 // The dense step's launch mapping and update; the block of a cell by
-// multiplication (row_magic of rb). LINKS = false: the body is a penalty one.
-template <int Q, bool LINKS>
+// multiplication (row_magic of rb). LINKS = false: the body is a penalty one;
+// WIN: a moving window.
+template <int Q, bool LINKS, bool WIN>
 __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) / 4 : kStepMinBlocks)
     amr3_coarse(const float *__restrict__ fin, float *__restrict__ fout, float *__restrict__ mac,
                 const __grid_constant__ StepParams sp, const int *__restrict__ block_slot, unsigned rb_magic, int nbx,
@@ -913,7 +914,7 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
   auto blk = [&](int v) { return (int)__umulhi((unsigned)v, rb_magic); };  // v / rb
   if (block_slot[(blk(m.bz) * nby + blk(y)) * nbx + blk(x)] >= 0) return;
   if (LINKS && block_kind(sp, m, kStepThreads) == kFluid) {
-    cell3_fluid<Q, float>(fin, fout, mac, sp, x, y, m.bz);
+    cell3_fluid<Q, float, false, WIN>(fin, fout, mac, sp, x, y, m.bz);
     return;
   }
   CellForce cf;
@@ -1476,9 +1477,10 @@ void launch_coarse(lbm_amr3d *a, int cp, bool write_mac, cudaStream_t st) {
   dim3 grid = step_grid(sp);
   if (!add_sum_layers(sp, grid, false))
     launch_force_sum(a->partials, force_chunks(a->p) * a->p.slots, a->force_groups, a->counter, a->force_out, st);
-  launch_pdl(grid, dim3(kStepThreads), st, sp.has_body && !sp.bb ? amr3_coarse<Q, false> : amr3_coarse<Q, true>,
-             (const float *)a->fc[cp], a->fc[1 - cp], a->macc, sp, (const int *)a->d_block_slot, row_magic(a->p.rb),
-             a->p.nbx, a->p.nby);
+  auto k = sp.has_body && !sp.bb ? amr3_coarse<Q, false, false>
+                                 : (sp.win.on ? amr3_coarse<Q, true, true> : amr3_coarse<Q, true, false>);
+  launch_pdl(grid, dim3(kStepThreads), st, k, (const float *)a->fc[cp], a->fc[1 - cp], a->macc, sp,
+             (const int *)a->d_block_slot, row_magic(a->p.rb), a->p.nbx, a->p.nby);
 }
 
 // One macro-step from L0 parity `cp`.

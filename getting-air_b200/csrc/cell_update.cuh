@@ -629,6 +629,22 @@ __device__ __forceinline__ Geom3 classify3(const StepParams &p, int x, int y, in
   return g;
 }
 
+// A 3D cell's position in window coordinates.
+__device__ __forceinline__ V3 window_pos(const StepParams &p, const V3 &pos) {
+  return {win_coord1(pos.x, win_offset1(p.body.cx, p.win.anchor[0], p.win.n[0]), p.win.n[0]),
+          win_coord1(pos.y, win_offset1(p.body.cy, p.win.anchor[1], p.win.n[1]), p.win.n[1]),
+          win_coord1(pos.z, win_offset1(p.body.cz, p.win.anchor[2], p.win.n[2]), p.win.n[2])};
+}
+
+// The sponge weight of a 3D cell (p.sponge_w > 0), from its position in window
+// coordinates: under a moving window the band travels with the body.
+__device__ __forceinline__ float sponge3(const StepParams &p, const V3 &pos) {
+  const float dx = p.sax ? fminf(pos.x, (float)(p.nx - 1) - pos.x) : 1e30f;
+  const float dy = p.say ? fminf(pos.y, (float)(p.ny - 1) - pos.y) : 1e30f;
+  const float dz = p.saz ? fminf(pos.z, (float)(p.nzg - 1) - pos.z) : 1e30f;
+  return sponge_weight_inv(fminf(dx, fminf(dy, dz)), p.sponge_inv);
+}
+
 // Everything after the pull gather, for one cell: bounce-back patches,
 // moments, forcing, collision into `sink`, mac, force. `fi` is the domain's
 // base in the input arena (own-cell loads of the bounce-back patches).
@@ -710,20 +726,7 @@ __device__ __forceinline__ void cell3_core(const S *__restrict__ fi, float (&f)[
   const float uz = fmaf(Fz, hinv, uzs);
 
   float spw = 0.f;
-  if (p.sponge_w > 0.f) {
-    // distances in window coordinates: under a moving window the band
-    // travels with the body (the identity without one)
-    V3 wp = pos;
-    if (p.win.on) {
-      wp.x = win_coord1(pos.x, win_offset1(p.body.cx, p.win.anchor[0], p.win.n[0]), p.win.n[0]);
-      wp.y = win_coord1(pos.y, win_offset1(p.body.cy, p.win.anchor[1], p.win.n[1]), p.win.n[1]);
-      wp.z = win_coord1(pos.z, win_offset1(p.body.cz, p.win.anchor[2], p.win.n[2]), p.win.n[2]);
-    }
-    const float dx = p.sax ? fminf(wp.x, (float)(nx - 1) - wp.x) : 1e30f;
-    const float dy = p.say ? fminf(wp.y, (float)(ny - 1) - wp.y) : 1e30f;
-    const float dz = p.saz ? fminf(wp.z, (float)(nz - 1) - wp.z) : 1e30f;
-    spw = sponge_weight_inv(fminf(dx, fminf(dy, dz)), p.sponge_inv);
-  }
+  if (p.sponge_w > 0.f) spw = sponge3(p, p.win.on ? window_pos(p, pos) : pos);
 
   // 4. Collide + sponge blend, 5. solid interior held at feq(1, u_body).
   if (!in_solid) {
@@ -841,12 +844,11 @@ __device__ __forceinline__ void cell3_any(const S *__restrict__ fin, S *__restri
 }
 
 // A cell that only fluid can reach: no body link within reach (or no body),
-// no wall on any of its links, no moving window, and not in the force
-// reduction. For such a cell cell3() finds phi = 1e30, u_s = 0 and chi = 0,
-// so its Guo force is the body force alone (rho chi (u_s - u*) = +-0, and
+// no wall on any of its links, and not in the force reduction. For such a
+// cell cell3() finds phi = 1e30, u_s = 0 and chi = 0, so its Guo force is the body force alone (rho chi (u_s - u*) = +-0, and
 // +-0 + F = F) and nothing is patched; this is that path with the dead
-// tests taken out, to the bit.
-template <int Q, typename S, bool TRT = false>
+// tests taken out, to the bit. WIN: the domain has a moving window.
+template <int Q, typename S, bool TRT = false, bool WIN = false>
 __device__ __forceinline__ void cell3_fluid(const S *__restrict__ fin, S *__restrict__ fout,
                                             float *__restrict__ mac, const StepParams &p, int x, int y, int z) {
   using L = Lattice<Q>;
@@ -863,11 +865,8 @@ __device__ __forceinline__ void cell3_fluid(const S *__restrict__ fin, S *__rest
   const float uz = fmaf(p.fz, hinv, uzs);
   float spw = 0.f;
   if (p.sponge_w > 0.f) {
-    const float dx = p.sax ? fminf((float)x, (float)(p.nx - 1) - (float)x) : 1e30f;
-    const float dy = p.say ? fminf((float)y, (float)(p.ny - 1) - (float)y) : 1e30f;
-    const float zg = (float)(z + p.zoff);
-    const float dz = p.saz ? fminf(zg, (float)(p.nzg - 1) - zg) : 1e30f;
-    spw = sponge_weight_inv(fminf(dx, fminf(dy, dz)), p.sponge_inv);
+    const V3 pos = {(float)x, (float)y, (float)(z + p.zoff)};
+    spw = sponge3(p, WIN ? window_pos(p, pos) : pos);
   }
   const int cell = (z * p.ny + y) * p.nx + x;
   MemSink<S> sink{fout + p.base, p.n, cell, p.pk};

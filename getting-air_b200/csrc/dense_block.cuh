@@ -31,8 +31,9 @@ __device__ __forceinline__ bool span_hits(int lo, int hi, int a, int len, int n)
 // What a launch block of the 3D step must evaluate, decided once per block
 // (warp-uniform): kGeneral runs cell3 for every cell; kFluid runs
 // cell3_fluid, for blocks that take no part in the force reduction, have no
-// cell within reach of a bounce-back body (or no body), touch no wall and
-// are not windowed. Penalty bodies reach every cell through chi and always
+// cell within reach of a bounce-back body (or no body) and touch no wall.
+// (Under a moving window the fluid update needs the body's position: a free
+// body's step, whose launch does not have it, takes kGeneral.) Penalty bodies reach every cell through chi and always
 // take kGeneral (the dense step has a kernel of its own for them). (A third kind without the sponge blend, for blocks beyond
 // the sponge band, had fewer instructions per update but a slower step: a
 // third hot copy of the update raised instruction-fetch and memory stalls.)
@@ -43,7 +44,7 @@ enum BlockKind { kGeneral = 0, kFluid = 1 };
 // The tests in the order that leaves most blocks early.
 __device__ __forceinline__ int block_kind(const StepParams &p, int lo, int hi, int y0, int y1, int z, bool region,
                                           int nbox_on, const int *nbox) {
-  if (region || p.win.on) return kGeneral;
+  if (region) return kGeneral;
   if (p.has_body) {
     if (!p.bb || !nbox_on) return kGeneral;
     if (span_hits(z, z, nbox[4], nbox[5] - nbox[4], p.nzg) && span_hits(y0, y1, nbox[2], nbox[3] - nbox[2], p.ny) &&

@@ -145,6 +145,34 @@ def test_pinned_free_body_equals_prescribed_pose(lbm, shape, bb, storage):
     assert np.allclose(out[0][2], out[1][2], rtol=1e-10, atol=1e-12 * np.abs(out[0][2]).max())
 
 
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("q,trt,dims,window,cx", [(19, 0, (130, 30, 28), "x", 4.3), (27, 1, (64, 27, 40), "xyz", 61.7),
+                                                  (19, 1, (96, 40, 26), "yz", 40.2)])
+def test_windowed_fluid_blocks_equal_the_general_update(lbm, q, trt, dims, window, cx, storage):
+    """A prescribed body's windowed step runs its fluid blocks apart; a free
+    body's, here pinned to the same pose, updates every cell alike."""
+    n = int(np.prod(dims))
+    rng = np.random.RandomState(4)
+    mac = np.empty((n, 4), np.float32)
+    mac[:, 0] = 1 + 0.01 * (rng.rand(n) - 0.5)
+    mac[:, 1:] = 0.04 * (rng.rand(n, 3) - 0.4)
+    body = dict(shape="sphere", centre=(cx, dims[1] - 2.4, 3.7), a=4.0)
+    cfg = lbm.config_from(q, dims, tau=0.6, storage=storage, trt=trt, trt_lambda=0.1875, window=window,
+                          win_anchor=(20, 11, 12), body=body, **dict(BODY, sponge_w=6.0))
+    out = []
+    for free in (False, True):
+        s = lbm.Solver(cfg)
+        s.init_macro(mac)
+        if free:
+            s.set_free_body(lbm.body_state(cfg.body, 1.0), lbm.body_opts(pinned=1))
+        s.step(5)
+        out.append((s.read_f(), s.read_mac(), s.forces()))
+        s.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.allclose(out[0][2], out[1][2], rtol=1e-10, atol=1e-12 * np.abs(out[0][2]).max())
+
+
 @pytest.mark.parametrize("q,rb,dynamic,shape", [(19, 4, 0, "roundbox"), (27, 4, 0, "sphere"), (19, 2, 0, "sphere"),
                                                 (19, 3, 0, "roundbox"), (19, 4, 1, "sphere")])
 def test_amr3d_live_chunks_equal_whole_tiles(lbm, q, rb, dynamic, shape):
