@@ -176,12 +176,23 @@ inline int sum_layers_for(const StepParams &p, unsigned layer) {
 }
 // Puts the blocks that sum p.prev_parts in front of a step's launch grid: rows
 // in front of a D2Q9 grid (rows = true), layers in front of a 3D one. False,
-// and the sum taken out of `p`, where the grid has no room for them: the sum
-// is a launch of its own then (launch_force_sum).
+// and the sum taken out of `p`, where the sum is better a launch of its own
+// (launch_force_sum): the grid has no room for the layers, or a 3D layer has
+// more than kSumLayer blocks. Most of a layer's blocks only start and leave, 0.4
+// ns each, and the launch costs 3 to 5 us: us per step of D3Q19 with a small
+// body, with the layer and with the launch, FP32 and FP16, 600x500x5 (4688
+// blocks) 40.8 and 44.5, 41.5 and 45.2; 1000x1000x8 (15,625) 198.1 and 197.7,
+// 184.2 and 183.3; 1024x1024x8 (16,384) 207.5 and 203.1, 191.7 and 187.2;
+// 2048x512x6 (16,384) 157.8 and 154.3, 146.8 and 143.0. (The sum in the grid's
+// own first blocks, before their cells: 2 us less for such domains, and 1 %
+// more for all others, as the kernel then held the sum and the update in one
+// path.)
+constexpr unsigned kSumLayer = 12288;
 inline bool add_sum_layers(StepParams &p, dim3 &grid, bool rows) {
   unsigned &along = rows ? grid.y : grid.z;
-  const int layers = sum_layers_for(p, rows ? grid.x : grid.x * grid.y);
-  if (along + (unsigned)layers > 65535u) {
+  const unsigned layer = rows ? grid.x : grid.x * grid.y;
+  const int layers = sum_layers_for(p, layer);
+  if (p.prev_parts && (along + (unsigned)layers > 65535u || (!rows && layer > kSumLayer))) {
     p.sum_layers = p.prev_parts = 0;
     return false;
   }

@@ -4,7 +4,9 @@ kernels and the sessions share, compiled into a small program.
 For every domain, body and slab, the launch blocks of the force region have
 the partials 0 .. force_parts - 1, each exactly once, and every cell of the
 body's force box lies in one of them: a block outside must write no partial,
-and a step reads as many as it has blocks.
+and a step reads as many as it has blocks. And the blocks in front of the grid
+that sum the previous step's partials hold each group of them once, the rest
+each block of the grid once.
 """
 import subprocess
 
@@ -63,7 +65,52 @@ static int check(const lbm_config &c, int z0, int nzl) {
   return 0;
 }
 
+// The launch with the sum of `parts` partials in front of the grid.
+static int check_sum(const lbm_config &c, int parts) {
+  StepParams p{};
+  fill_step_params(c, (int64_t)c.nx * c.ny * c.nz, 0, p);
+  const bool rows = c.q == 9;
+  const dim3 g0 = rows ? dim3((c.nx + kStepThreads - 1) / kStepThreads, c.ny, 1) : step_grid(p);
+  dim3 g = g0;
+  p.prev_parts = parts;
+  if (!add_sum_layers(p, g, rows)) {
+    if (parts && !p.prev_parts && g.x == g0.x && g.y == g0.y && g.z == g0.z) return 0;
+    return fail(c, "a sum left out changes the grid", 0, parts);
+  }
+  const int groups = sum_groups(parts);
+  std::vector<int> sums(groups, 0);
+  std::vector<char> cells((size_t)g0.x * g0.y * g0.z, 0);
+  for (int z = 0; z < (int)g.z; ++z)
+    for (int y = 0; y < (int)g.y; ++y)
+      for (int x = 0; x < (int)g.x; ++x) {
+        const int64_t b = x + (int64_t)g.x * (y + (int64_t)g.y * z);
+        if ((rows ? y : z) < p.sum_layers) {
+          if (b < groups && sums[b]++) return fail(c, "group twice", 0, parts);
+          continue;
+        }
+        const int by = rows ? y - p.sum_layers : y, bz = rows ? z : z - p.sum_layers;
+        if (by >= (int)g0.y || bz >= (int)g0.z || cells[((size_t)bz * g0.y + by) * g0.x + x]++)
+          return fail(c, "block outside the grid or twice", 0, parts);
+      }
+  for (int k = 0; k < groups; ++k)
+    if (parts && sums[k] != 1) return fail(c, "group without a block", 0, parts);
+  for (char k : cells)
+    if (k != 1) return fail(c, "cells without a block", 0, parts);
+  return 0;
+}
+
 int main() {
+  for (int parts : {0, 1, 64, 256, 257, 5000, 70000})
+    for (int q : {9, 19})
+      for (auto &d : {std::vector<int>{40, 24, 26}, {64, 20, 30}, {1024, 300, 4}, {100, 90, 3}, {7, 9, 2000}, {256, 128, 128},
+                      {2048, 3, 3}, {2048, 512, 6}, {1000, 1000, 3}}) {
+        lbm_config c;
+        lbm_config_default(&c, q, d[0], d[1], q == 9 ? 1 : d[2]);
+        if (check_sum(c, parts)) return 1;
+      }
+  lbm_config deep;
+  lbm_config_default(&deep, 19, 12, 12, 65532);
+  if (check_sum(deep, 612)) return 1;
   const int dims[][3] = {{40, 24, 26}, {64, 20, 30}, {128, 12, 17}, {130, 30, 9}, {7, 9, 40}, {192, 5, 3}, {100, 10, 12}};
   const float at[][3] = {{0.33f, 0.5f, 0.5f}, {0.05f, 0.1f, 0.95f}, {0.9f, 0.9f, 0.02f}, {0.5f, 0.5f, 0.75f}, {0.5f, 3.0f, 0.5f}};
   int n = 0;
