@@ -100,7 +100,7 @@ __device__ __forceinline__ bool tile_cell(const Amr3Params &p, TileCell &t) {
 // substep), so only the last macro-step's first substep updates the dead
 // cells with links (need), and one whose every link bounces keeps its value
 // (hold). A moving body's bounce depends on the whole history: then every
-// substep updates the cells of need. Where dead cells are read after all (the
+// substep updates the cells of need (or all, where those are most). Where dead cells are read after all (the
 // penalty force's tile-clamped gather; the interp interface, whose ring
 // collides), and without the link table, every substep runs over every cell
 // (p.live = 0). Bound by instruction issue and the latency of the neighbour
@@ -108,6 +108,10 @@ __device__ __forceinline__ bool tile_cell(const Amr3Params &p, TileCell &t) {
 // tiles around a box in 180^3: 660 -> 447 us; 160 tiles around a
 // sphere in 192x128x128, where the coarse step is most of it: 154 -> 139 us.
 constexpr int kListThreads = 128;
+constexpr int kWorkCounts = 4;  // lengths of the work lists, and the chunks of all tiles
+// Threads and CTAs of amr3_work, a thread per slot: one CTA where it holds all.
+inline int work_threads(int capacity) { return capacity <= 1024 ? (capacity + 31) / 32 * 32 : 128; }
+inline int work_ctas(int capacity) { return (capacity + work_threads(capacity) - 1) / work_threads(capacity); }
 
 // Work items (slot << 8 | chunk) of a launch; items NULL: a 2D grid of
 // (chunk, slot). count (dynamic hierarchies): the items in use of the grid.
@@ -285,16 +289,27 @@ __device__ __forceinline__ V3 tile_pos(const Amr3Params &p, const TileCell &t) {
 }
 
 // Every cell (ring included) of every live tile, or of the tiles flagged in
-// only_new (the manager's grants).
+// only_new (the manager's grants). And per (chunk, slot), in need, whether a
+// ring cell has links into the body and is not on hold (substep_cell).
 template <int Q>
 __global__ void __launch_bounds__(kListThreads)
     amr3_links(const __grid_constant__ Amr3Params p, uint32_t *__restrict__ links, const uint32_t *__restrict__ cells,
-               const unsigned char *__restrict__ only_new) {
+               const unsigned char *__restrict__ only_new, unsigned char *__restrict__ need) {
+  constexpr uint32_t kAll = (1u << Q) - 1u;
   TileCell t;
   __shared__ int nb27[27];
-  if (!list_cell(p, cells, {nullptr, nullptr}, nb27, t)) return;
-  if (only_new && !only_new[t.slot]) return;
-  links[t.cell] = link_code<Q>(p, t, phi3(tile_pos(p, t), p.c.body, p.c.win));
+  t.slot = blockIdx.y;
+  if ((only_new && !only_new[t.slot]) || !list_tile(p, nb27, t, false)) return;  // the whole CTA
+  const int k = blockIdx.x * kListThreads + threadIdx.x;
+  bool mine = false;
+  if (k < p.T3) {
+    list_at(p, cells, k, t);
+    const uint32_t code = link_code<Q>(p, t, phi3(tile_pos(p, t), p.c.body, p.c.win));
+    links[t.cell] = code;
+    mine = t.nb != 13 && (code & kAll) && !(p.resting && (code & kAll) == kAll);
+  }
+  const int any = __syncthreads_or(mine);
+  if (threadIdx.x == 0) need[t.slot * gridDim.x + blockIdx.x] = any ? 1 : 0;
 }
 
 // ---- explode ------------------------------------------------------------
@@ -1150,75 +1165,76 @@ __global__ void __launch_bounds__(kManageThreads)
   }
 }
 
-// Per (chunk, slot): whether a ring cell has links into the body and is not
-// on hold (substep_cell).
-template <int Q>
-__global__ void __launch_bounds__(kListThreads)
-    amr3_need(const __grid_constant__ Amr3Params p, const uint32_t *__restrict__ cells,
-              unsigned char *__restrict__ need) {
-  constexpr uint32_t kAll = (1u << Q) - 1u;
-  const int k = blockIdx.x * kListThreads + threadIdx.x, slot = blockIdx.y;
-  bool mine = false;
-  if (k < p.T3 && p.links && p.slot_to_block[slot] >= 0) {
-    const uint32_t c = __ldg(cells + k);
-    const int fx = c & 0xff, fy = (c >> 8) & 0xff, fz = (c >> 16) & 0xff;
-    const uint32_t code = p.links[(int64_t)slot * p.T3 + (fz * p.FB + fy) * p.FB + fx] & kAll;
-    mine = (c >> 24) != 13 && code && !(p.resting && code == kAll);
-  }
-  const int any = __syncthreads_or(mine);
-  if (threadIdx.x == 0) need[slot * gridDim.x + blockIdx.x] = any ? 1 : 0;
-}
-
-// The work lists, one CTA, after each change of the tiles or of the body: in
-// slot order, the chunks whose groups of cells (mask, one bit per neighbour
-// block, bit 13 the interior) hold a live one (the substeps'), those with a
-// live ring cell (explode's), and the substeps' with those that amr3_need
-// flagged; n their lengths.
-__global__ void __launch_bounds__(kManageThreads)
+// The work lists, after each change of the tiles or of the body: in slot order,
+// the chunks whose groups of cells (mask, one bit per neighbour block, bit 13 the
+// interior) hold a live one (the substeps'), those with a live ring cell
+// (explode's), and the substeps' with those that amr3_links flagged. A thread
+// per slot. One CTA, where it holds all slots; else two launches: each CTA's
+// counts, then (FILL) the items, each CTA behind those before it. From the last
+// one the lengths and the number of all tiles' chunks (n). In one CTA over all slots they took 63 us for 2262
+// tiles, at every decision of a manager; appended by atomics, out of slot order,
+// the substeps that walked them took 1.3 % longer.
+template <bool FILL>
+__global__ void __launch_bounds__(1024)
     amr3_work(const int *__restrict__ block_slot, const int *__restrict__ slot_to_block,
               const uint32_t *__restrict__ masks, int nch, int nbx, int nby, int nbz, int capacity,
               const unsigned char *__restrict__ need, uint32_t *__restrict__ sub, uint32_t *__restrict__ expl,
-              uint32_t *__restrict__ with_need, int *__restrict__ n) {
+              uint32_t *__restrict__ with_need, int4 *__restrict__ counts, int *__restrict__ n) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // a no-op unless launched by launch_pdl
   __shared__ int sm[64];
-  int ns = 0, ne = 0, nw = 0;
-  for (int base = 0; base < capacity; base += kManageThreads) {
-    const int slot = base + threadIdx.x;
-    const int id = slot < capacity ? slot_to_block[slot] : -1;
-    uint32_t live = 0;  // the neighbours that hold no tile
-    if (id >= 0) {
-      const int bx = id % nbx, by = (id / nbx) % nby, bz = id / (nbx * nby);
-      for (int d = 0; d < 27; ++d) {
-        const int x = (bx + d % 3 - 1 + nbx) % nbx, y = (by + (d / 3) % 3 - 1 + nby) % nby,
-                  z = (bz + d / 9 - 1 + nbz) % nbz;
-        if (d != 13 && block_slot[(z * nby + y) * nbx + x] < 0) live |= 1u << d;
-      }
+  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+  const int id = slot < capacity ? slot_to_block[slot] : -1;
+  uint32_t live = 0;  // the neighbours that hold no tile
+  if (id >= 0) {
+    const int bx = id % nbx, by = (id / nbx) % nby, bz = id / (nbx * nby);
+    for (int d = 0; d < 27; ++d) {
+      const int x = (bx + d % 3 - 1 + nbx) % nbx, y = (by + (d / 3) % 3 - 1 + nby) % nby,
+                z = (bz + d / 9 - 1 + nbz) % nbz;
+      if (d != 13 && block_slot[(z * nby + y) * nbx + x] < 0) live |= 1u << d;
     }
-    int cs = 0, ce = 0, cw = 0;
-    for (int c = 0; c < nch && id >= 0; ++c) {
-      const bool l = masks[c] & (live | 1u << 13);
-      cs += l;
-      ce += (masks[c] & live) != 0;
-      cw += l || need[slot * nch + c];
-    }
-    int ts, te, tw;
-    int rs = ns + block_scan(cs, sm, ts);
-    int re = ne + block_scan(ce, sm, te);
-    int rw = nw + block_scan(cw, sm, tw);
-    for (int c = 0; c < nch && id >= 0; ++c) {
-      const bool l = masks[c] & (live | 1u << 13);
-      const uint32_t item = (uint32_t)slot << 8 | c;
-      if (l) sub[rs++] = item;
-      if (masks[c] & live) expl[re++] = item;
-      if (l || need[slot * nch + c]) with_need[rw++] = item;
-    }
-    ns += ts;
-    ne += te;
-    nw += tw;
   }
-  if (threadIdx.x == 0) {
-    n[0] = ns;
-    n[1] = ne;
-    n[2] = nw;
+  int cs = 0, ce = 0, cw = 0;
+  for (int c = 0; c < nch && id >= 0; ++c) {
+    const bool l = masks[c] & (live | 1u << 13);
+    cs += l;
+    ce += (masks[c] & live) != 0;
+    cw += l || need[slot * nch + c];
+  }
+  int4 t;
+  int rs = block_scan(cs, sm, t.x), re = block_scan(ce, sm, t.y), rw = block_scan(cw, sm, t.z);
+  block_scan(id >= 0 ? nch : 0, sm, t.w);
+  if (!FILL) {
+    if (threadIdx.x == 0) counts[blockIdx.x] = t;
+    return;
+  }
+  int4 before = {0, 0, 0, 0};
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) {
+    const int4 c = counts[k];
+    before.x += c.x;
+    before.y += c.y;
+    before.z += c.z;
+    before.w += c.w;
+  }
+  int4 base;
+  block_scan(before.x, sm, base.x);
+  block_scan(before.y, sm, base.y);
+  block_scan(before.z, sm, base.z);
+  block_scan(before.w, sm, base.w);
+  rs += base.x;
+  re += base.y;
+  rw += base.z;
+  for (int c = 0; c < nch && id >= 0; ++c) {
+    const bool l = masks[c] & (live | 1u << 13);
+    const uint32_t item = (uint32_t)slot << 8 | c;
+    if (l) sub[rs++] = item;
+    if (masks[c] & live) expl[re++] = item;
+    if (l || need[slot * nch + c]) with_need[rw++] = item;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    n[0] = base.x + t.x;
+    n[1] = base.y + t.y;
+    n[2] = base.z + t.z;
+    n[3] = base.w + t.w;
   }
 }
 
@@ -1285,11 +1301,13 @@ struct lbm_amr3d {
   uint32_t *d_links = nullptr;  // bounce-back link code per pool cell (bounce-back bodies only)
   // the work lists of the substeps and of explode (TileWork), their lengths
   // on the device (dynamic) or in n_work, each chunk's groups of cells, and
-  // the chunks amr3_need flags
+  // the chunks amr3_links flags
   uint32_t *d_work[3] = {nullptr, nullptr, nullptr}, *d_masks = nullptr;
   int *d_nwork = nullptr;
+  int4 *d_counts_cta = nullptr;
   unsigned char *d_need = nullptr;
   int n_work[3] = {0, 0, 0}, nch = 0;
+  bool work_stale = true, need_pays = true;  // kNeed's list (update_work)
   uint32_t *d_pulls = nullptr;  // substep pull sources per (direction, cell list position), of both lists
   int coalesce_subs = 1;        // threads per L0 cell in the coalesce
   float *d_block_q = nullptr;   // field criterion: per-block max Q (NULL = off)
@@ -1330,32 +1348,47 @@ cudaError_t launch_interp(lbm_amr3d *a, const float *fc, int ring_only, const un
 cudaError_t launch_links(lbm_amr3d *a, const unsigned char *only_new) {
   if (!a->p.slots || !a->p.links) return cudaSuccess;
   const dim3 gl((a->p.T3 + kListThreads - 1) / kListThreads, a->p.slots);
-  AMR3_DISPATCH(a->q, amr3_links<Q><<<gl, kListThreads, 0, a->stream>>>(a->p, a->d_links, a->d_cells, only_new));
+  AMR3_DISPATCH(a->q, amr3_links<Q><<<gl, kListThreads, 0, a->stream>>>(a->p, a->d_links, a->d_cells, only_new, a->d_need));
 }
 
 // The work lists for the current tiles and links.
 cudaError_t launch_work(lbm_amr3d *a) {
   const Amr3Params &p = a->p;
-  const auto lists = [&] {
-    amr3_work<<<1, kManageThreads, 0, a->stream>>>(a->d_block_slot, a->d_slot_to_block, a->d_masks, a->nch, p.nbx, p.nby,
-                                                   p.nbz, a->capacity, a->d_need, a->d_work[0], a->d_work[1],
-                                                   a->d_work[2], a->d_nwork);
+  const int grid = work_ctas(a->capacity);
+  auto run = [&](auto k) {
+    launch_pdl(dim3(grid), dim3(work_threads(a->capacity)), a->stream, k, (const int *)a->d_block_slot,
+               (const int *)a->d_slot_to_block, (const uint32_t *)a->d_masks, a->nch, p.nbx, p.nby, p.nbz, a->capacity,
+               (const unsigned char *)a->d_need, a->d_work[0], a->d_work[1], a->d_work[2], a->d_counts_cta, a->d_nwork);
   };
-  const dim3 g(a->nch, p.slots);
-  AMR3_DISPATCH(a->q, amr3_need<Q><<<g, kListThreads, 0, a->stream>>>(p, a->d_cells, a->d_need); lists());
+  if (grid > 1) run(amr3_work<false>);
+  run(amr3_work<true>);
+  return cudaGetLastError();
 }
 
-// The same outside the manager's graph: a static hierarchy also learns its
-// lists' lengths, its launches' grids.
-int rebuild_work(lbm_amr3d *a) {
+// What the work lists depend on besides the tiles, from the body and the link
+// table: kNeed's list is out of date until update_work.
+void set_work_rules(lbm_amr3d *a) {
   const bool bb = a->p.c.has_body && a->p.c.bb;
   const lbm_body &b = a->p.c.body;
   a->p.resting = bb && b.vx == 0.f && b.vy == 0.f && b.vz == 0.f && b.wx == 0.f && b.wy == 0.f && b.wz == 0.f;
   a->p.live = a->cfg.iface != 1 && (!a->p.c.has_body || (bb && a->p.links)) ? 1 : 0;
+  a->work_stale = true;
+}
+
+// The work lists outside the manager's graph, with their lengths to the host:
+// a static hierarchy's launches' grids, and whether kNeed's list is short
+// enough to pay (a chunk of it costs 7.8 ns, one of the whole-tile launch, its
+// ring in rows, 6.1). Not for a call of one macro-step after set_body: its
+// first substep over every cell costs less than the lists.
+int update_work(lbm_amr3d *a) {
+  int n[kWorkCounts];
   ACK(a, launch_work(a));
-  if (a->dynamic) return LBM_OK;
-  ACK(a, cudaMemcpyAsync(a->n_work, a->d_nwork, sizeof(a->n_work), cudaMemcpyDeviceToHost, a->stream));
+  ACK(a, cudaMemcpyAsync(n, a->d_nwork, sizeof(n), cudaMemcpyDeviceToHost, a->stream));
   ACK(a, cudaStreamSynchronize(a->stream));
+  if (!a->dynamic)
+    for (int k = 0; k < 3; ++k) a->n_work[k] = n[k];
+  a->need_pays = 4 * (int64_t)n[2] <= 3 * (int64_t)n[3];
+  a->work_stale = false;
   return LBM_OK;
 }
 
@@ -1523,8 +1556,9 @@ cudaError_t launch_macro(lbm_amr3d *a, int cp, bool write_mac) {
   }
   if (p.slots) {
     // the last macro-step of a call leaves every cell up to date
-    const Cells most = p.resting || !p.c.has_body ? Cells::kLive : Cells::kNeed;
-    const Cells first = !p.live ? Cells::kAll : (write_mac ? Cells::kNeed : most);
+    const Cells need = a->work_stale || !a->need_pays ? Cells::kAll : Cells::kNeed;
+    const Cells most = p.resting || !p.c.has_body ? Cells::kLive : need;
+    const Cells first = !p.live ? Cells::kAll : (write_mac ? need : most);
     const Cells second = !p.live || write_mac ? Cells::kAll : most;
     auto body = [&]() -> cudaError_t {
       AMR3_DISPATCH(q, {
@@ -1827,7 +1861,8 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
     for (auto *&w : a->d_work)
       if ((e = mem.take(&w, (size_t)a->capacity * a->nch * sizeof(uint32_t)))) return bail(e, "work list");
     if ((e = mem.take(&a->d_masks, a->nch * sizeof(uint32_t)))) return bail(e, "work list");
-    if ((e = mem.take(&a->d_nwork, 3 * sizeof(int)))) return bail(e, "work list");
+    if ((e = mem.take(&a->d_nwork, kWorkCounts * sizeof(int)))) return bail(e, "work list");
+    if ((e = mem.take(&a->d_counts_cta, work_ctas(a->capacity) * sizeof(int4)))) return bail(e, "work list");
     if ((e = mem.take(&a->d_need, (size_t)a->capacity * a->nch))) return bail(e, "work list");
     if (r.has_body && r.use_bounceback && (e = mem.take(&a->d_links, (size_t)p.P * sizeof(uint32_t))))
       return bail(e, "link table");
@@ -1861,6 +1896,7 @@ int amr3_create_impl(const lbm_amr3d_config *c, const uint8_t *block_want, DevCa
     if ((e = cudaMemsetAsync(a->fp[k], 0, fpb, a->own))) return bail(e, "memset pool f");
   if (a->flux && (e = cudaMemsetAsync(a->flux, 0, (size_t)p.N * 16, a->own))) return bail(e, "memset flux");
   if ((e = cudaMemsetAsync(a->macp, 0, (size_t)p.P * 16, a->own))) return bail(e, "memset pool mac");
+  if ((e = cudaMemsetAsync(a->d_need, 0, (size_t)a->capacity * a->nch, a->own))) return bail(e, "memset work list");
   cudaMemcpyAsync(a->d_block_slot, a->block_slot.data(), nb * sizeof(int), cudaMemcpyHostToDevice, a->own);
   cudaMemcpyAsync(a->d_slot_to_block, a->slot_to_block.data(), a->capacity * sizeof(int), cudaMemcpyHostToDevice,
                   a->own);
@@ -1980,8 +2016,9 @@ int lbm_amr3d_init_macro(lbm_amr3d *a, const float *mac) {
   for (int k = 0; k < 2; ++k)
     ACK(a, launch_init_eq(a->q, LBM_STORE_FP32, a->macc, a->fc[k], a->p.N, a->sp.pk, a->stream));
   ACK(a, launch_interp(a, a->fc[0], 0, nullptr));
+  set_work_rules(a);
   ACK(a, launch_links(a, nullptr));
-  if (int rc = rebuild_work(a)) return rc;
+  if (int rc = update_work(a)) return rc;
   ACK(a, launch_moments(a));
   ACK(a, cudaStreamSynchronize(a->stream));
   a->cp = 0;
@@ -1994,6 +2031,10 @@ int lbm_amr3d_step(lbm_amr3d *a, int n) {
   if (!a) return LBM_EINVAL;
   if (n < 0) return afail(a, LBM_EINVAL, "step count must be >= 0");
   if (!a->seeded) return afail(a, LBM_EINVAL, "call lbm_amr3d_init_macro first");
+  if (n > 1 && a->p.live && a->work_stale) {
+    if (int rc = update_work(a)) return rc;
+    destroy_graphs(a);  // captured for one macro-step, without the lists
+  }
   if ((n > 1 || a->dynamic) && !a->graph[0]) {
     int rc = build_graphs(a);
     if (rc) return rc;
@@ -2044,8 +2085,9 @@ int lbm_amr3d_set_body(lbm_amr3d *a, const lbm_body *body) {
   a->p.c = a->sp;
   destroy_graphs(a);
   if (!a->seeded) return LBM_OK;
+  set_work_rules(a);
   ACK(a, launch_links(a, nullptr));
-  return rebuild_work(a);
+  return LBM_OK;
 }
 
 int lbm_amr3d_set_links(lbm_amr3d *a, int on) {
@@ -2054,8 +2096,9 @@ int lbm_amr3d_set_links(lbm_amr3d *a, int on) {
   destroy_graphs(a);
   a->p.links = on ? a->d_links : nullptr;
   if (!a->seeded) return LBM_OK;
+  set_work_rules(a);
   ACK(a, launch_links(a, nullptr));
-  return rebuild_work(a);
+  return LBM_OK;
 }
 
 int lbm_amr3d_links(const lbm_amr3d *a) { return a && a->p.links ? 1 : 0; }

@@ -198,6 +198,34 @@ def test_amr3d_live_chunks_equal_whole_tiles(lbm, q, rb, dynamic, shape):
     assert abs(runs[0][4][0]) > 0
 
 
+@pytest.mark.parametrize("dynamic", [0, 1])
+@pytest.mark.parametrize("vx", [0.0, 0.1])
+def test_amr3d_work_lists_of_many_tiles(lbm, dynamic, vx):
+    """As above with more tiles than one CTA builds the lists of (1024),
+    a body at rest and a moving one, whose solid inside is most of the tiles.
+    Calls of one macro-step right after set_body run without the lists."""
+    from getting_air_b200 import scenarios as sc
+    dims = (56, 40, 40)
+    body = dict(shape="roundbox", centre=(20.3, 20.0, 19.9), a=11.0, b=11.0, c=11.0, r=2.0, v=(vx, 0.0, 0.0))
+    runs = []
+    for single in (False, True):
+        a = lbm.Amr3D(lbm.amr3d_config(19, dims, refine="body", rb=2, margin=2.0, dynamic=dynamic, manage_every=2,
+                                       slot_headroom=1.5, tau=0.62, has_body=1, use_bounceback=1, sponge_w=4.0,
+                                       sponge_u=(0.04, 0.0, 0.0), body=body))
+        a.init_macro(sc.uniform_macro(int(np.prod(dims)), (0.04, 0.0, 0.0)))
+        assert a.slots > 1024
+        for k in range(3):
+            for n in [1] * 5 if single else (5,):
+                a.step(n)
+            a.set_body(lbm.make_body(**dict(body, centre=(20.3 + vx * (k + 1) * 8, 20.0, 19.9))))
+            a.step(1)
+        runs.append(a.read_coarse() + a.read_pool() + (a.forces(), a.topology()["block_slot"]))
+        a.close()
+    for x, y in zip(*runs):
+        assert np.array_equal(x, y)
+    assert abs(runs[0][4][0]) > 0
+
+
 @pytest.mark.parametrize("bounceback", [0, 1])
 def test_fused_2d_macro_steps_with_more_tiles_than_blocks(lbm, bounceback):
     from getting_air_b200 import scenarios as sc
