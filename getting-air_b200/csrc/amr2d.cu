@@ -20,9 +20,11 @@
 //   root step (dense d2 kernel, writes mac)   amr_step1.wgsl NO_PARENT
 //   pool substep a->b, b->a at tau_f          amr_step1.wgsl stepCell
 //   restriction of the pool into the root     common_average.wgsl
-// Every pool kernel runs one CTA per slot of the active list (count read on
-// the device), so the non-refine macro-step is topology-independent and is
-// replayed from a CUDA graph.
+// The interp macro-steps between two refine rounds run in one cooperative
+// launch (amr_macro_loop, up to 32 of them). The explode interface, and a
+// session whose fused form is off, launch the kernels above one by one: each
+// walks the active list (its count is read on the device), so the macro-step
+// does not depend on the topology and is replayed from a CUDA graph.
 
 #include <algorithm>
 #include <cmath>

@@ -100,10 +100,10 @@ __device__ __forceinline__ bool tile_cell(const Amr3Params &p, TileCell &t) {
 // substep), so only the last macro-step's first substep updates the dead
 // cells with links (need), and one whose every link bounces keeps its value
 // (hold). A moving body's bounce depends on the whole history: then every
-// substep updates the cells of need (or all, where those are most). Where dead cells are read after all (the
-// penalty force's tile-clamped gather; the interp interface, whose ring
-// collides), and without the link table, every substep runs over every cell
-// (p.live = 0). Bound by instruction issue and the latency of the neighbour
+// substep updates the cells of need (or all, where those are most). Where dead
+// cells are read after all (the penalty force's tile-clamped gather; the interp
+// interface, whose ring collides), and without the link table, every substep
+// runs over every cell (p.live = 0). Bound by instruction issue and the latency of the neighbour
 // gathers; per macro-step, together with the merged launches below, 2262
 // tiles around a box in 180^3: 660 -> 447 us; 160 tiles around a
 // sphere in 192x128x128, where the coarse step is most of it: 154 -> 139 us.

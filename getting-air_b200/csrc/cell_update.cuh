@@ -39,7 +39,6 @@ constexpr float kInvCS2 = 3.0f;
 template <typename S> struct Codec;
 template <> struct Codec<float> {
   static __device__ __forceinline__ float ld(const float *p, int, const Pack &) { return __ldg(p); }
-  static __device__ __forceinline__ float dec(float v, int, const Pack &) { return v; }
   static __device__ __forceinline__ void st(float *p, float v, int, const Pack &) {
     if (LBM_STREAMING_STORES) __stcs(p, v); else *p = v;
   }
@@ -133,8 +132,8 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sm) {
 }
 
 // The fixed-order sum of nparts partials by one warp (lane = threadIdx.x):
-// lane l adds partials l, l + 32, ... in order, then the warp's fixed tree. Every caller that sums the same partials this way gets the
-// same bits.
+// lane l adds partials l, l + 32, ... in order, then the warp's fixed tree.
+// Every caller that sums the same partials this way gets the same bits.
 template <int NV>
 __device__ __forceinline__ void sum_partials_warp(const double *partials, int nparts, double *out) {
   const int lane = threadIdx.x & 31;

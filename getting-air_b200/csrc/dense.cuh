@@ -69,7 +69,7 @@ struct StepParams {
   // with `counter` as its ticket and `groups` as its first-level sums): with
   // defer_force = 0 launch_step() follows the step with a launch that does
   // it; with defer_force = 1 it is left to the next launch on the stream,
-  // whose first blocks sum the prev_parts partials at prev_partials.
+  // which sums the prev_parts partials at prev_partials (add_sum_layers).
   double *groups;
   int defer_force;
   int prev_parts;
@@ -92,7 +92,7 @@ struct StepParams {
   int flat;
   unsigned magic;
   // Layers (along z; D2Q9: rows) of blocks in front of the grid that only sum
-  // the previous launch's force partials (sum_layers_for).
+  // the previous launch's force partials (add_sum_layers).
   int sum_layers;
   // The plane (3D) or row (D2Q9) that the launch's first blocks take: the
   // force region's first, so that its blocks, whose chain of link tests, own

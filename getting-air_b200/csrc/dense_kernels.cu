@@ -14,9 +14,10 @@
 // Layout in HBM: f is Q planes, plane-major, `f[i * n + cell]` with
 // cell = (z*NY + y)*NX + x -- the reference's layout, which is also the one
 // that gives every warp a coalesced 128-byte row per plane. One thread owns
-// one cell: it issues the Q pull loads up front (periodic sources), patches
-// the few bounce-back links afterwards, collides in registers and writes
-// the Q planes of its own cell. The mac field is written only when the
+// one cell: it decides which of its links the body or a wall cuts (in a block
+// that either can reach; the others skip this), issues the Q pull loads
+// (periodic sources), patches the few cut links, collides in registers and
+// writes the Q planes of its own cell. The mac field is written only when the
 // host asks for it (the last step of a batch), not every step.
 //
 // The body force is summed INSIDE the step: the reference runs a separate
@@ -25,14 +26,15 @@
 // is already in this kernel's registers. Only the launch blocks whose cells
 // can touch the body reduce; each writes one FP64 partial, and the partials
 // are summed in a fixed order after the launch, so the result is
-// deterministic: by the first blocks of the next step when steps follow one
-// another, else by a small launch of the same blocks. The kernel boundary is
-// what orders the partials before the sum. A last-block ticket inside the
-// step needs a release fence per partial, and under the step's full write
-// traffic each fence held its CTA for microseconds; one block summing all
-// partials waits on dozens of rounds of loads; and a one-block launch after
-// every step costs its launch gaps (measured at 256x128x128: +9 %, +10 %
-// and +7 % of the step against no force at all, and +1 % for this form).
+// deterministic: by blocks of their own in front of the next step's grid when
+// steps follow one another (add_sum_layers), else by a small launch of the
+// same blocks. The kernel boundary is what orders the partials before the sum.
+// A last-block ticket inside the step needs a release fence per partial, and
+// under the step's full write traffic each fence held its CTA for
+// microseconds; one block with cells summing all partials first waits on
+// dozens of rounds of loads; and a one-block launch after every step costs its
+// launch gaps (measured at 256x128x128: +9 %, +10 % and +7 % of the step
+// against no force at all, and +1 % for the sum in the next launch).
 
 #include <algorithm>
 
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepMinBlocks)
 }
 
 // The force of a step that no following launch sums: the same blocks, with
-// the same arithmetic, as the first blocks of a following step.
+// the same arithmetic, as those in front of a following step's grid.
 __global__ void __launch_bounds__(kStepThreads)
     force_finish(const double *__restrict__ partials, int nparts, double *__restrict__ groups,
                  unsigned int *__restrict__ counter, double *__restrict__ out) {

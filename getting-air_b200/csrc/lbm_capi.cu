@@ -416,8 +416,9 @@ int lbm_step(lbm_session *s, int n) {
     }
     return LBM_OK;
   }
-  // Each step's force partials are summed by the next step's first block;
-  // the last step's by the one-CTA sum launch_step() adds after it.
+  // Each step's force partials are summed by blocks in front of the next
+  // step's grid; the last step's by the launch of such blocks that
+  // launch_step() adds after it.
   const int64_t half = (int64_t)s->force_nparts * kForceSlots;
   const int parts = s->sp.force_on ? force_parts(s->q, s->sp) : 0;
   for (int k = 0; k < n; ++k) {
