@@ -103,10 +103,10 @@ __device__ __forceinline__ bool tile_cell(const Amr3Params &p, TileCell &t) {
 // substep updates the cells of need (or all, where those are most). Where dead
 // cells are read after all (the penalty force's tile-clamped gather; the interp
 // interface, whose ring collides), and without the link table, every substep
-// runs over every cell (p.live = 0). Bound by instruction issue and the latency of the neighbour
-// gathers; per macro-step, together with the merged launches below, 2262
-// tiles around a box in 180^3: 660 -> 447 us; 160 tiles around a
-// sphere in 192x128x128, where the coarse step is most of it: 154 -> 139 us.
+// runs over every cell (p.live = 0). Bound by instruction issue and the latency
+// of the neighbour gathers; per macro-step, together with the merged launches
+// below, 2262 tiles around a box in 180^3: 660 -> 445 us; 160 tiles around a
+// sphere in 192x128x128, where the coarse step is most of it: 154 -> 138 us.
 constexpr int kListThreads = 128;
 constexpr int kWorkCounts = 4;  // lengths of the work lists, and the chunks of all tiles
 // Threads and CTAs of amr3_work, a thread per slot: one CTA where it holds all.
@@ -1171,9 +1171,10 @@ __global__ void __launch_bounds__(kManageThreads)
 // (explode's), and the substeps' with those that amr3_links flagged. A thread
 // per slot. One CTA, where it holds all slots; else two launches: each CTA's
 // counts, then (FILL) the items, each CTA behind those before it. From the last
-// one the lengths and the number of all tiles' chunks (n). In one CTA over all slots they took 63 us for 2262
-// tiles, at every decision of a manager; appended by atomics, out of slot order,
-// the substeps that walked them took 1.3 % longer.
+// one the lengths and the number of all tiles' chunks (n). In one CTA over all
+// slots they took 63 us for 2262 tiles, at every decision of a manager (now 12
+// and 15); appended by atomics, out of slot order, the substeps that walked them
+// took 1.3 % longer.
 template <bool FILL>
 __global__ void __launch_bounds__(1024)
     amr3_work(const int *__restrict__ block_slot, const int *__restrict__ slot_to_block,
@@ -1466,8 +1467,8 @@ void launch_coalesce(cudaStream_t st, const float *fp, float *fc, float4 *macc, 
 // A pool substep, with 32-bit population indices when the pool allows, over
 // every cell, the live ones, or those and the dead ones with links. Over every
 // cell it takes the list whose ring is in rows: grouped by neighbour the ring
-// splits sectors that rows share (2262 tiles, a macro-step whose second substep is
-// over every cell: 633 -> 577 us; the interp interface, both: 1125 -> 1034).
+// splits sectors that rows share (2262 tiles, a substep: 248 -> 191 us; the
+// interp interface, both substeps: 1125 -> 1034 us per macro-step).
 enum class Cells { kAll, kLive, kNeed };
 template <int Q>
 void launch_substep(lbm_amr3d *a, cudaStream_t st, const float *fin, float *fout, const Amr3Params &p, Cells which) {
