@@ -933,7 +933,7 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
     return;
   }
   CellForce cf;
-  cell3<Q, float, false, LINKS>(fin, fout, mac, sp, x, y, m.bz, false, cf);
+  cell3<Q, float, false, LINKS, WIN>(fin, fout, mac, sp, x, y, m.bz, false, cf);
 }
 
 // ---- the refinement manager (common_d3_manage.wgsl) ------------------------

@@ -84,8 +84,10 @@ __device__ __forceinline__ void stage_pose(const StepParams &p, StepParams &sp) 
 // registers, so fewer warps to hide the gather.)
 // WIN: a domain with a moving window, whose fluid blocks take the sponge in
 // window coordinates (an instantiation of its own: in the other it would cost
-// 1 to 2 %). us per step of a windowed FP32 sphere with every block general
-// and like this: 128^3 72.7 -> 67.2, 256x128x128 129.2 -> 117.6.
+// 1 to 2 %) and whose links see which image of the body they lead to
+// (solid_links_call). us per step of a windowed FP32 sphere with every block
+// general, with fluid blocks, and with those links: 128^3 72.7, 67.2, 62.9;
+// 256x128x128 129.2, 117.6, 112.9.
 template <int Q, typename S, bool TRT, bool WIN>
 __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) / 4 : kStepMinBlocks)
     d3_step(const S *__restrict__ fin, S *__restrict__ fout, float *__restrict__ mac,
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(kStepThreads, Q == 27 ? (kStepMinBlocks * 3) /
     return;
   }
   CellForce cf;
-  if (c < m.lim) cell3<Q, S, TRT>(fin, fout, mac, p, x, y, m.bz, m.region, cf);
+  if (c < m.lim) cell3<Q, S, TRT, true, WIN>(fin, fout, mac, p, x, y, m.bz, m.region, cf);
   if (m.region) publish_force<kStepThreads>(cf, p.partials, m.part);
 }
 
