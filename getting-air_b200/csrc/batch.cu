@@ -94,11 +94,19 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS)
   }
 }
 
-// c / nx by multiplication where the host found it exact (row_magic): the
-// lean kernel's two divisions a cell were 70.3 -> 68.8 us per step of 64
-// domains (4.9 M cells).
-__device__ __forceinline__ int row_of(unsigned c, int nx, unsigned magic) {
-  return magic ? (int)__umulhi(c, magic) : (int)c / nx;
+// Row and column of cell c by multiplication: with magic = row_magic(nx) the
+// product's upper half is c / nx or, for rows and domains too long for
+// row_magic's bound, one more. The lean kernel's two divisions a cell were 70.3
+// -> 68.8 us per step of 64 domains (4.9 M cells, FP32). (Multiplying within
+// the bound and dividing beyond it kept both in the loop, where 16-bit storage
+// has no registers left: 74.2 us had become 88.0 there, with this 65.4.)
+__device__ __forceinline__ void row_of(unsigned c, int nx, unsigned magic, int &x, int &r) {
+  r = (int)__umulhi(c, magic);
+  x = (int)c - r * nx;
+  if (x < 0) {
+    x += nx;
+    --r;
+  }
 }
 
 // The fluid tiles of a D2Q9 batch (cell2_fluid). Without the bounce-back
@@ -121,7 +129,10 @@ __global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1024 : 768) / THREA
     int *dst = reinterpret_cast<int *>(sp_raw);
     for (int j = threadIdx.x; j < (int)(sizeof(StepParams) / 4); j += THREADS) dst[j] = __ldg(src + j);
     __syncthreads();
-    if (threadIdx.x == 0) sp.write_mac = write_mac;
+    if (threadIdx.x == 0) {
+      sp.write_mac = write_mac;
+      if (!sp.magic) sp.magic = row_magic(sp.nx);
+    }
     __syncthreads();
     const int nx = sp.nx;
     const int end = min(td.y + cells_per_tile, nx * sp.ny);
@@ -129,8 +140,9 @@ __global__ void __launch_bounds__(THREADS, (sizeof(S) == 4 ? 1024 : 768) / THREA
     for (int c = td.y + threadIdx.x; c < end; c += 2 * THREADS) {
       const int c2 = c + THREADS;
       const bool two = c2 < end;
-      const int r = row_of((unsigned)c, nx, sp.magic), x = c - r * nx;
-      const int r2 = two ? row_of((unsigned)c2, nx, sp.magic) : 0, x2 = two ? c2 - r2 * nx : 0;
+      int x, r, x2 = 0, r2 = 0;
+      row_of((unsigned)c, nx, sp.magic, x, r);
+      if (two) row_of((unsigned)c2, nx, sp.magic, x2, r2);
       float f[9], g[9];
       gather2<S>(fin + sp.base, sp, x, r, f);
       if (two) gather2<S>(fin + sp.base, sp, x2, r2, g);

@@ -145,6 +145,14 @@ def test_pinned_free_body_equals_prescribed_pose(lbm, shape, bb, storage):
     assert np.allclose(out[0][2], out[1][2], rtol=1e-10, atol=1e-12 * np.abs(out[0][2]).max())
 
 
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("dims", [(3, 3, 1), (4, 257, 1), (1625, 40, 1), (37838, 3, 1), (37837, 3, 1), (70001, 5, 1)])
+def test_2d_rows_of_any_length_equal_batch(lbm, dims, storage):
+    """The batch finds a cell's row by a multiplication, exact on its own up to
+    nx^2 ny = 2^32 (between the fourth and the fifth of these domains)."""
+    dense_and_batch(lbm, 9, dims, 3, tau=0.6, force=(1e-5, -2e-5, 0.0), storage=storage, wall=(0, 1, 0), sponge_w=4.0)
+
+
 QUAT = (0.8, 0.36, 0.48, 0.0)
 
 
